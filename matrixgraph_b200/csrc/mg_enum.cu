@@ -256,7 +256,7 @@ __device__ __forceinline__ bool contains(const uint32_t* __restrict__ a, uint32_
 
 __device__ __forceinline__ void slice_of(const GraphDev& g, uint32_t dir, uint32_t y,
                                          uint32_t lab, uint32_t& s, uint32_t& e) {
-  const uint32_t* p = g.loff[dir] + uint64_t(y) * g.L + lab;
+  const uint32_t* p = g.loff[dir] + uint64_t(lab) * g.n + y;
   s = __ldg(p);
   e = __ldg(p + 1);
 }
@@ -376,9 +376,10 @@ __global__ void __launch_bounds__(256) k_tail_dense(GraphDev g, TailKey tk,
   const uint64_t warp = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5;
   const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
   const uint32_t nh = g.n_hubs[tk.da];
+  const uint32_t b0 = __ldg(g.bucket_off + tk.lp), b1 = __ldg(g.bucket_off + tk.lp + 1);
   for (uint64_t h = warp; h < nh; h += nwarps) {
     const uint32_t y = __ldg(g.hub_vid[tk.da] + h);
-    if (__ldg(g.label + y) != tk.lp) continue;
+    if (y < b0 || y >= b1) continue;
     uint32_t s, e;
     slice_of(g, tk.da, y, tk.la, s, e);
     unsigned long long sa = 0, sd = 0;
@@ -420,7 +421,7 @@ __device__ __forceinline__ void tail_agg(const StepArgs& a, const PlanDev& P, ui
   }
   unsigned long long* slot = nullptr;
   if (tk.lazy != ~0ull) {
-    slot = a.tdL + tk.lazy + __ldg(g.bucket_pos + mp);
+    slot = a.tdL + tk.lazy + (mp - tk.b0);
     const unsigned long long w = *reinterpret_cast<volatile unsigned long long*>(slot);
     if (w != ~0ull) {
       c = (long long)(w & 0xFFFFFFFFull);
@@ -785,7 +786,7 @@ __global__ void __launch_bounds__(EXPAND_BLOCK) k_expand(StepArgs a) {
         const uint32_t lab = P.label[i];
         uint32_t ddir = 0;
         if (ci == DCI_BUCKET) {
-          x = __ldg(g.bucket_vid + ds + (i == 0 ? uint64_t(e) * a.root_step : uint64_t(e)));
+          x = ds + (i == 0 ? e * a.root_step : e);
         } else {
           ddir = P.cons[i][ci] >> 8;
           x = __ldg(g.adj[ddir] + ds + e);
@@ -1299,6 +1300,7 @@ static int setup_tails(DevGraph* dg, std::vector<PlanDev>& plans, TailStore& ts,
       tk.base = (nh && entries + nh <= (1ull << 27)) ? entries : ~0ull;
       if (tk.base != ~0ull) entries += nh;
       const uint64_t nb = dg->h_bucket_off[tk.lp + 1] - dg->h_bucket_off[tk.lp];
+      tk.b0 = dg->h_bucket_off[tk.lp];
       tk.lazy = (lazy + nb <= (1ull << 30)) ? lazy : ~0ull;
       if (tk.lazy != ~0ull) lazy += nb;
       keys.push_back(tk);
@@ -2112,10 +2114,7 @@ static int selftest_wait(DevGraph* dg, const mg_csr_view* q, uint32_t spin_limit
   MG_CK(cudaMemcpyAsync(L.ctr, ctr.data(), C_NUM * 8, cudaMemcpyHostToDevice, st));
   // every row holds the first vertex of the bucket of position 0
   const uint32_t b0 = dg->h_bucket_off[P.label[0]];
-  std::vector<uint32_t> col(rows, 0);
-  MG_CK(cudaMemcpyAsync(col.data(), dg->g.bucket_vid + b0, 4, cudaMemcpyDeviceToHost, st));
-  MG_CK(cudaStreamSynchronize(st));
-  for (uint64_t r = 1; r < rows; ++r) col[r] = col[0];
+  std::vector<uint32_t> col(rows, b0);
   MG_CK(cudaMemcpyAsync(L.col[1][0], col.data(), rows * 4, cudaMemcpyHostToDevice, st));
   StepArgs a;
   std::memset(&a, 0, sizeof(a));

@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(kMfBlock) k_matrix_filter(
     const float* __restrict__ data_emb, const float* __restrict__ eu,
     const float* __restrict__ w1t, const float* __restrict__ b1, const float* __restrict__ w2,
     float b2, uint32_t dim, uint32_t hidden, const uint32_t* __restrict__ cand, uint64_t ncand,
-    uint8_t* keep_bytes, uint32_t* keep_bits) {
+    uint8_t* keep_bytes, uint32_t* keep_bits, uint32_t bit0) {
   extern __shared__ float smem[];
   const uint32_t lane = threadIdx.x & 31, wib = threadIdx.x >> 5, wpb = blockDim.x >> 5;
   float* sim = smem + wib * (dim + kMfMaxHidden);
@@ -110,7 +110,8 @@ __global__ void __launch_bounds__(kMfBlock) k_matrix_filter(
       const float s = 1.0f / (1.0f + expf(-z2));
       const bool keep = !(s < 0.1f);
       if (keep_bytes) keep_bytes[c] = keep ? 1 : 0;
-      if (keep_bits && keep) atomicOr(keep_bits + (v >> 5), 1u << (v & 31));
+      if (keep_bits && keep)
+        atomicOr(keep_bits + ((bit0 + c) >> 5), 1u << ((bit0 + c) & 31));
     }
     __syncwarp();
   }
@@ -141,7 +142,7 @@ int matrix_filter_roots(void* filter, const DevGraph* dg, uint32_t u, uint32_t l
                                              uint64_t(dg->sms) * 16);
   k_matrix_filter<<<unsigned(blocks), kMfBlock, smem, st>>>(
       F->data_emb, F->eu, F->w1t, F->b1, F->w2, F->b2, F->dim, F->hidden,
-      dg->g.bucket_vid + b0, nb, nullptr, bits);
+      dg->g.input_id + b0, nb, nullptr, bits, uint32_t(b0));
   MG_CK(cudaGetLastError());
   // F->eu is rewritten by the next call: finish this one first
   MG_CK(cudaStreamSynchronize(st));
@@ -250,7 +251,8 @@ int mg_matrix_filter_keep(void* filter, uint32_t u, const uint32_t* v, uint64_t 
   const uint64_t blocks = std::min<uint64_t>((nv + mg::kMfBlock / 32 - 1) / (mg::kMfBlock / 32),
                                              4096);
   mg::k_matrix_filter<<<unsigned(blocks), mg::kMfBlock, smem, st>>>(
-      F->data_emb, F->eu, F->w1t, F->b1, F->w2, F->b2, F->dim, F->hidden, dv, nv, dk, nullptr);
+      F->data_emb, F->eu, F->w1t, F->b1, F->w2, F->b2, F->dim, F->hidden, dv, nv, dk, nullptr,
+      0);
   MG_CK(cudaGetLastError());
   MG_CK(cudaMemcpyAsync(keep, dk, nv, cudaMemcpyDeviceToHost, st));
   cudaFreeAsync(dv, st);
