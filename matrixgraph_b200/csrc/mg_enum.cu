@@ -12,12 +12,12 @@
 //   * the work kernel picks, per row, the shortest label slice among the
 //     backward neighbours' adjacency (the driving list) and the scan turns
 //     the driving lengths into an element index space;
-//   * the expand kernel assigns one element (row, driving entry) per thread,
-//     so hub rows spread over many warps; the other backward slices are
-//     probed in the hub bitmap when their vertex is a hub, else by binary
-//     search, injectivity is checked against the row, the
-//     label/degree/neighbour-label filter prunes, and survivors are appended
-//     with warp-aggregated atomics (__ballot_sync / __popc);
+//   * the expand kernel deals that space to warps in tasks of consecutive
+//     elements (row, driving entry), so hub rows spread over many warps; the
+//     other backward slices are probed in the hub bitmap when their vertex is
+//     a hub, else by binary search, injectivity is checked against the row,
+//     and the survivors of a task are filtered (label, degree, neighbour
+//     labels) and appended with one atomic (__ballot_sync / __popc ranks);
 //   * a table chunk never holds more than `cap` rows: the host walks the
 //     levels depth-first, expanding at most `cap` elements of a level before
 //     descending, so intermediate results never exceed the scratch budget;
@@ -29,6 +29,7 @@
 #include <algorithm>
 #include <cstring>
 #include <numeric>
+#include <type_traits>
 
 #include "mg_device.cuh"
 
@@ -119,7 +120,9 @@ static int ws_alloc(Workspace* ws, void** p, size_t bytes) {
 constexpr uint64_t kDefaultCap = 1ull << 24;
 constexpr uint32_t kProbeMin = 1;  // default: every hub slice is probed in the bitmap
 constexpr int SCAN_TILE = 4096;
-constexpr int EXPAND_BLOCK = 256;                 // elements per expand tile
+constexpr int EXPAND_BLOCK = 256;
+constexpr int EXPAND_TILE = 1024;                 // elements per expand tile
+constexpr int XSTAGE = 256;                       // survivors a warp stages at a time
 constexpr uint64_t kSegment = 1ull << 26;         // elements per expand launch
 
 static uint64_t level_row_bytes(int l) { return uint64_t(l) * 4 + 4 + 4 + 8 + 4 + 1; }
@@ -145,7 +148,7 @@ static int ensure_ws(DevGraph* dg, uint64_t cap, int levels, uint32_t nq) {
     MG_CK(cudaEventCreate(&ws->ev3));
     ws->bsum_cap = uint32_t((std::max<uint64_t>(cap, ws->rows0) + SCAN_TILE - 1) / SCAN_TILE + 1);
     if ((rc = ws_alloc(ws, (void**)&ws->bsum, uint64_t(ws->bsum_cap) * 8))) return rc;
-    if ((rc = ws_alloc(ws, (void**)&ws->tile_row, (kSegment / EXPAND_BLOCK + 2) * 4))) return rc;
+    if ((rc = ws_alloc(ws, (void**)&ws->tile_row, (kSegment / EXPAND_TILE + 2) * 4))) return rc;
   }
   if (ws->counts_cap < nq) {
     int rc;
@@ -696,13 +699,13 @@ __global__ void __launch_bounds__(256) k_scan_apply(const uint32_t* __restrict__
 }
 
 // First row of every tile of the element range [t0, t1): tile_row[j] is the
-// row holding element t0 + j*EXPAND_BLOCK (clamped to t1 - 1), j = 0..ntiles.
+// row holding element t0 + j*EXPAND_TILE (clamped to t1 - 1), j = 0..ntiles.
 __global__ void __launch_bounds__(256) k_tile_rows(const uint64_t* __restrict__ woff, uint32_t R,
                                                    uint64_t t0, uint64_t t1, uint32_t ntiles,
                                                    uint32_t* tile_row) {
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j <= ntiles;
        j += gridDim.x * blockDim.x) {
-    uint64_t t = t0 + uint64_t(j) * EXPAND_BLOCK;
+    uint64_t t = t0 + uint64_t(j) * EXPAND_TILE;
     if (t > t1 - 1) t = t1 - 1;
     tile_row[j] = find_row(woff, 0, R - 1, t);
   }
@@ -718,12 +721,117 @@ enum : int {
   X_ONE = 16,   // one query, no row query ids: its plan is staged in shared memory
 };
 
-// Expand kernel: one element (row, driving entry) per thread.
+// One set-up row of an expand task (shared memory, a row per slot).  A further
+// constraint is probed at p: the hub bitmap row of its vertex (len HUB_LEN), or
+// its sorted label slice of len entries.  The stride of 80 bytes keeps 16-byte
+// reads of eight consecutive rows free of bank conflicts.
+struct alignas(16) XRow {
+  const uint32_t* list;  // list[e] is element e of the task (nullptr: a bucket row)
+  const uint32_t* p0;    // first further constraint
+  uint32_t len0, m0;     // m0, m1: earlier matches a candidate must differ from
+  uint32_t row, beg;     // table row; its first element of the task
+  const uint32_t* p1;    // second further constraint
+  uint32_t len1, m1;
+  uint32_t q, ci, v0;    // query; driving constraint; bucket row: element e is
+  uint32_t end;          // vertex v0 + e * root_step
+  uint32_t pad[4];
+};
+constexpr uint32_t HUB_LEN = FULL;
+
+// Probe data of constraint cs for row r (see XRow); an empty slice points at
+// readable memory.
+__device__ __forceinline__ void probe_of(const StepArgs& a, uint32_t cs, uint32_t lab, uint32_t r,
+                                         const uint32_t*& p, uint32_t& len) {
+  const GraphDev& g = a.g;
+  const uint32_t d = cs >> 8;
+  const uint32_t y = a.in.col[cs & 0xFF][r];
+  uint32_t h = NO_HUB, s = 0, e = 0;
+  if (g.hub_slot[d]) h = __ldg(g.hub_slot[d] + y);
+  if (h == NO_HUB || a.probe_min > 1) slice_of(g, d, y, lab, s, e);
+  if (h == NO_HUB || (a.probe_min > 1 && e - s < a.probe_min)) {
+    p = e > s ? g.adj[d] + s : g.bucket_off;
+    len = e - s;
+  } else {
+    p = g.hub_bits[d] + uint64_t(h) * g.hub_words;
+    len = HUB_LEN;
+  }
+}
+
+// Probes U candidates per lane, each against a constraint of its own: p[u],
+// len[u] as in XRow; ok[u] is cleared where x[u] is not in it.  No load hangs
+// on a condition, so the loads of the U candidates overlap.  Searches halve
+// together until the longest slice of the warp is done.
+template <int U>
+__device__ __forceinline__ void probe_all(const uint32_t* const (&p)[U], const uint32_t (&len)[U],
+                                          const uint32_t (&x)[U], bool (&ok)[U]) {
+  uint32_t w[U], longest = 0;
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    w[u] = __ldg(p[u] + (len[u] == HUB_LEN ? x[u] >> 5 : 0u));
+    if (len[u] != HUB_LEN && ok[u]) longest = max(longest, len[u]);
+  }
+  longest = __reduce_max_sync(FULL, longest);
+  if (longest) {
+    uint32_t at[U], n[U];  // the last entry <= x[u], if any, lies in [at, at + n)
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      at[u] = 0;
+      n[u] = len[u] == HUB_LEN ? 0u : len[u];
+    }
+    for (; longest > 1; longest -= longest >> 1) {
+      uint32_t v[U];
+#pragma unroll
+      for (int u = 0; u < U; ++u) v[u] = __ldg(p[u] + (at[u] + (n[u] >> 1)));
+#pragma unroll
+      for (int u = 0; u < U; ++u) {
+        const uint32_t half = n[u] >> 1;
+        at[u] += v[u] <= x[u] ? half : 0u;
+        n[u] -= half;
+      }
+    }
+#pragma unroll
+    for (int u = 0; u < U; ++u) {
+      const uint32_t v = __ldg(p[u] + at[u]);
+      if (len[u] != HUB_LEN) ok[u] = ok[u] && len[u] && v == x[u];
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (len[u] == HUB_LEN) ok[u] = ok[u] && ((w[u] >> (x[u] & 31)) & 1u);
+}
+
+// Expand kernel: a warp takes tasks of up to EXPAND_TILE consecutive elements
+// (row, driving entry).
+//
+// What bounds it: chains of dependent loads that mostly hit L2 (row offset ->
+// matched vertices -> hub slot or slice -> candidate -> probe), and then the
+// instructions per candidate.  So
+//   * the state of a row (XRow) is set up for 32 rows at once, a row per lane,
+//     and kept in shared memory: one chain of loads per 32 rows;
+//   * candidates are taken 32 * XU at a time whatever their rows, every lane
+//     finding its rows by the row starts up to its element; the candidates of
+//     the next group are loaded while this one is probed, and the XU probes of
+//     a lane are independent loads;
+//   * survivors are staged in shared memory, so that what follows them
+//     (filters, closed forms, appending to the next table, emitting) runs on
+//     full warps, with one reservation per staged group and no block barriers.
+// Against one element per thread with a search for its row in global memory
+// and 256-thread tiles (R-MAT scale 22): 4-cycle 15.7 -> 11.9 ms, 4-clique
+// 12.1 -> 7.3 ms, 256 batched queries 110 -> 67 ms.  A table that overflows is
+// flagged once per warp, not once per survivor: runs past their budget on
+// scale 20 took 577 ms and take 65.  Two candidates a lane (XU) and four
+// blocks per SM (64 registers) were the best of 1-4 and 3-6: more candidates
+// spill, fewer expose the probe latency.  Walking each row by its own, 32-128
+// candidates at a time, was no better (11.3-12.5 ms for the 4-cycle).
 template <int MODE>
-__global__ void __launch_bounds__(EXPAND_BLOCK) k_expand(StepArgs a) {
+__global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
+  constexpr bool ONE = (MODE & X_ONE) != 0;
+  // Launches that only count complete matches keep nothing of a survivor.
+  constexpr bool STAGE = (MODE & (X_WRITE | X_EMIT | X_FUSED | X_TAIL)) != 0 || !ONE;
+  constexpr int XU = 2;
   const uint32_t i = a.level;
   const GraphDev& g = a.g;
-  const uint32_t lane = threadIdx.x & 31;
+  const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   uint64_t t0 = a.t0, t1 = a.t1;
   if (a.lane) {  // lane pipeline: this level's elements, capped (k_tile_rows_lane flags it)
     t0 = 0;
@@ -731,217 +839,376 @@ __global__ void __launch_bounds__(EXPAND_BLOCK) k_expand(StepArgs a) {
     if (t1 > a.seg_cap) t1 = a.seg_cap;
   }
   const uint64_t span = t1 - t0;
-  const uint64_t ntiles = (span + EXPAND_BLOCK - 1) / EXPAND_BLOCK;
-  unsigned long long cnt = 0, bal = 0, balc = 0, s1 = 0, sk = 0, s2 = 0;
-  uint32_t cnt_q = 0;
-  // Device work queue: each block takes `grab` consecutive tiles at a time,
-  // so a block walks contiguous element ranges (same rows, same query) and a
-  // hub row's elements still spread over many blocks.
-  __shared__ unsigned long long s_base, s_wbase;
-  __shared__ uint32_t s_wcnt[EXPAND_BLOCK / 32];
-  // A single query's plan is read by every element: staged once per block,
-  // its fields are shared-memory loads with 32-bit addressing.
+  const uint32_t ntiles = uint32_t((span + EXPAND_TILE - 1) / EXPAND_TILE);
+  __shared__ XRow s_rows[EXPAND_BLOCK / 32][32];
+  __shared__ uint32_t s_x[STAGE ? EXPAND_BLOCK / 32 : 1][STAGE ? XSTAGE : 1];
+  __shared__ uint32_t s_r[STAGE ? EXPAND_BLOCK / 32 : 1][STAGE ? XSTAGE : 1];
+  // A single query's plan is read by every row: staged once per block.
   __shared__ PlanDev s_plan;
-  if constexpr ((MODE & X_ONE) != 0) {
+  if constexpr (ONE) {
     const uint32_t* src = reinterpret_cast<const uint32_t*>(a.plans);
     uint32_t* dst = reinterpret_cast<uint32_t*>(&s_plan);
     for (uint32_t w = threadIdx.x; w < sizeof(PlanDev) / 4; w += EXPAND_BLOCK) dst[w] = src[w];
     __syncthreads();
   }
-  // Tiles per grab: about 16 grabs per block over the launch (fewer queue
-  // atomics and barriers), at least 4, at most 32.
-  uint64_t grab = a.grab;
-  if (!grab) {
-    grab = ntiles / (uint64_t(gridDim.x) * 16);
-    grab = grab < 4 ? 4 : (grab > 32 ? 32 : grab);
-  }
-  for (;;) {
-    if (threadIdx.x == 0) s_base = atomicAdd(&a.ctr[a.tile_slot], (unsigned long long)grab);
-    __syncthreads();
-    const uint64_t gbase = s_base;
-    __syncthreads();
-    if (gbase >= ntiles) break;
-    const uint64_t gend = min(gbase + grab, ntiles);
-    for (uint64_t tile = gbase; tile < gend; ++tile) {
-      const uint64_t tb = t0 + tile * EXPAND_BLOCK;
-      const uint64_t te = min(tb + EXPAND_BLOCK, t1);
-      const uint32_t rlo = __ldg(a.tile_row + tile), rhi = __ldg(a.tile_row + tile + 1);
-      const uint64_t t = tb + threadIdx.x;
-      const bool valid = t < te;
-      bool ok = false, fin = false, fused = false, ftail = false;
-      uint32_t r = 0, x = 0, q = 0;
-      if (valid) {
-        r = find_row(a.woff, rlo, rhi, t);
-        const uint32_t e = uint32_t(t - a.woff[r]);
-        const uint8_t ci = a.dci[r];
-        const uint32_t ds = a.dstart[r];
-        const PlanDev* Pp;
-        if constexpr ((MODE & X_ONE) != 0) {
-          Pp = &s_plan;
-        } else {
-          q = a.in.qid ? a.in.qid[r] : 0u;
-          Pp = a.plans + q;
-        }
-        const PlanDev& P = *Pp;
-        const uint32_t lab = P.label[i];
-        uint32_t ddir = 0;
-        if (ci == DCI_BUCKET) {
-          x = ds + (i == 0 ? e * a.root_step : e);
-        } else {
-          ddir = P.cons[i][ci] >> 8;
-          x = __ldg(g.adj[ddir] + ds + e);
-        }
-        ok = true;
-        // the lossy matrix filter drops level-0 candidates it rejects
-        if (i == 0 && a.root_keep && !((__ldg(a.root_keep + (x >> 5)) >> (x & 31)) & 1u))
-          ok = false;
-        // injectivity: only earlier positions with the same label can collide
-        for (uint32_t m = P.samelab[i]; m && ok; m &= m - 1) {
-          const uint32_t j = __ffs(m) - 1;
-          if (a.in.col[j][r] == x) ok = false;
-        }
-        // remaining backward neighbours: binary search in their label slices
-        const uint32_t nc = P.ncons[i];
-        for (uint32_t c = 0; c < nc && ok; ++c) {
-          if (c == ci) continue;
-          const uint32_t cs = P.cons[i][c];
-          const uint32_t y = a.in.col[cs & 0xFF][r];
-          ok = in_slice(g, cs >> 8, y, lab, x, a.probe_min);
-        }
-        if (ok && ((P.selfloop_mask >> i) & 1u)) ok = has_self(g, x);
-        fin = (i + 1 == P.k);
-        if constexpr ((MODE & X_FUSED) != 0)
-          fused = !fin && a.count_mode && (i + 2 == P.k) && P.last_o1;
-        if constexpr ((MODE & X_TAIL) != 0)
-          ftail = ((a.tail_dense && P.tail2) || (a.star && P.star2)) && i + 3 == P.k;
-        // Filters prune positions whose survivors are extended further; the
-        // position before a last position counted in closed form is not
-        // filtered (the closed form already yields 0 for hopeless candidates).
-        if (ok && !fin && a.filters && !(i + 2 == P.k && P.last_o1))
-          ok = pass_filters(g, P, i, x, a.filters);
-        if (ok) {
+  // A lane whose tables overflowed stops: its query is counted again on the
+  // chunked path.
+  if (a.lane && a.ctr[C_ERR]) return;
+  auto plan = [&](uint32_t q) -> const PlanDev& { return ONE ? s_plan : a.plans[q]; };
+  auto query = [&](uint32_t r) -> uint32_t { return !ONE && a.in.qid ? a.in.qid[r] : 0u; };
+  // What candidates of this level are checked for (one query; a batch looks at
+  // every row's plan): further constraints, equal labels, and the rare checks.
+  const uint32_t others = ONE ? plan(0).ncons[i] - (plan(0).ncons[i] ? 1u : 0u) : 3u;
+  const uint32_t sames = ONE ? __popc(plan(0).samelab[i]) : 3u;
+  const bool extra = (i == 0 && a.root_keep) || ((plan(0).selfloop_mask >> i) & 1u);
+
+  unsigned long long cnt = 0, bal = 0, balc = 0, s1 = 0, sk = 0, s2 = 0;
+  uint32_t cnt_q = 0;
+  bool full = false;  // the output table is full (lane pipeline)
+  uint32_t staged = 0;
+
+  // What follows the staged survivors.
+  auto flush = [&]() {
+    __syncwarp();
+    uint32_t kept = 0;
+    for (uint32_t v0 = 0; v0 < staged; v0 += 32) {
+      bool ok = v0 + lane < staged;
+      const uint32_t x = ok ? s_x[wid][v0 + lane] : 0u, rr = ok ? s_r[wid][v0 + lane] : 0u;
+      const uint32_t q = ok ? query(rr) : 0u;
+      const PlanDev& P = plan(q);
+      const bool fin = i + 1 == P.k;
+      bool fused = false, ftail = false;
+      if constexpr ((MODE & X_FUSED) != 0)
+        fused = !fin && a.count_mode && (i + 2 == P.k) && P.last_o1;
+      if constexpr ((MODE & X_TAIL) != 0)
+        ftail = ((a.tail_dense && P.tail2) || (a.star && P.star2)) && i + 3 == P.k;
+      // Filters prune positions whose survivors are extended further; the
+      // position before a last position counted in closed form is not
+      // filtered (the closed form already yields 0 for hopeless candidates).
+      if (ok && !fin && a.filters && !(i + 2 == P.k && P.last_o1))
+        ok = pass_filters(g, P, i, x, a.filters);
+      if (ok) {
+        if constexpr (!ONE) {
           if (q != cnt_q) {
             acc_flush(a, cnt_q, i, cnt, s1, sk, s2);
             cnt = s1 = sk = s2 = 0;
             cnt_q = q;
           }
-          s1 += 1;
-          if (fin) {
-            if (a.count_mode) cnt += 1;
-          } else if ((MODE & X_TAIL) && ftail && P.star2) {
-            // The prefix ending in x has length k-2 and the plan ends in two
-            // leaves of one anchor: counted here, not stored.
-            unsigned long long tc, tp, tb, tbc;
-            star_close(a, P, [&](uint32_t j) { return j == i ? x : a.in.col[j][r]; }, tc, tp,
-                       tb, tbc);
-            cnt += tc;
-            sk += tc;
-            s2 += tp;
-            bal += tb;
-            balc += tbc;
-          } else if ((MODE & X_TAIL) && ftail) {
-            // The prefix ending in x has length k-2: its two-position pendant
-            // tail is counted here from the dense aggregates, not stored.
-            const uint32_t mp = P.tail_p == i ? x : a.in.col[P.tail_p][r];
-            uint32_t ts, te;
-            slice_of(g, P.tail_da, mp, P.label[P.k - 2], ts, te);
-            long long ac, ad;
-            tail_agg(a, P, mp, ts, te, ac, ad);
-            unsigned long long tc, tp, td;
-            tail_close(a, P, [&](uint32_t j) { return j == i ? x : a.in.col[j][r]; }, mp, ts, te,
-                       ac, ad, tc, tp, td);
-            cnt += tc;
-            sk += tc;
-            s2 += tp;
-            bal += 8ull + 4ull * (te - ts) + 8ull * tp + 4ull * td;
-            balc += 8ull + 4ull * (te - ts) + 8ull * tp;
-          } else if ((MODE & X_FUSED) && fused) {
-            const uint32_t kl = P.k - 1;
-            const uint32_t cs = P.cons[kl][0];
-            const uint32_t pos = cs & 0xFF, dir = cs >> 8;
-            const uint32_t y = pos == i ? x : a.in.col[pos][r];
-            uint32_t s, en;
-            slice_of(g, dir, y, P.label[kl], s, en);
-            unsigned long long c1 = en - s;
-            bal += 8ull + 4ull * c1;
-            balc += 8ull;
-            for (uint32_t m = P.samelab[kl]; m; m &= m - 1) {
-              const uint32_t j = __ffs(m) - 1;
-              if ((P.guar[kl] >> j) & 1u) {
-                c1 -= 1;
-              } else {
-                const uint32_t mj = j == i ? x : a.in.col[j][r];
-                c1 -= in_slice_se(g, dir, y, s, en, mj, a.probe_min) ? 1ull : 0ull;
-              }
-            }
-            sk += c1;
-            cnt += c1;
-          }
         }
-      }
-      // Survivors that extend the prefix: append to the next level table.  One
-      // reservation per tile keeps a tile's survivors (one row run, usually one
-      // query) contiguous in the next table.
-      // Launches without an output table (last or closed-form positions) skip
-      // the reservation and its barriers.
-      const bool wr = ok && !fin && !fused && !ftail;
-      if constexpr ((MODE & X_WRITE) != 0) {
-        const uint32_t wm = __ballot_sync(FULL, wr);
-        if (lane == 0) s_wcnt[threadIdx.x >> 5] = __popc(wm);
-        __syncthreads();
-        if (threadIdx.x == 0) {
-          uint32_t tot = 0;
-          for (uint32_t w = 0; w < EXPAND_BLOCK / 32; ++w) {
-            const uint32_t c = s_wcnt[w];
-            s_wcnt[w] = tot;
-            tot += c;
-          }
-          s_wbase = tot ? atomicAdd(&a.ctr[a.out_slot], (unsigned long long)tot) : 0ull;
-        }
-        __syncthreads();
-        if (wm) {
-          if (wr) {
-            const unsigned long long idx = s_wbase + s_wcnt[threadIdx.x >> 5] + __popc(wm & lanemask_lt());
-            if (idx < a.out_cap) {
-              for (uint32_t j = 0; j < i; ++j) a.out.col[j][idx] = a.in.col[j][r];
-              a.out.col[i][idx] = x;
-              if (a.out.qid) a.out.qid[idx] = q;
+        s1 += 1;
+        if (fin) {
+          if (!ONE && a.count_mode) cnt += 1;
+        } else if ((MODE & X_TAIL) && ftail && P.star2) {
+          // The prefix ending in x has length k-2 and the plan ends in two
+          // leaves of one anchor: counted here, not stored.
+          unsigned long long tc, tp, tb, tbc;
+          star_close(a, P, [&](uint32_t j) { return j == i ? x : a.in.col[j][rr]; }, tc, tp, tb,
+                     tbc);
+          cnt += tc;
+          sk += tc;
+          s2 += tp;
+          bal += tb;
+          balc += tbc;
+        } else if ((MODE & X_TAIL) && ftail) {
+          // The prefix ending in x has length k-2: its two-position pendant
+          // tail is counted here from the dense aggregates, not stored.
+          const uint32_t mp = P.tail_p == i ? x : a.in.col[P.tail_p][rr];
+          uint32_t ts, ten;
+          slice_of(g, P.tail_da, mp, P.label[P.k - 2], ts, ten);
+          long long ac, ad;
+          tail_agg(a, P, mp, ts, ten, ac, ad);
+          unsigned long long tc, tp, td;
+          tail_close(a, P, [&](uint32_t j) { return j == i ? x : a.in.col[j][rr]; }, mp, ts, ten,
+                     ac, ad, tc, tp, td);
+          cnt += tc;
+          sk += tc;
+          s2 += tp;
+          bal += 8ull + 4ull * (ten - ts) + 8ull * tp + 4ull * td;
+          balc += 8ull + 4ull * (ten - ts) + 8ull * tp;
+        } else if ((MODE & X_FUSED) && fused) {
+          const uint32_t kl = P.k - 1;
+          const uint32_t cs = P.cons[kl][0];
+          const uint32_t pos = cs & 0xFF, dir = cs >> 8;
+          const uint32_t y = pos == i ? x : a.in.col[pos][rr];
+          uint32_t s, en;
+          slice_of(g, dir, y, P.label[kl], s, en);
+          unsigned long long c1 = en - s;
+          bal += 8ull + 4ull * c1;
+          balc += 8ull;
+          for (uint32_t m = P.samelab[kl]; m; m &= m - 1) {
+            const uint32_t j = __ffs(m) - 1;
+            if ((P.guar[kl] >> j) & 1u) {
+              c1 -= 1;
             } else {
-              atomicOr(&a.ctr[C_ERR], (unsigned long long)ERR_OVERFLOW);
+              const uint32_t mj = j == i ? x : a.in.col[j][rr];
+              c1 -= in_slice_se(g, dir, y, s, en, mj, a.probe_min) ? 1ull : 0ull;
             }
           }
+          sk += c1;
+          cnt += c1;
         }
-      } else if (wr) {
-        atomicOr(&a.ctr[C_ERR], (unsigned long long)ERR_OVERFLOW);  // no table to append to
       }
-      // Emit mode: complete matches as rows in query-vertex order.
-      if constexpr ((MODE & X_EMIT) != 0) {
-      const bool em = ok && fin && !a.count_mode;
-      const uint32_t emm = __ballot_sync(FULL, em);
-      if (emm) {
-        const uint32_t leader = __ffs(emm) - 1;
+      if constexpr ((MODE & (X_WRITE | X_EMIT)) != 0) {
+        // compact what stays, in place
+        const bool keep = ok && !fused && !ftail && fin == ((MODE & X_EMIT) != 0);
+        const uint32_t km = __ballot_sync(FULL, keep);
+        if (keep) {
+          const uint32_t at = kept + __popc(km & lanemask_lt());
+          s_x[wid][at] = x;
+          s_r[wid][at] = rr;
+        }
+        kept += __popc(km);
+      } else if (ok && !fin && !fused && !ftail) {  // no table to append to
+        atomicOr(&a.ctr[C_ERR], (unsigned long long)ERR_OVERFLOW);
+      }
+    }
+    if constexpr ((MODE & (X_WRITE | X_EMIT)) != 0) {
+      __syncwarp();
+      if (kept) {
+        const uint32_t slot = (MODE & X_EMIT) ? uint32_t(C_EMIT) : a.out_slot;
+        const uint64_t cap = (MODE & X_EMIT) ? a.emit_cap : a.out_cap;
         unsigned long long base = 0;
-        if (lane == leader) base = atomicAdd(&a.ctr[C_EMIT], (unsigned long long)__popc(emm));
-        base = __shfl_sync(FULL, base, leader);
-        if (em) {
-          const unsigned long long idx = base + __popc(emm & lanemask_lt());
-          if (idx < a.emit_cap) {
-            const PlanDev& P = (MODE & X_ONE) ? s_plan : a.plans[q];
+        if (lane == 0) base = atomicAdd(&a.ctr[slot], (unsigned long long)kept);
+        base = __shfl_sync(FULL, base, 0);
+        if (base + kept > cap) {
+          // flagged once per warp; nothing is written past the table
+          if (lane == 0) atomicOr(&a.ctr[C_ERR], (unsigned long long)ERR_OVERFLOW);
+          full = true;
+          kept = base < cap ? uint32_t(cap - base) : 0u;
+        }
+        if constexpr ((MODE & X_EMIT) != 0) {
+          for (uint32_t v = lane; v < kept; v += 32) {
+            const uint32_t rr = s_r[wid][v];
             for (uint32_t j = 0; j < i; ++j)
-              a.emit_col[P.perm[j]][idx] = __ldg(g.globalid + a.in.col[j][r]);
-            a.emit_col[P.perm[i]][idx] = __ldg(g.globalid + x);
-          } else {
-            atomicOr(&a.ctr[C_ERR], (unsigned long long)ERR_OVERFLOW);
+              a.emit_col[s_plan.perm[j]][base + v] = __ldg(g.globalid + a.in.col[j][rr]);
+            a.emit_col[s_plan.perm[i]][base + v] = __ldg(g.globalid + s_x[wid][v]);
+          }
+        } else {
+          for (uint32_t v = lane; v < kept; v += 32) {
+            const uint32_t rr = s_r[wid][v];
+            for (uint32_t j = 0; j < i; ++j) a.out.col[j][base + v] = a.in.col[j][rr];
+            a.out.col[i][base + v] = s_x[wid][v];
+            if (!ONE && a.out.qid) a.out.qid[base + v] = query(rr);
           }
         }
       }
-      }  // X_EMIT
-      if constexpr ((MODE & X_WRITE) != 0) __syncthreads();  // s_wcnt / s_wbase reused next tile
     }
-    // Once per grab in a batch: fold the per-thread counts of a warp that holds
-    // one query (a single query's counts are folded once, at the end).
-    if (a.in.qid) acc_flush_warp(a, cnt_q, i, cnt, s1, sk, s2, false);
-  }  // grab loop
+    __syncwarp();  // the stage is filled again
+    staged = 0;
+  };
+
+  // A launch with fewer tiles than warps splits its tiles into parts of down
+  // to 64 elements, so that small levels still use every warp; a large one
+  // takes several tiles per grab of the work queue.  The first grab is by warp
+  // index, the queue serves the others.
+  const uint32_t nwarps = gridDim.x * (EXPAND_BLOCK / 32);
+  uint32_t split = 0;  // parts per tile, as a power of two
+  while ((EXPAND_TILE >> split) > 64 && (ntiles << (split + 1)) <= nwarps) ++split;
+  const uint32_t ntasks = ntiles << split;
+  const uint32_t part = EXPAND_TILE >> split;
+  uint32_t grab = a.grab;
+  if (!grab) {
+    grab = ntasks / (nwarps * 8);
+    grab = grab < 1 ? 1 : (grab > 16 ? 16 : grab);
+  }
+  const uint32_t rstep = i == 0 ? a.root_step : 1u;  // stride of the level-0 candidates
+  XRow* rows = s_rows[wid];
+  uint64_t gbase = uint64_t(blockIdx.x * (EXPAND_BLOCK / 32) + wid) * grab;
+  while (gbase < ntasks && !full) {
+    const uint32_t gend = uint32_t(min(gbase + grab, uint64_t(ntasks)));
+    for (uint32_t task = uint32_t(gbase); task < gend && !full; ++task) {
+      const uint32_t tile = task >> split;
+      uint64_t t = t0 + uint64_t(tile) * EXPAND_TILE + (task & ((1u << split) - 1)) * part;
+      const uint64_t te = min(t + part, t1);
+      if (t >= te) continue;
+      uint32_t r0 = __ldg(a.tile_row + tile);
+      const uint32_t rhi = __ldg(a.tile_row + tile + 1);
+      while (t < te && !full) {
+        if (r0 < rhi) r0 = find_row(a.woff, r0, rhi, t);
+        // Set up 32 rows, one per lane: consecutive ones, or, where more rows
+        // than elements are left (many are empty), the rows of the next 32
+        // elements.
+        const uint32_t left = uint32_t(te - t);
+        uint32_t row = min(r0 + lane, rhi);
+        bool mine = r0 + lane <= rhi;
+        if (rhi - r0 >= 32 && rhi - r0 > left) {
+          row = find_row(a.woff, r0, rhi, min(t + lane, te - 1));
+          const uint32_t prev = __shfl_up_sync(FULL, row, 1);
+          mine = lane == 0 || row != prev;
+        }
+        const uint64_t o0 = a.woff[row], o1 = a.woff[row + 1];
+        // the row's elements in this task, relative to t
+        const uint32_t beg = uint32_t(min(max(o0, t), te) - t);
+        const uint32_t end = uint32_t(min(max(o1, t), te) - t);
+        mine = mine && end > beg;
+        const uint32_t act = __ballot_sync(FULL, mine);
+        const uint32_t nrows = __popc(act);
+        __syncwarp();  // the previous rows are no longer read
+        if (mine) {
+          XRow R;
+          R.row = row;
+          R.q = query(row);
+          R.beg = beg;
+          R.end = end;
+          const PlanDev& P = plan(R.q);
+          const uint32_t lab = P.label[i], nc = P.ncons[i], ci = a.dci[row];
+          const uint32_t ds = a.dstart[row];
+          const uint64_t skip = t + beg - o0;  // elements of the row before the task
+          R.list = ci == DCI_BUCKET ? nullptr
+                                    : g.adj[P.cons[i][ci] >> 8] + int64_t(ds + skip) - beg;
+          R.v0 = ds + uint32_t(skip) * rstep - beg * rstep;
+          R.ci = ci;
+          R.m0 = R.m1 = FULL;
+          uint32_t m = P.samelab[i];
+          if (m) {
+            R.m0 = a.in.col[__ffs(m) - 1][row];
+            m &= m - 1;
+            if (m) R.m1 = a.in.col[__ffs(m) - 1][row];
+          }
+          R.p0 = R.p1 = nullptr;
+          R.len0 = R.len1 = 0;
+          uint32_t c = ci == 0 ? 1u : 0u;
+          if (c < nc) {
+            probe_of(a, P.cons[i][c], lab, row, R.p0, R.len0);
+            if (++c == ci) ++c;
+            if (c < nc) probe_of(a, P.cons[i][c], lab, row, R.p1, R.len1);
+          }
+          rows[__popc(act & lanemask_lt())] = R;
+        }
+        __syncwarp();
+        const uint32_t covered = rows[nrows - 1].end;  // elements these rows hold
+        const uint32_t mybeg = lane < nrows ? rows[lane].beg : FULL;
+        uint32_t before = 0;  // rows that begin before the next group
+        uint32_t x[XU], h[XU], xn[XU], hn[XU];
+        // Candidates and row slots of the elements from e0 on (past the last
+        // element: the last element's).
+        auto load = [&](uint32_t e0, uint32_t (&xx)[XU], uint32_t (&hh)[XU]) {
+#pragma unroll
+          for (int u = 0; u < XU; ++u) {
+            const uint32_t d = mybeg - (e0 + u * 32);
+            const uint32_t starts = __reduce_or_sync(FULL, d < 32 ? 1u << d : 0u);
+            hh[u] = before + __popc(starts & (lanemask_lt() | (1u << lane))) - 1;
+            before += __popc(starts);
+          }
+#pragma unroll
+          for (int u = 0; u < XU; ++u) {
+            const uint32_t e = min(e0 + u * 32 + lane, covered - 1);
+            const XRow& R = rows[hh[u]];
+            if (R.list) xx[u] = __ldg(R.list + e);
+            else xx[u] = R.v0 + e * rstep;
+          }
+        };
+        load(0, xn, hn);
+        for (uint32_t e0 = 0; e0 < covered && !full; e0 += 32 * XU) {
+          bool ok[XU];
+#pragma unroll
+          for (int u = 0; u < XU; ++u) {
+            x[u] = xn[u];
+            h[u] = hn[u];
+            ok[u] = e0 + u * 32 + lane < covered;
+          }
+          if (e0 + 32 * XU < covered) load(e0 + 32 * XU, xn, hn);
+          // (in a batch a row may have no such constraint)
+          auto probe_some = [&](const uint32_t* (&p)[XU], uint32_t (&len)[XU]) {
+            if constexpr (ONE) {
+              probe_all<XU>(p, len, x, ok);
+            } else {
+              bool in[XU];
+#pragma unroll
+              for (int u = 0; u < XU; ++u) {
+                in[u] = ok[u] && p[u];
+                if (!p[u]) p[u] = g.bucket_off;
+              }
+              bool res[XU];
+#pragma unroll
+              for (int u = 0; u < XU; ++u) res[u] = in[u];
+              probe_all<XU>(p, len, x, res);
+#pragma unroll
+              for (int u = 0; u < XU; ++u) ok[u] = in[u] ? res[u] : ok[u];
+            }
+          };
+          if (sames || !ONE) {
+#pragma unroll
+            for (int u = 0; u < XU; ++u)
+              ok[u] = ok[u] && x[u] != rows[h[u]].m0 && x[u] != rows[h[u]].m1;
+          }
+          if (others > 0 || !ONE) {
+            const uint32_t* p[XU];
+            uint32_t len[XU];
+#pragma unroll
+            for (int u = 0; u < XU; ++u) {
+              p[u] = rows[h[u]].p0;
+              len[u] = rows[h[u]].len0;
+            }
+            probe_some(p, len);
+          }
+          if (others > 1 || !ONE) {
+            const uint32_t* p[XU];
+            uint32_t len[XU];
+#pragma unroll
+            for (int u = 0; u < XU; ++u) {
+              p[u] = rows[h[u]].p1;
+              len[u] = rows[h[u]].len1;
+            }
+            probe_some(p, len);
+          }
+          // constraints and equal labels past the two that a row keeps, and the
+          // rare checks
+          if (others > 2 || sames > 2 || extra) {
+#pragma unroll
+            for (int u = 0; u < XU; ++u) {
+              if (!ok[u]) continue;
+              const XRow& R = rows[h[u]];
+              const PlanDev& P = plan(R.q);
+              uint32_t m = P.samelab[i];
+              m &= m - 1;
+              for (m &= m - 1; m && ok[u]; m &= m - 1)
+                ok[u] = a.in.col[__ffs(m) - 1][R.row] != x[u];
+              const uint32_t k0 = R.ci == 0 ? 1u : 0u, k1 = k0 + 1 == R.ci ? k0 + 2 : k0 + 1;
+              for (uint32_t c = k1 + 1; c < P.ncons[i] && ok[u]; ++c) {
+                if (c == R.ci) continue;
+                const uint32_t cs = P.cons[i][c];
+                ok[u] = in_slice(g, cs >> 8, a.in.col[cs & 0xFF][R.row], P.label[i], x[u],
+                                 a.probe_min);
+              }
+              // the lossy matrix filter drops level-0 candidates it rejects
+              if (i == 0 && a.root_keep && ok[u])
+                ok[u] = (__ldg(a.root_keep + (x[u] >> 5)) >> (x[u] & 31)) & 1u;
+              if (ok[u] && ((P.selfloop_mask >> i) & 1u)) ok[u] = has_self(g, x[u]);
+            }
+          }
+          if constexpr (STAGE) {
+#pragma unroll
+            for (int u = 0; u < XU; ++u) {
+              const uint32_t km = __ballot_sync(FULL, ok[u]);
+              if (ok[u]) {
+                const uint32_t w = staged + __popc(km & lanemask_lt());
+                s_x[wid][w] = x[u];
+                s_r[wid][w] = rows[h[u]].row;
+              }
+              staged += __popc(km);
+            }
+            // a task's survivors stay contiguous in the output
+            if (staged > XSTAGE - 32 * XU ||
+                (staged && e0 + 32 * XU >= covered && t + covered >= te))
+              flush();
+          } else {
+            uint32_t n = 0;
+#pragma unroll
+            for (int u = 0; u < XU; ++u) n += ok[u] ? 1u : 0u;
+            s1 += n;
+          }
+        }
+        t += covered;
+        if (r0 + 32 <= rhi && t < te) r0 = __shfl_sync(FULL, row, 31);
+      }
+      // In a batch: fold the per-thread counts of a warp that holds one query.
+      if (!ONE && a.in.qid) acc_flush_warp(a, cnt_q, i, cnt, s1, sk, s2, false);
+    }
+    if (lane == 0) gbase = atomicAdd(&a.ctr[a.tile_slot], (unsigned long long)grab);
+    gbase = __shfl_sync(FULL, gbase, 0) + uint64_t(nwarps) * grab;
+  }
+  if (ONE && a.count_mode && s_plan.k == i + 1) cnt = s1;  // complete matches
   acc_flush_warp(a, cnt_q, i, cnt, s1, sk, s2, true);
   bal = warp_sum(bal);
   balc = warp_sum(balc);
@@ -1062,10 +1329,10 @@ __global__ void __launch_bounds__(256) k_tile_rows_lane(StepArgs a) {
     T = a.seg_cap;
   }
   if (T == 0 || R == 0) return;
-  const uint64_t ntiles = (T + EXPAND_BLOCK - 1) / EXPAND_BLOCK;
+  const uint64_t ntiles = (T + EXPAND_TILE - 1) / EXPAND_TILE;
   for (uint64_t j = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; j <= ntiles;
        j += uint64_t(gridDim.x) * blockDim.x) {
-    uint64_t t = j * EXPAND_BLOCK;
+    uint64_t t = j * EXPAND_TILE;
     if (t > T - 1) t = T - 1;
     const_cast<uint32_t*>(a.tile_row)[j] = find_row(a.woff, 0, uint32_t(R - 1), t);
   }
@@ -1271,10 +1538,9 @@ static void launch_expand(const StepArgs& a, const PlanDev* plans, uint32_t npla
   case m:       \
     k_expand<m><<<grid, EXPAND_BLOCK, 0, st>>>(a); \
     break;
-    MG_X(0) MG_X(1) MG_X(2) MG_X(3) MG_X(4) MG_X(5) MG_X(6) MG_X(7)
-    MG_X(8) MG_X(9) MG_X(10) MG_X(11) MG_X(12) MG_X(13) MG_X(14) MG_X(15)
-    MG_X(16) MG_X(17) MG_X(18) MG_X(19) MG_X(20) MG_X(21) MG_X(22) MG_X(23)
-    MG_X(24) MG_X(25) MG_X(26) MG_X(27) MG_X(28) MG_X(29) MG_X(30) MG_X(31)
+    // emit runs hold one query, whose level either writes or emits
+    MG_X(0) MG_X(1) MG_X(4) MG_X(5) MG_X(8) MG_X(9) MG_X(12) MG_X(13)
+    MG_X(16) MG_X(17) MG_X(18) MG_X(20) MG_X(21) MG_X(24) MG_X(25) MG_X(28) MG_X(29)
 #undef MG_X
   }
 }
@@ -1507,7 +1773,7 @@ static int run_levels(DevGraph* dg, std::vector<PlanDev> plans, bool count_mode,
       MG_CK(cudaMemsetAsync(ws->ctr + C_OUT, 0, 8, st));
       for (uint64_t s0 = t0; s0 < t1; s0 += kSegment) {
         const uint64_t s1 = std::min(t1, s0 + kSegment);
-        const uint32_t ntiles = uint32_t((s1 - s0 + EXPAND_BLOCK - 1) / EXPAND_BLOCK);
+        const uint32_t ntiles = uint32_t((s1 - s0 + EXPAND_TILE - 1) / EXPAND_TILE);
         a.t0 = s0;
         a.t1 = s1;
         k_tile_rows<<<grid_for(uint64_t(ntiles) + 1, 256, sms * 16), 256, 0, st>>>(
@@ -1515,7 +1781,7 @@ static int run_levels(DevGraph* dg, std::vector<PlanDev> plans, bool count_mode,
         MG_CK(cudaMemsetAsync(ws->ctr + C_TILE, 0, 8, st));
         if (o.kernel_events) MG_CK(cudaEventRecord(ws->ev2, st));
         launch_expand(a, plans.data(), nq, count_mode, writes[lvl],
-                      grid_for(s1 - s0, EXPAND_BLOCK, sms * 8), st);
+                      grid_for(s1 - s0, 256, sms * 4), st);
         if (o.kernel_events) {
           MG_CK(cudaEventRecord(ws->ev3, st));
           MG_CK(cudaEventSynchronize(ws->ev3));
@@ -1894,7 +2160,7 @@ static int ensure_lanes(DevGraph* dg, uint32_t nl, uint64_t cap, uint32_t kmax) 
     const uint64_t ntiles = cap / WS_ROWS + 2;
     if ((rc = lane_alloc(ls, (void**)&L.status, ntiles * 8))) return rc;
     MG_CK(cudaMemset(L.status, 0, ntiles * 8));
-    if ((rc = lane_alloc(ls, (void**)&L.tile_row, (ls->seg_cap / EXPAND_BLOCK + 2) * 4))) return rc;
+    if ((rc = lane_alloc(ls, (void**)&L.tile_row, (ls->seg_cap / EXPAND_TILE + 2) * 4))) return rc;
     for (uint32_t l = 0; l < ls->kmax; ++l) {
       const uint64_t rows = l == 0 ? 1 : cap;
       for (uint32_t j = 0; j < l; ++j)
@@ -2425,7 +2691,7 @@ uint64_t noalloc_carve(unsigned char* base, uint64_t cap, uint32_t k, NoallocLay
   L->lvl_rows = reinterpret_cast<unsigned long long*>(take((MAXK + 1) * 8));
   L->plan = reinterpret_cast<PlanDev*>(take(sizeof(PlanDev)));
   L->bsum = reinterpret_cast<uint64_t*>(take((cap / SCAN_TILE + 2) * 8));
-  L->tile_row = reinterpret_cast<uint32_t*>(take((kNoallocSegment / EXPAND_BLOCK + 2) * 4));
+  L->tile_row = reinterpret_cast<uint32_t*>(take((kNoallocSegment / EXPAND_TILE + 2) * 4));
   for (uint32_t l = 0; l < k; ++l) {
     const uint64_t rows = l == 0 ? 1 : cap;
     for (uint32_t j = 0; j < l; ++j) L->col[l][j] = reinterpret_cast<uint32_t*>(take(rows * 4));
@@ -2572,14 +2838,14 @@ int noalloc_count(DevGraph* dg, const mg_csr_view* q, const mg_opts* opts, uint6
       const uint64_t seg = writes[lvl] ? std::min<uint64_t>(cap, kNoallocSegment) : kNoallocSegment;
       for (uint64_t s0 = t0; s0 < t1; s0 += seg) {
         const uint64_t s1 = std::min(t1, s0 + seg);
-        const uint32_t ntiles = uint32_t((s1 - s0 + EXPAND_BLOCK - 1) / EXPAND_BLOCK);
+        const uint32_t ntiles = uint32_t((s1 - s0 + EXPAND_TILE - 1) / EXPAND_TILE);
         a.t0 = s0;
         a.t1 = s1;
         k_tile_rows<<<grid_for(uint64_t(ntiles) + 1, 256, sms * 16), 256, 0, st>>>(
             L.woff[lvl], R[lvl], s0, s1, ntiles, L.tile_row);
         MG_CK(cudaMemsetAsync(L.ctr + C_TILE, 0, 8, st));
         launch_expand(a, &P, 1, true, writes[lvl],
-                      grid_for(s1 - s0, EXPAND_BLOCK, sms * 8), st);
+                      grid_for(s1 - s0, 256, sms * 4), st);
       }
       MG_CK(cudaGetLastError());
       cur[lvl] = t1;
