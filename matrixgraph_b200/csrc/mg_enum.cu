@@ -58,22 +58,22 @@ struct Workspace {
   int levels = 0;         // level tables allocated: 0..levels-1
   uint32_t* col[MAXK][MAXK] = {};
   uint32_t* qid[MAXK] = {};
-  uint32_t* work[MAXK] = {};
   uint64_t* woff[MAXK] = {};
   uint32_t* dstart[MAXK] = {};
   uint8_t* dci[MAXK] = {};
-  uint64_t* bsum = nullptr;
-  uint32_t bsum_cap = 0;
   uint32_t* tile_row = nullptr;  // first row of every expand tile of a segment
+  unsigned long long* status = nullptr;  // look-back words of the work/scan kernel
+  uint64_t status_bytes = 0;
+  uint32_t epoch = 0;
   uint32_t* root_keep = nullptr; // matrix-filter keep bits of the level-0 candidates
   uint64_t root_keep_words = 0;
   TailStore tails;
-  unsigned long long* ctr = nullptr;     // device counters
-  unsigned long long* h_ctr = nullptr;   // pinned mirror
-  unsigned long long* counts = nullptr;  // per query
-  unsigned long long* lvl_rows = nullptr;  // per query, MAXK + 1 prefix lengths
-  unsigned long long* q_elems = nullptr;   // per query, elements scheduled
-  uint32_t counts_cap = 0;
+  // Results of a call of nq queries, one block: counters (C_NUM), counts (nq),
+  // rows per prefix length (nq * (MAXK + 1)), elements scheduled (nq).
+  unsigned long long* res = nullptr;
+  uint32_t res_cap = 0;                  // queries
+  unsigned long long* h_res = nullptr;   // pinned mirror of one query's block
+  PlanDev* h_plan = nullptr;             // pinned, one plan
   PlanDev* plans = nullptr;
   uint32_t plans_cap = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr;
@@ -81,21 +81,25 @@ struct Workspace {
   uint64_t bytes = 0;
 };
 
-// Counter slots.
+// Counter slots.  A level's slots lie together, so that clearing everything
+// from a level on is one memset.
 enum : int {
   C_OUT = 0, C_BALG = 1, C_BALGC = 2, C_ERR = 3, C_EMIT = 4, C_TILE = 6,
-  // Lane pipeline (sizes live on the device), one slot per level l:
-  C_LOUT = 8,                // rows the expand of level l wrote (= rows of level l+1)
-  C_LTILE = C_LOUT + MAXK,   // work-queue position of the expand of level l
-  C_LT = C_LTILE + MAXK,     // candidate elements of level l
-  C_LSCAN = C_LT + MAXK,     // tile counter of the work/scan kernel of level l
-  C_NUM = C_LSCAN + MAXK
+  C_LVL = 8,                    // slots of level l from C_LVL + 4 * l on:
+  L_OUT = 0,                    // rows the expand of level l wrote (= rows of level l+1)
+  L_TILE = 1,                   // work-queue position of the expand of level l
+  L_T = 2,                      // candidate elements of level l
+  L_SCAN = 3,                   // tile counter of the work/scan kernel of level l
+  C_STOP = C_LVL + 4 * MAXK,    // 1 + the level whose elements passed their limit
+  C_NUM
 };
+constexpr int lvl_slot(int l, int what) { return C_LVL + 4 * l + what; }
 
 void free_workspace(Workspace* ws) {
   if (!ws) return;
   for (void* p : ws->allocs) cudaFree(p);
-  if (ws->h_ctr) cudaFreeHost(ws->h_ctr);
+  if (ws->h_res) cudaFreeHost(ws->h_res);
+  if (ws->h_plan) cudaFreeHost(ws->h_plan);
   if (ws->ev0) cudaEventDestroy(ws->ev0);
   if (ws->ev1) cudaEventDestroy(ws->ev1);
   if (ws->ev2) cudaEventDestroy(ws->ev2);
@@ -123,7 +127,12 @@ constexpr int SCAN_TILE = 4096;
 constexpr int EXPAND_BLOCK = 256;
 constexpr int EXPAND_TILE = 1024;                 // elements per expand tile
 constexpr int XSTAGE = 256;                       // survivors a warp stages at a time
-constexpr uint64_t kSegment = 1ull << 26;         // elements per expand launch
+constexpr uint64_t kSegment = 1ull << 30;         // elements per expand launch
+constexpr int WS_ROWS = 1024;                     // rows per work/scan tile (4 per thread)
+constexpr uint32_t kSpinLimit = 1u << 22;         // polls of a look-back wait (~0.3 s)
+constexpr uint32_t kEpochMax = (1u << 20) - 1;
+// Words of the result block of nq queries.
+constexpr uint64_t res_words(uint64_t nq) { return C_NUM + nq * (MAXK + 3); }
 
 static uint64_t level_row_bytes(int l) { return uint64_t(l) * 4 + 4 + 4 + 8 + 4 + 1; }
 
@@ -140,23 +149,23 @@ static int ensure_ws(DevGraph* dg, uint64_t cap, int levels, uint32_t nq) {
     ws->cap = cap;
     ws->rows0 = std::max<uint32_t>(nq, 1024);
     int rc;
-    if ((rc = ws_alloc(ws, (void**)&ws->ctr, C_NUM * 8))) return rc;
-    MG_CK(cudaMallocHost((void**)&ws->h_ctr, C_NUM * 8));
+    MG_CK(cudaMallocHost((void**)&ws->h_res, res_words(1) * 8));
+    MG_CK(cudaMallocHost((void**)&ws->h_plan, sizeof(PlanDev)));
     MG_CK(cudaEventCreate(&ws->ev0));
     MG_CK(cudaEventCreate(&ws->ev1));
     MG_CK(cudaEventCreate(&ws->ev2));
     MG_CK(cudaEventCreate(&ws->ev3));
-    ws->bsum_cap = uint32_t((std::max<uint64_t>(cap, ws->rows0) + SCAN_TILE - 1) / SCAN_TILE + 1);
-    if ((rc = ws_alloc(ws, (void**)&ws->bsum, uint64_t(ws->bsum_cap) * 8))) return rc;
+    const uint64_t status = (std::max<uint64_t>(cap, ws->rows0) / WS_ROWS + 2) * 8;
+    if ((rc = ws_alloc(ws, (void**)&ws->status, status))) return rc;
+    ws->status_bytes = status;
+    MG_CK(cudaMemsetAsync(ws->status, 0, status, dg->stream));
     if ((rc = ws_alloc(ws, (void**)&ws->tile_row, (kSegment / EXPAND_TILE + 2) * 4))) return rc;
   }
-  if (ws->counts_cap < nq) {
+  if (ws->res_cap < nq) {
     int rc;
-    if ((rc = ws_alloc(ws, (void**)&ws->counts, uint64_t(nq) * 8))) return rc;
-    if ((rc = ws_alloc(ws, (void**)&ws->lvl_rows, uint64_t(nq) * (MAXK + 1) * 8))) return rc;
-    if ((rc = ws_alloc(ws, (void**)&ws->q_elems, uint64_t(nq) * 8))) return rc;
+    if ((rc = ws_alloc(ws, (void**)&ws->res, res_words(nq) * 8))) return rc;
     if ((rc = ws_alloc(ws, (void**)&ws->plans, uint64_t(nq) * sizeof(PlanDev)))) return rc;
-    ws->counts_cap = ws->plans_cap = nq;
+    ws->res_cap = ws->plans_cap = nq;
   }
   for (int l = ws->levels; l < levels; ++l) {
     const uint64_t rows = l == 0 ? ws->rows0 : cap;
@@ -164,7 +173,6 @@ static int ensure_ws(DevGraph* dg, uint64_t cap, int levels, uint32_t nq) {
     for (int j = 0; j < l; ++j)
       if ((rc = ws_alloc(ws, (void**)&ws->col[l][j], rows * 4))) return rc;
     if ((rc = ws_alloc(ws, (void**)&ws->qid[l], rows * 4))) return rc;
-    if ((rc = ws_alloc(ws, (void**)&ws->work[l], rows * 4))) return rc;
     if ((rc = ws_alloc(ws, (void**)&ws->woff[l], (rows + 1) * 8))) return rc;
     if ((rc = ws_alloc(ws, (void**)&ws->dstart[l], rows * 4))) return rc;
     if ((rc = ws_alloc(ws, (void**)&ws->dci[l], rows))) return rc;
@@ -185,9 +193,8 @@ struct StepArgs {
   GraphDev g;
   const PlanDev* plans;
   uint32_t level;   // rows hold positions 0..level-1; position `level` is extended
-  uint32_t R;       // rows of the input table
+  uint32_t R;       // rows of the input table (level 0)
   TabPtrs in;
-  uint32_t* work;
   uint64_t* woff;
   uint32_t* dstart;
   uint8_t* dci;
@@ -201,14 +208,13 @@ struct StepArgs {
   unsigned long long q_budget;   // per-query element budget (0: none)
   uint32_t count_mode;
   uint32_t filters;
-  uint32_t stats;
   uint32_t nq;
   uint32_t* emit_col[MAXK];
   uint64_t emit_cap;
   uint64_t root_begin, root_end;  // level-0 candidate range (root_end 0: all)
   uint32_t root_step;             // level-0 stride inside the range (>= 1)
   uint32_t probe_min;             // shortest hub slice probed in the hub bitmap
-  const uint32_t* tile_row;        // first row of each tile of [t0, t1)
+  uint32_t* tile_row;              // first row of each tile of [t0, t1)
   uint32_t grab;   // expand tiles taken per work-queue grab
   const TailKey* tkeys;
   // Two-position pendant tails (tail_dense): counted while expanding
@@ -219,23 +225,28 @@ struct StepArgs {
   const unsigned long long* tdA;
   const unsigned long long* tdAD;
   unsigned long long* tdL;  // lazily filled aggregates of non-hub vertices
-  // Lane pipeline: row and element counts come from the counters (C_LOUT,
-  // C_LT), the expand's queue and output use the per-level slots, and no
-  // host value of R, t0 or t1 is read.
-  uint32_t lane;
+  // Level 0 of a single query is one row that needs no table: its candidates
+  // are root_first + e * root_step, e < T0.
+  uint64_t T0;
+  uint32_t root_first;
+  // Sizes on the device: row and element counts come from the level's counter
+  // slots and no host value of R, t0 or t1 is read.  lane: a batch lane, whose
+  // query is counted again when it does not fit.
+  uint32_t dev, lane;
   uint32_t out_slot, tile_slot;  // counter slots of the output rows / work queue
-  uint64_t cap_rows;             // rows of a lane's level table
-  uint64_t seg_cap;              // elements one lane expand launch can tile
+  uint64_t cap_rows;             // rows of a level table
+  uint64_t t_limit;              // a level with more elements stops the walk
+  uint64_t seg_cap;              // elements the tile-row table covers
   unsigned long long* scan_status;  // look-back words of the work/scan kernel
   uint32_t spin_limit;           // bounded device waits (iterations)
   const uint32_t* root_keep;     // level-0 candidates kept by the matrix filter
                                  // (bit per vertex; nullptr: no filter)
 };
 
-// Rows of the input table of a lane launch at level a.level.
-__device__ __forceinline__ uint64_t lane_rows(const StepArgs& a) {
-  if (a.level == 0) return 1;
-  const uint64_t r = a.ctr[C_LOUT + a.level - 1];
+// Rows of the input table of a launch with sizes on the device.
+__device__ __forceinline__ uint64_t dev_rows(const StepArgs& a) {
+  if (a.level == 0) return a.R;
+  const uint64_t r = a.ctr[lvl_slot(int(a.level) - 1, L_OUT)];
   return r < a.cap_rows ? r : a.cap_rows;
 }
 
@@ -528,9 +539,6 @@ __device__ __forceinline__ void star_close(const StepArgs& a, const PlanDev& P, 
   balc = 8ull + 4ull * (ea - sa) + A * 8ull;
 }
 
-// Work kernel: per row, the driving slice (shortest backward slice, or the
-// label bucket for a position without backward neighbours) and the
-// algorithmic-byte charge of extending the row.
 // Driving slice of table row r at position a.level: its length (the row's
 // candidate elements, 0 when nothing is to be expanded), start and constraint
 // index (DCI_BUCKET: the label bucket), and the row's algorithmic-byte
@@ -583,33 +591,6 @@ __device__ __forceinline__ uint32_t row_work(const StepArgs& a, const PlanDev& P
   return best;
 }
 
-__global__ void __launch_bounds__(256) k_work(StepArgs a) {
-  unsigned long long bal = 0, balc = 0;
-  // Contiguous rows per block: rows of one query stay together.
-  const uint64_t per = ((a.R + gridDim.x - 1) / gridDim.x + blockDim.x - 1) / blockDim.x *
-                       blockDim.x;
-  const uint64_t r_end = min(uint64_t(a.R), (uint64_t(blockIdx.x) + 1) * per);
-  for (uint64_t r = blockIdx.x * per + threadIdx.x; r < r_end; r += blockDim.x) {
-    const uint32_t q = a.in.qid ? a.in.qid[r] : 0u;
-    const PlanDev& P = a.plans[q];
-    uint32_t bs;
-    uint8_t bci;
-    unsigned long long ch, chc;
-    a.work[r] = row_work(a, P, r, q, bs, bci, ch, chc);
-    a.dstart[r] = bs;
-    a.dci[r] = bci;
-    bal += ch;
-    balc += chc;
-  }
-  bal = warp_sum(bal);
-  balc = warp_sum(balc);
-  if ((threadIdx.x & 31) == 0 && (bal | balc)) {
-    atomicAdd(&a.ctr[C_BALG], bal);
-    atomicAdd(&a.ctr[C_BALGC], balc);
-  }
-}
-
-// Scan of the per-row driving lengths into 64-bit element offsets.
 __device__ __forceinline__ unsigned long long block_exclusive_scan(unsigned long long v,
                                                                    unsigned long long* total) {
   __shared__ unsigned long long wsum[33];
@@ -833,10 +814,11 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
   const GraphDev& g = a.g;
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   uint64_t t0 = a.t0, t1 = a.t1;
-  if (a.lane) {  // lane pipeline: this level's elements, capped (k_tile_rows_lane flags it)
+  if (a.dev) {
+    if (a.ctr[C_STOP]) return;
     t0 = 0;
-    t1 = a.ctr[C_LT + i];
-    if (t1 > a.seg_cap) t1 = a.seg_cap;
+    t1 = ONE && i == 0 ? a.T0 : a.ctr[lvl_slot(int(i), L_T)];
+    if (t1 > a.seg_cap) return;  // flagged by the work/scan kernel
   }
   const uint64_t span = t1 - t0;
   const uint32_t ntiles = uint32_t((span + EXPAND_TILE - 1) / EXPAND_TILE);
@@ -1012,6 +994,7 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
     grab = grab < 1 ? 1 : (grab > 16 ? 16 : grab);
   }
   const uint32_t rstep = i == 0 ? a.root_step : 1u;  // stride of the level-0 candidates
+  const bool root = ONE && i == 0;                   // one row, no table
   XRow* rows = s_rows[wid];
   uint64_t gbase = uint64_t(blockIdx.x * (EXPAND_BLOCK / 32) + wid) * grab;
   while (gbase < ntasks && !full) {
@@ -1021,8 +1004,8 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
       uint64_t t = t0 + uint64_t(tile) * EXPAND_TILE + (task & ((1u << split) - 1)) * part;
       const uint64_t te = min(t + part, t1);
       if (t >= te) continue;
-      uint32_t r0 = __ldg(a.tile_row + tile);
-      const uint32_t rhi = __ldg(a.tile_row + tile + 1);
+      uint32_t r0 = root ? 0u : __ldg(a.tile_row + tile);
+      const uint32_t rhi = root ? 0u : __ldg(a.tile_row + tile + 1);
       while (t < te && !full) {
         if (r0 < rhi) r0 = find_row(a.woff, r0, rhi, t);
         // Set up 32 rows, one per lane: consecutive ones, or, where more rows
@@ -1036,7 +1019,7 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
           const uint32_t prev = __shfl_up_sync(FULL, row, 1);
           mine = lane == 0 || row != prev;
         }
-        const uint64_t o0 = a.woff[row], o1 = a.woff[row + 1];
+        const uint64_t o0 = root ? 0ull : a.woff[row], o1 = root ? a.T0 : a.woff[row + 1];
         // the row's elements in this task, relative to t
         const uint32_t beg = uint32_t(min(max(o0, t), te) - t);
         const uint32_t end = uint32_t(min(max(o1, t), te) - t);
@@ -1051,8 +1034,9 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
           R.beg = beg;
           R.end = end;
           const PlanDev& P = plan(R.q);
-          const uint32_t lab = P.label[i], nc = P.ncons[i], ci = a.dci[row];
-          const uint32_t ds = a.dstart[row];
+          const uint32_t lab = P.label[i], nc = P.ncons[i];
+          const uint32_t ci = root ? uint32_t(DCI_BUCKET) : uint32_t(a.dci[row]);
+          const uint32_t ds = root ? a.root_first : a.dstart[row];
           const uint64_t skip = t + beg - o0;  // elements of the row before the task
           R.list = ci == DCI_BUCKET ? nullptr
                                     : g.adj[P.cons[i][ci] >> 8] + int64_t(ds + skip) - beg;
@@ -1218,11 +1202,10 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
   }
 }
 
-// ---- lane pipeline kernels --------------------------------------------------
+// ---- work and scan -----------------------------------------------------------
 // Look-back words of the single-pass work/scan: [epoch:20 | status:2 | value:42].
 constexpr int LB_VALUE_BITS = 42;
 constexpr unsigned long long LB_AGG = 1, LB_INC = 2;
-constexpr int WS_ROWS = 1024;  // rows per work/scan tile (4 per thread)
 
 __device__ __forceinline__ unsigned long long lb_word(uint32_t epoch, unsigned long long st,
                                                       unsigned long long v) {
@@ -1230,22 +1213,65 @@ __device__ __forceinline__ unsigned long long lb_word(uint32_t epoch, unsigned l
          (v & ((1ull << LB_VALUE_BITS) - 1));
 }
 
-// Work + scan of one lane level in one pass: tiles of WS_ROWS rows are taken
-// in launch order from a counter; each computes its rows' driving slices,
-// publishes its sum, and adds the sums of the tiles before it (decoupled
-// look-back: a predecessor's inclusive prefix, or its sum and keep looking).
-// A tile only ever waits for tiles claimed before it, whose blocks are
-// running, and every wait gives up after spin_limit polls (ERR_TIMEOUT).
-// The last tile writes the level's element total to woff[R] and C_LT.
+// Sum of the tiles before `tile` (decoupled look-back by one warp, 32
+// predecessors at a time: back to the nearest inclusive prefix).  A tile only
+// waits for tiles claimed before it, whose blocks are running; every wait gives
+// up after spin_limit polls (ERR_TIMEOUT).
+__device__ __forceinline__ unsigned long long look_back(const StepArgs& a, uint32_t epoch,
+                                                        uint64_t tile) {
+  const uint32_t lane = threadIdx.x & 31;
+  unsigned long long prefix = 0;
+  for (int64_t t = int64_t(tile) - 1; t >= 0; t -= 32) {
+    const int64_t at = t - int64_t(lane);
+    unsigned long long w = lb_word(epoch, LB_INC, 0);  // before the first tile
+    if (at >= 0) {
+      volatile unsigned long long* st = a.scan_status + at;
+      uint32_t spins = 0;
+      for (;;) {
+        w = *st;
+        if ((w >> (LB_VALUE_BITS + 2)) == epoch && ((w >> LB_VALUE_BITS) & 3ull)) break;
+        if (++spins > a.spin_limit) {
+          atomicOr(&a.ctr[C_ERR], (unsigned long long)ERR_TIMEOUT);
+          w = lb_word(epoch, LB_INC, 0);
+          break;
+        }
+        __nanosleep(32);
+      }
+    }
+    __syncwarp();
+    const uint32_t inc = __ballot_sync(FULL, ((w >> LB_VALUE_BITS) & 3ull) == LB_INC);
+    const uint32_t upto = inc ? __ffs(inc) - 1 : 31u;
+    unsigned long long v = lane <= upto ? w & ((1ull << LB_VALUE_BITS) - 1) : 0ull;
+    v = warp_sum(v);
+    prefix += __shfl_sync(FULL, v, 0);
+    if (inc) break;
+  }
+  return prefix;
+}
+
+// Work and scan of one level in one pass: tiles of WS_ROWS rows are taken in
+// launch order from a counter; each computes its rows' driving slices (the
+// shortest backward slice, or the label bucket for a position without backward
+// neighbours) and their algorithmic-byte charge, publishes its sum, adds the
+// sums of the tiles before it, and writes its rows' element offsets and the
+// first row of every expand tile that begins among its elements.  The last
+// tile writes the level's element total; a total past t_limit (or, on a lane,
+// past seg_cap) stops the walk before the level is expanded.
+//
+// One launch and one pass over the rows in place of a work kernel, three scan
+// kernels and a tile-row search, with no size returned to the host.
 __global__ void __launch_bounds__(256) k_work_scan(StepArgs a, uint32_t epoch) {
   const uint32_t i = a.level;
-  const uint64_t R = lane_rows(a);
+  if (a.ctr[C_STOP] || a.ctr[C_ERR]) return;
+  const uint64_t R = dev_rows(a);
   const uint64_t ntiles = (R + WS_ROWS - 1) / WS_ROWS;
   unsigned long long bal = 0, balc = 0;
   __shared__ uint32_t s_tile;
   __shared__ unsigned long long s_prefix;
+  __shared__ unsigned long long s_off[WS_ROWS];
   for (;;) {
-    if (threadIdx.x == 0) s_tile = uint32_t(atomicAdd(&a.ctr[C_LSCAN + i], 1ull));
+    if (threadIdx.x == 0)
+      s_tile = uint32_t(atomicAdd(&a.ctr[lvl_slot(int(i), L_SCAN)], 1ull));
     __syncthreads();
     const uint64_t tile = s_tile;
     __syncthreads();
@@ -1256,85 +1282,70 @@ __global__ void __launch_bounds__(256) k_work_scan(StepArgs a, uint32_t epoch) {
       const uint64_t r = base + j;
       v[j] = 0;
       if (r < R) {
-        const PlanDev& P = a.plans[0];
+        const uint32_t q = a.in.qid ? a.in.qid[r] : 0u;
         uint32_t bs;
         uint8_t bci;
         unsigned long long ch, chc;
-        const uint32_t w = row_work(a, P, r, 0, bs, bci, ch, chc);
-        a.work[r] = w;
+        v[j] = row_work(a, a.plans[q], r, q, bs, bci, ch, chc);
         a.dstart[r] = bs;
         a.dci[r] = bci;
         bal += ch;
         balc += chc;
-        v[j] = w;
-        sum += w;
+        sum += v[j];
       }
     }
     unsigned long long tot;
     const unsigned long long ex = block_exclusive_scan(sum, &tot);
-    if (threadIdx.x == 0) {
-      unsigned long long* st = a.scan_status;
-      atomicExch(st + tile, lb_word(epoch, tile == 0 ? LB_INC : LB_AGG, tot));
-      unsigned long long prefix = 0;
-      for (int64_t t = int64_t(tile) - 1; t >= 0; --t) {
-        unsigned long long w = 0;
-        uint32_t spins = 0;
-        for (;;) {
-          w = atomicAdd(st + t, 0ull);
-          if ((w >> (LB_VALUE_BITS + 2)) == epoch && ((w >> LB_VALUE_BITS) & 3ull)) break;
-          if (++spins > a.spin_limit) {
-            atomicOr(&a.ctr[C_ERR], (unsigned long long)ERR_TIMEOUT);
-            w = lb_word(epoch, LB_INC, 0);
-            break;
-          }
-          __nanosleep(64);
+    if (threadIdx.x < 32) {
+      if (threadIdx.x == 0)
+        atomicExch(a.scan_status + tile, lb_word(epoch, tile == 0 ? LB_INC : LB_AGG, tot));
+      const unsigned long long prefix = look_back(a, epoch, tile);
+      if (threadIdx.x == 0) {
+        if (tile > 0) atomicExch(a.scan_status + tile, lb_word(epoch, LB_INC, prefix + tot));
+        if (prefix + tot >= (1ull << LB_VALUE_BITS))
+          atomicOr(&a.ctr[C_ERR], (unsigned long long)ERR_OVERFLOW);
+        s_prefix = prefix;
+        if (tile + 1 == ntiles) {
+          const unsigned long long T = prefix + tot;
+          a.woff[R] = T;
+          a.ctr[lvl_slot(int(i), L_T)] = T;
+          if (T <= a.seg_cap)
+            a.tile_row[(T + EXPAND_TILE - 1) / EXPAND_TILE] = uint32_t(R - 1);
+          else if (a.lane)
+            atomicOr(&a.ctr[C_ERR], (unsigned long long)ERR_OVERFLOW);
+          if (!a.lane && T > a.t_limit) a.ctr[C_STOP] = i + 1;
         }
-        prefix += w & ((1ull << LB_VALUE_BITS) - 1);
-        if (((w >> LB_VALUE_BITS) & 3ull) == LB_INC) break;
-      }
-      if (tile > 0) atomicExch(st + tile, lb_word(epoch, LB_INC, prefix + tot));
-      if (prefix + tot >= (1ull << LB_VALUE_BITS))
-        atomicOr(&a.ctr[C_ERR], (unsigned long long)ERR_OVERFLOW);
-      s_prefix = prefix;
-      if (tile + 1 == ntiles) {
-        a.woff[R] = prefix + tot;
-        a.ctr[C_LT + i] = prefix + tot;
       }
     }
-    __syncthreads();
-    unsigned long long o = s_prefix + ex;
+    unsigned long long o = ex;
     for (int j = 0; j < 4; ++j) {
-      const uint64_t r = base + j;
-      if (r < R) a.woff[r] = o;
+      s_off[threadIdx.x * 4 + j] = o;
       o += v[j];
     }
+    __syncthreads();
+    const unsigned long long prefix = s_prefix;
+    for (uint32_t x = threadIdx.x; x < WS_ROWS; x += 256) {
+      const uint64_t r = tile * WS_ROWS + x;
+      if (r < R) a.woff[r] = prefix + s_off[x];
+    }
+    // expand tiles that begin among these rows' elements: the last row that
+    // starts at or before their first element
+    const uint64_t j1 = (prefix + tot + EXPAND_TILE - 1) / EXPAND_TILE;
+    for (uint64_t j = (prefix + EXPAND_TILE - 1) / EXPAND_TILE + threadIdx.x; j < j1; j += 256) {
+      if (j * EXPAND_TILE >= a.seg_cap) break;
+      const unsigned long long t = j * EXPAND_TILE - prefix;
+      uint32_t lo = 0;
+      for (uint32_t d = WS_ROWS / 2; d > 0; d >>= 1)
+        if (s_off[lo + d] <= t) lo += d;
+      a.tile_row[j] = uint32_t(min(tile * WS_ROWS + lo, R - 1));
+    }
+    __syncthreads();  // s_off and s_prefix are written again
   }
   bal = warp_sum(bal);
   balc = warp_sum(balc);
   if ((threadIdx.x & 31) == 0 && (bal | balc)) {
     atomicAdd(&a.ctr[C_BALG], bal);
     atomicAdd(&a.ctr[C_BALGC], balc);
-  }
-}
-
-// First row of every expand tile of a lane level (the element total is read
-// from the device; a total beyond the lane's tile buffer is flagged and the
-// query is re-run on the chunked path).
-__global__ void __launch_bounds__(256) k_tile_rows_lane(StepArgs a) {
-  const uint64_t R = lane_rows(a);
-  uint64_t T = a.ctr[C_LT + a.level];
-  if (T > a.seg_cap) {
-    if (blockIdx.x == 0 && threadIdx.x == 0)
-      atomicOr(&a.ctr[C_ERR], (unsigned long long)ERR_OVERFLOW);
-    T = a.seg_cap;
-  }
-  if (T == 0 || R == 0) return;
-  const uint64_t ntiles = (T + EXPAND_TILE - 1) / EXPAND_TILE;
-  for (uint64_t j = blockIdx.x * uint64_t(blockDim.x) + threadIdx.x; j <= ntiles;
-       j += uint64_t(gridDim.x) * blockDim.x) {
-    uint64_t t = j * EXPAND_TILE;
-    if (t > T - 1) t = T - 1;
-    const_cast<uint32_t*>(a.tile_row)[j] = find_row(a.woff, 0, uint32_t(R - 1), t);
   }
 }
 
@@ -1345,7 +1356,7 @@ __global__ void __launch_bounds__(256) k_tile_rows_lane(StepArgs a) {
 __global__ void k_lane_done(unsigned long long* ctr, unsigned long long* counts,
                             unsigned long long* lvl, unsigned long long* qel,
                             unsigned long long budget, uint32_t q,
-                            unsigned long long* out_counts, unsigned long long* out_lvl,
+                            unsigned long long next_elems, unsigned long long* out_counts, unsigned long long* out_lvl,
                             unsigned long long* out_err, unsigned long long* out_balg) {
   const uint32_t t = threadIdx.x;
   if (t <= MAXK) {
@@ -1359,13 +1370,15 @@ __global__ void k_lane_done(unsigned long long* ctr, unsigned long long* counts,
     out_balg[2ull * q] = ctr[C_BALG];
     out_balg[2ull * q + 1] = ctr[C_BALGC];
     counts[0] = 0;
-    qel[0] = 0;
+    qel[0] = next_elems;  // the next query's level-0 candidates
     ctr[C_ERR] = 0;
     ctr[C_BALG] = 0;
     ctr[C_BALGC] = 0;
   }
-  for (int c = C_LOUT + int(t); c < C_NUM; c += 32) ctr[c] = 0;
+  for (int c = C_LVL + int(t); c < C_NUM; c += 32) ctr[c] = 0;
 }
+
+__global__ void k_set_u64(unsigned long long* p, unsigned long long v) { *p = v; }
 
 __global__ void k_iota(uint32_t* p, uint32_t n) {
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
@@ -1516,13 +1529,12 @@ static inline unsigned grid_for(uint64_t items, unsigned block, unsigned cap) {
   return unsigned(std::max<uint64_t>(1, std::min<uint64_t>(g, cap)));
 }
 
-// Launches the expand kernel specialised for what the rows of level `lvl`
-// can need: a write when the level writes a table, emit rows in emit mode,
-// in-place closing of a last position or of a pendant tail when a plan has
-// one right after this position.
-static void launch_expand(const StepArgs& a, const PlanDev* plans, uint32_t nplans,
-                          bool count_mode, bool writes, unsigned grid, cudaStream_t st) {
-  const uint32_t i = a.level;
+// Shape of the expand kernel for what the rows of level i can need: a write
+// when the level writes a table, emit rows in emit mode, in-place closing of a
+// last position or of a pendant tail when a plan has one right after this
+// position.
+static int expand_mode(const StepArgs& a, uint32_t i, const PlanDev* plans, uint32_t nplans,
+                       bool count_mode, bool writes) {
   bool fused = false, tail = false, emit = false;
   for (uint32_t pi = 0; pi < nplans; ++pi) {
     const PlanDev& p = plans[pi];
@@ -1530,9 +1542,11 @@ static void launch_expand(const StepArgs& a, const PlanDev* plans, uint32_t npla
     if (((a.tail_dense && p.tail2) || (a.star && p.star2)) && p.k == i + 3) tail = true;
     if (!count_mode && p.k == i + 1) emit = true;
   }
-  const bool one = nplans == 1 && a.in.qid == nullptr;
-  const int mode = (writes ? X_WRITE : 0) | (emit ? X_EMIT : 0) | (fused ? X_FUSED : 0) |
-                   (tail ? X_TAIL : 0) | (one ? X_ONE : 0);
+  return (writes ? X_WRITE : 0) | (emit ? X_EMIT : 0) | (fused ? X_FUSED : 0) |
+         (tail ? X_TAIL : 0) | (nplans == 1 ? X_ONE : 0);
+}
+
+static void launch_expand(const StepArgs& a, int mode, unsigned grid, cudaStream_t st) {
   switch (mode) {
 #define MG_X(m) \
   case m:       \
@@ -1606,6 +1620,252 @@ static int setup_tails(DevGraph* dg, std::vector<PlanDev>& plans, TailStore& ts,
   return MG_OK;
 }
 
+// Last level a plan expands in count mode: k-1, or k-2 when the last
+// position is closed in place, or k-3 when a pendant tail is closed from
+// dense aggregates.
+static int last_level(const PlanDev& P, bool dense, bool star) {
+  int l = int(P.k) - 1;
+  if (P.k >= 2 && P.last_o1) l = int(P.k) - 2;
+  if ((dense && P.tail2) || (star && P.star2)) l = int(P.k) - 3;
+  return l;
+}
+
+// Candidates of level 0 (see row_work): the label bucket of the first position,
+// or the part of it that the options name.
+static uint64_t root_range(const DevGraph* dg, const PlanDev& P, const StepArgs& a,
+                           uint32_t* first) {
+  const uint64_t b0 = dg->h_bucket_off[P.label[0]];
+  const uint64_t size = dg->h_bucket_off[P.label[0] + 1] - b0;
+  *first = uint32_t(b0);
+  if (P.zero) return 0;
+  if (!a.root_end) return size;
+  const uint64_t rb = std::min<uint64_t>(a.root_begin, size), re = std::min(a.root_end, size);
+  *first = uint32_t(b0 + rb);
+  return re > rb ? (re - rb + a.root_step - 1) / a.root_step : 0;
+}
+
+// Algorithmic bytes of a level-0 candidate: its id, degree and label bits.
+static uint64_t root_charge(const DevGraph* dg) { return 12ull + 4ull * dg->g.W; }
+
+// Upper bound of the elements of a row of level l.
+static uint64_t row_bound(const DevGraph* dg, const PlanDev* plans, uint32_t nq, int l) {
+  for (uint32_t q = 0; q < nq; ++q)
+    if (uint32_t(l) < plans[q].k && plans[q].ncons[l] == 0) return dg->g.n;
+  return dg->g.symmetric ? std::max(dg->info.max_degree, 1u) : dg->g.n;
+}
+
+static uint64_t bounded_product(uint64_t a, uint64_t b) {
+  return b && a > (1ull << 40) / b ? 1ull << 40 : a * b;
+}
+
+// Scratch of a walk over the levels.
+struct WalkBufs {
+  uint64_t cap = 0;  // rows per level table
+  uint32_t* (*col)[MAXK] = nullptr;
+  uint32_t** qid = nullptr;  // nullptr: single queries only
+  uint64_t** woff = nullptr;
+  uint32_t** dstart = nullptr;
+  uint8_t** dci = nullptr;
+  uint32_t* tile_row = nullptr;
+  uint64_t seg = 0;  // elements that tile_row covers
+  unsigned long long* status = nullptr;
+  uint64_t status_bytes = 0;
+  uint32_t* epoch = nullptr;
+  unsigned long long* res = nullptr;    // device result block, zeroed
+  unsigned long long* h_res = nullptr;  // host mirror: one query's block, or the counters
+  cudaEvent_t done = nullptr, ev2 = nullptr, ev3 = nullptr;
+};
+
+// Depth-first walk over the level tables.  From a level whose rows are known,
+// all deeper levels are queued at once with their sizes on the device (work/scan
+// and expand per level, no host in between): a level with more elements than
+// its table or the budget allows stops the chain (C_STOP), and the host goes on
+// from there, one chunk of that level at a time, each followed by the chain of
+// the levels below.  So a query that fits its tables costs one synchronisation,
+// and a larger one costs one per chunk.
+//
+// With a work kernel, three scan kernels, a tile-row kernel and two host waits
+// per level, a labelled 4-cycle on a 10,000-vertex graph took 24 launches and
+// 312 us; it takes 7 and 120 us.  R-MAT scale 22, 4-clique: 7.3 -> 6.9 ms; 48
+// budgeted runs on scale 20: 65 -> 19 ms (a run past its budget on a batch
+// lane is not counted again); 256 single queries 128 -> 105 ms.
+static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool count_mode,
+                       const mg_opts& o, StepArgs a, WalkBufs& B, RunResult* res) {
+  const bool one = nq == 1;
+  const unsigned sms = dg->sms;
+  cudaStream_t st = dg->stream;
+  const bool dense = a.tail_dense != 0, star = a.star != 0;
+  // writes[l]: some query can append rows to the level-(l+1) table.
+  bool writes[MAXK] = {};
+  int last = -1;
+  for (uint32_t q = 0; q < nq; ++q) {
+    const PlanDev& p = plans[q];
+    if (p.zero) continue;
+    const int lp = count_mode ? last_level(p, dense, star) : int(p.k) - 1;
+    for (int l = 0; l < lp; ++l) writes[l] = true;
+    last = std::max(last, lp);
+  }
+  int mode[MAXK] = {};
+  uint64_t widest[MAXK] = {};  // elements of a row, at most
+  for (int l = 0; l <= last; ++l) {
+    mode[l] = expand_mode(a, uint32_t(l), plans, nq, count_mode, writes[l]);
+    widest[l] = row_bound(dg, plans, nq, l);
+  }
+  a.ctr = B.res;
+  a.counts = B.res + C_NUM;
+  a.lvl_rows = a.counts + nq;
+  a.q_elems = a.lvl_rows + uint64_t(nq) * (MAXK + 1);
+  a.cap_rows = B.cap;
+  a.seg_cap = B.seg;
+  a.tile_row = B.tile_row;
+  a.scan_status = B.status;
+  a.spin_limit = kSpinLimit;
+  a.R = nq;
+  unsigned long long* h = B.h_res;
+  uint64_t T[MAXK] = {}, cur[MAXK] = {}, elements = 0;
+  uint32_t R[MAXK] = {};
+  R[0] = nq;
+  int rc;
+
+  auto set_level = [&](int l) {
+    a.level = uint32_t(l);
+    auto tab = [&](int x) {
+      TabPtrs t{};
+      for (int j = 0; j < x; ++j) t.col[j] = B.col[x][j];
+      t.qid = one ? nullptr : B.qid[x];
+      return t;
+    };
+    a.in = tab(l);
+    a.woff = B.woff[l];
+    a.dstart = B.dstart[l];
+    a.dci = B.dci[l];
+    a.out = writes[l] ? tab(l + 1) : TabPtrs{};
+    a.out_cap = writes[l] ? B.cap : 0;
+    a.out_slot = lvl_slot(l, L_OUT);
+    a.tile_slot = lvl_slot(l, L_TILE);
+  };
+  auto expand = [&](int l, uint64_t bound) -> int {
+    if (o.kernel_events && B.ev2) MG_CK(cudaEventRecord(B.ev2, st));
+    launch_expand(a, mode[l], grid_for(bound, 256, sms * 4), st);
+    if (o.kernel_events && B.ev2) {
+      MG_CK(cudaEventRecord(B.ev3, st));
+      MG_CK(cudaEventSynchronize(B.ev3));
+      float kms = 0;
+      MG_CK(cudaEventElapsedTime(&kms, B.ev2, B.ev3));
+      res->expand_ms += kms;
+    }
+    res->expand_launches++;
+    res->launches++;
+    return MG_OK;
+  };
+  auto refuse = [&]() {
+    cudaStreamSynchronize(st);
+    return set_error(MG_E_LIMIT, "work budget of %llu candidate elements exceeded",
+                     (unsigned long long)o.max_elements);
+  };
+  // Queues levels l0..last, whose first table has at most `rows` rows.
+  auto descend = [&](int l0, uint64_t rows) -> int {
+    a.dev = 1;
+    for (int l = l0; l <= last; ++l) {
+      set_level(l);
+      a.t_limit = writes[l] ? std::min(B.cap, B.seg) : B.seg;
+      if (one && o.max_elements) a.t_limit = std::min(a.t_limit, o.max_elements - elements);
+      if (++*B.epoch > kEpochMax) {
+        MG_CK(cudaMemsetAsync(B.status, 0, B.status_bytes, st));
+        *B.epoch = 1;
+      }
+      k_work_scan<<<grid_for(rows, WS_ROWS, sms * 4), 256, 0, st>>>(a, *B.epoch);
+      res->launches++;
+      const uint64_t bound = std::min(bounded_product(rows, widest[l]), a.t_limit);
+      if (int r = expand(l, bound)) return r;
+      rows = std::min(bound, B.cap);
+    }
+    return MG_OK;
+  };
+  // Waits for what is queued and takes over the sizes of levels l0..last, which
+  // ran to their end, or up to the one that stopped (returned in *stop).
+  auto settle = [&](int l0, int* stop) -> int {
+    if (B.done) MG_CK(cudaEventRecord(B.done, st));
+    MG_CK(cudaMemcpyAsync(h, B.res, (one ? res_words(1) : C_NUM) * 8, cudaMemcpyDeviceToHost, st));
+    MG_CK(cudaStreamSynchronize(st));
+    MG_CK(cudaGetLastError());
+    if (h[C_ERR] & ERR_TIMEOUT) return set_error(MG_E_TIMEOUT, "a device wait gave up");
+    if (h[C_ERR] & ERR_OVERFLOW) return set_error(MG_E_CUDA, "device table overflow");
+    *stop = -1;
+    const uint64_t budget = one && o.max_elements ? o.max_elements : ~0ull;
+    for (int l = l0; l <= last; ++l) {
+      R[l] = l == 0 ? nq : uint32_t(h[lvl_slot(l - 1, L_OUT)]);
+      T[l] = h[lvl_slot(l, L_T)];
+      if (h[C_STOP] == uint64_t(l) + 1) {
+        cur[l] = 0;
+        *stop = l;
+        return T[l] > budget - elements ? refuse() : int(MG_OK);
+      }
+      if (T[l] > budget - elements) return refuse();
+      cur[l] = T[l];
+      elements += T[l];
+      res->chunks += T[l] > 0;
+    }
+    return MG_OK;
+  };
+
+  int top = -1;
+  bool waited = false;
+  if (one && last >= 0) {
+    T[0] = a.T0 = root_range(dg, plans[0], a, &a.root_first);
+    res->balg += T[0] * root_charge(dg);
+    res->balgc += T[0] * root_charge(dg);
+    top = T[0] ? 0 : -1;
+  } else if (last >= 0) {
+    if ((rc = descend(0, nq))) return rc;
+    if ((rc = settle(0, &top))) return rc;
+    waited = true;
+  }
+  while (top >= 0) {
+    if (cur[top] >= T[top]) {
+      --top;
+      continue;
+    }
+    const uint64_t t0 = cur[top];
+    const uint64_t t1 = writes[top] ? std::min(T[top], t0 + B.cap) : T[top];
+    if (one && o.max_elements && t1 - t0 > o.max_elements - elements) return refuse();
+    elements += t1 - t0;
+    if (waited)  // the slots of this level and below
+      MG_CK(cudaMemsetAsync(B.res + lvl_slot(top, 0), 0, (C_NUM - lvl_slot(top, 0)) * 8, st));
+    set_level(top);
+    a.dev = 0;
+    for (uint64_t s0 = t0; s0 < t1; s0 += B.seg) {
+      a.t0 = s0;
+      a.t1 = std::min(t1, s0 + B.seg);
+      if (!(one && top == 0)) {
+        const uint32_t ntiles = uint32_t((a.t1 - s0 + EXPAND_TILE - 1) / EXPAND_TILE);
+        k_tile_rows<<<grid_for(uint64_t(ntiles) + 1, 256, sms * 16), 256, 0, st>>>(
+            B.woff[top], R[top], s0, a.t1, ntiles, B.tile_row);
+        res->launches++;
+      }
+      if (s0 > t0) MG_CK(cudaMemsetAsync(B.res + a.tile_slot, 0, 8, st));
+      if ((rc = expand(top, a.t1 - s0))) return rc;
+    }
+    res->chunks++;
+    cur[top] = t1;
+    if ((rc = descend(top + 1, std::min(t1 - t0, B.cap)))) return rc;
+    int stop;
+    if ((rc = settle(top + 1, &stop))) return rc;
+    waited = true;
+    if (stop >= 0) top = stop;
+  }
+  if (!waited) {  // nothing to expand
+    int stop;
+    last = -1;
+    if ((rc = settle(0, &stop))) return rc;
+  }
+  res->elements = elements;
+  res->balg += h[C_BALG];
+  res->balgc += h[C_BALGC];
+  res->emitted = h[C_EMIT];
+  return MG_OK;
+}
+
 static int run_levels(DevGraph* dg, std::vector<PlanDev> plans, bool count_mode,
                       const EmitBuf* emit, const mg_opts& o, uint64_t* counts_out,
                       RunResult* res, uint64_t* lvl_rows_out = nullptr) {
@@ -1632,27 +1892,18 @@ static int run_levels(DevGraph* dg, std::vector<PlanDev> plans, bool count_mode,
   if (rc) return rc;
   Workspace* ws = dg->ws;
   cudaStream_t st = dg->stream;
-  MG_CK(cudaMemcpyAsync(ws->plans, plans.data(), nq * sizeof(PlanDev), cudaMemcpyHostToDevice, st));
-  MG_CK(cudaMemsetAsync(ws->counts, 0, nq * 8ull, st));
-  MG_CK(cudaMemsetAsync(ws->lvl_rows, 0, uint64_t(nq) * (MAXK + 1) * 8, st));
-  MG_CK(cudaMemsetAsync(ws->q_elems, 0, uint64_t(nq) * 8, st));
-  MG_CK(cudaMemsetAsync(ws->ctr, 0, C_NUM * 8, st));
+  const bool batch = nq > 1;
   MG_CK(cudaEventRecord(ws->ev0, st));
-
+  MG_CK(cudaMemsetAsync(ws->res, 0, res_words(nq) * 8, st));
 
   StepArgs a;
   std::memset(&a, 0, sizeof(a));
   a.g = dg->g;
   a.plans = ws->plans;
-  a.ctr = ws->ctr;
-  a.counts = ws->counts;
-  a.lvl_rows = ws->lvl_rows;
-  a.q_elems = ws->q_elems;
-  a.q_budget = nq > 1 ? o.max_elements : 0;  // batch: per-query budget
+  a.q_budget = batch ? o.max_elements : 0;  // batch: per-query budget
   a.count_mode = count_mode ? 1u : 0u;
   a.filters = o.filters & MG_FILTER_ALL;
   a.grab = o.grab;
-  a.stats = nq == 1 ? 1u : 0u;
   a.nq = nq;
   if (emit) {
     for (int j = 0; j < MAXK; ++j) a.emit_col[j] = emit->col[j];
@@ -1660,13 +1911,10 @@ static int run_levels(DevGraph* dg, std::vector<PlanDev> plans, bool count_mode,
   }
   a.root_step = o.root_step > 1 ? o.root_step : 1u;
   a.probe_min = o.probe_min ? o.probe_min : kProbeMin;
-  a.out_slot = C_OUT;
-  a.tile_slot = C_TILE;
   if (o.root_end || a.root_step > 1) {
     a.root_begin = o.root_begin;
     a.root_end = o.root_end ? o.root_end : ~0ull;
   }
-  const bool batch = nq > 1;
   if (batch) {
     k_iota<<<grid_for(nq, 256, 1024), 256, 0, st>>>(ws->qid[0], nq);
     res->launches++;
@@ -1683,159 +1931,62 @@ static int run_levels(DevGraph* dg, std::vector<PlanDev> plans, bool count_mode,
     a.root_keep = ws->root_keep;
     res->launches++;
   }
-  uint64_t T[MAXK] = {}, cur[MAXK] = {};
-  uint32_t R[MAXK] = {};
-  R[0] = nq;
-  int lvl = 0;
-  bool need_work = true;
-  const unsigned sms = dg->sms;
-  uint64_t elements = 0;
-
   // Pendant tails counted in closed form (count mode): tail-key table and
   // memo table of two-hop aggregates, shared by every query of the call.
-  bool dense = false;
   if (count_mode && o.no_tail != 1) {
     rc = setup_tails(dg, plans, ws->tails,
                      [&](void** p, size_t bytes) { return ws_alloc(ws, p, bytes); }, st, &a,
                      &res->launches);
     if (rc) return rc;
-    dense = a.tail_dense != 0;
-    if (dense)
-      MG_CK(cudaMemcpyAsync(ws->plans, plans.data(), nq * sizeof(PlanDev),
-                            cudaMemcpyHostToDevice, st));
   }
   a.star = count_mode && o.no_tail != 1;
-  // writes[l]: some query can append rows to the level-(l+1) table.
-  bool writes[MAXK] = {};
-  for (uint32_t l = 0; l < kmax; ++l)
-    for (auto& p : plans)
-      if (p.k > l + 1 && !(count_mode && p.k == l + 2 && p.last_o1) &&
-          !(dense && p.tail2 && p.k == l + 3) && !(a.star && p.star2 && p.k == l + 3))
-        writes[l] = true;
+  if (batch) {
+    MG_CK(cudaMemcpyAsync(ws->plans, plans.data(), nq * sizeof(PlanDev), cudaMemcpyHostToDevice,
+                          st));
+  } else {
+    *ws->h_plan = plans[0];
+    MG_CK(cudaMemcpyAsync(ws->plans, ws->h_plan, sizeof(PlanDev), cudaMemcpyHostToDevice, st));
+  }
 
-  auto launch_work_scan = [&](int l) -> int {
-    k_work<<<grid_for(R[l], 256, sms * 16), 256, 0, st>>>(a);
-    const uint32_t nb = (R[l] + SCAN_TILE - 1) / SCAN_TILE;
-    k_scan_reduce<<<nb, 256, 0, st>>>(ws->work[l], R[l], ws->bsum);
-    k_scan_bsum<<<1, 1024, 0, st>>>(ws->bsum, nb, ws->woff[l] + R[l]);
-    k_scan_apply<<<nb, 256, 0, st>>>(ws->work[l], R[l], ws->bsum, ws->woff[l]);
-    res->launches += 4;
-    MG_CK(cudaMemcpyAsync(&ws->h_ctr[0], ws->woff[l] + R[l], 8, cudaMemcpyDeviceToHost, st));
-    MG_CK(cudaStreamSynchronize(st));
-    return MG_OK;
-  };
-  auto tab = [&](int l) {
-    TabPtrs t{};
-    for (int j = 0; j < l; ++j) t.col[j] = ws->col[l][j];
-    t.qid = batch ? ws->qid[l] : nullptr;
-    return t;
-  };
-  while (true) {
-    if (need_work) {
-      a.level = uint32_t(lvl);
-      a.R = R[lvl];
-      a.in = tab(lvl);
-      a.work = ws->work[lvl];
-      a.woff = ws->woff[lvl];
-      a.dstart = ws->dstart[lvl];
-      a.dci = ws->dci[lvl];
-      if ((rc = launch_work_scan(lvl))) return rc;
-      T[lvl] = ws->h_ctr[0];
-      cur[lvl] = 0;
-      need_work = false;
-    }
-    if (cur[lvl] < T[lvl]) {
-      const uint64_t t0 = cur[lvl];
-      const uint64_t t1 = writes[lvl] ? std::min(T[lvl], t0 + cap) : T[lvl];
-      elements += t1 - t0;
-      if (nq == 1 && o.max_elements && elements > o.max_elements) {
-        cudaStreamSynchronize(st);
-        return set_error(MG_E_LIMIT, "work budget of %llu candidate elements exceeded",
-                         (unsigned long long)o.max_elements);
-      }
-      a.tile_row = ws->tile_row;
-      a.level = uint32_t(lvl);
-      a.R = R[lvl];
-      a.in = tab(lvl);
-      a.work = ws->work[lvl];
-      a.woff = ws->woff[lvl];
-      a.dstart = ws->dstart[lvl];
-      a.dci = ws->dci[lvl];
-      a.t0 = t0;
-      a.t1 = t1;
-      if (writes[lvl]) {
-        a.out = tab(lvl + 1);
-        a.out_cap = cap;
-      } else {
-        a.out = TabPtrs{};
-        a.out_cap = 0;
-      }
-      MG_CK(cudaMemsetAsync(ws->ctr + C_OUT, 0, 8, st));
-      for (uint64_t s0 = t0; s0 < t1; s0 += kSegment) {
-        const uint64_t s1 = std::min(t1, s0 + kSegment);
-        const uint32_t ntiles = uint32_t((s1 - s0 + EXPAND_TILE - 1) / EXPAND_TILE);
-        a.t0 = s0;
-        a.t1 = s1;
-        k_tile_rows<<<grid_for(uint64_t(ntiles) + 1, 256, sms * 16), 256, 0, st>>>(
-            ws->woff[lvl], R[lvl], s0, s1, ntiles, ws->tile_row);
-        MG_CK(cudaMemsetAsync(ws->ctr + C_TILE, 0, 8, st));
-        if (o.kernel_events) MG_CK(cudaEventRecord(ws->ev2, st));
-        launch_expand(a, plans.data(), nq, count_mode, writes[lvl],
-                      grid_for(s1 - s0, 256, sms * 4), st);
-        if (o.kernel_events) {
-          MG_CK(cudaEventRecord(ws->ev3, st));
-          MG_CK(cudaEventSynchronize(ws->ev3));
-          float kms = 0;
-          MG_CK(cudaEventElapsedTime(&kms, ws->ev2, ws->ev3));
-          res->expand_ms += kms;
-        }
-        res->expand_launches++;
-        res->launches += 2;
-      }
-      res->chunks++;
-      MG_CK(cudaGetLastError());
-      cur[lvl] = t1;
-      if (writes[lvl]) {
-        MG_CK(cudaMemcpyAsync(&ws->h_ctr[0], ws->ctr + C_OUT, 8, cudaMemcpyDeviceToHost, st));
-        MG_CK(cudaStreamSynchronize(st));
-        const uint64_t rows = ws->h_ctr[0];
-        if (rows > cap) return set_error(MG_E_CUDA, "level table overflow (%llu > %llu)",
-                                         (unsigned long long)rows, (unsigned long long)cap);
-        if (rows > 0) {
-          R[lvl + 1] = uint32_t(rows);
-          ++lvl;
-          need_work = true;
-        }
-      }
-    } else {
-      if (lvl == 0) break;
-      --lvl;
-    }
+  WalkBufs B;
+  B.cap = cap;
+  B.col = ws->col;
+  B.qid = ws->qid;
+  B.woff = ws->woff;
+  B.dstart = ws->dstart;
+  B.dci = ws->dci;
+  B.tile_row = ws->tile_row;
+  B.seg = kSegment;
+  B.status = ws->status;
+  B.status_bytes = ws->status_bytes;
+  B.epoch = &ws->epoch;
+  B.res = ws->res;
+  B.h_res = ws->h_res;
+  B.done = ws->ev1;
+  B.ev2 = ws->ev2;
+  B.ev3 = ws->ev3;
+  if ((rc = walk_levels(dg, plans.data(), nq, count_mode, o, a, B, res))) {
+    cudaStreamSynchronize(st);
+    return rc;
   }
-  MG_CK(cudaEventRecord(ws->ev1, st));
-  MG_CK(cudaMemcpyAsync(ws->h_ctr, ws->ctr, C_NUM * 8, cudaMemcpyDeviceToHost, st));
-  MG_CK(cudaMemcpyAsync(counts_out, ws->counts, nq * 8ull, cudaMemcpyDeviceToHost, st));
-  if (lvl_rows_out)
-    MG_CK(cudaMemcpyAsync(lvl_rows_out, ws->lvl_rows, uint64_t(nq) * (MAXK + 1) * 8,
-                          cudaMemcpyDeviceToHost, st));
-  MG_CK(cudaMemcpyAsync(res->surv, ws->lvl_rows, (MAXK + 1) * 8, cudaMemcpyDeviceToHost, st));
-  std::vector<unsigned long long> qel;
-  if (a.q_budget) {
-    qel.resize(nq);
-    MG_CK(cudaMemcpyAsync(qel.data(), ws->q_elems, uint64_t(nq) * 8, cudaMemcpyDeviceToHost, st));
-  }
-  MG_CK(cudaStreamSynchronize(st));
-  MG_CK(cudaGetLastError());
   float ms = 0;
   MG_CK(cudaEventElapsedTime(&ms, ws->ev0, ws->ev1));
   res->ms = ms;
-  res->elements = elements;
-  for (uint32_t q = 0; q < qel.size(); ++q)
-    if (qel[q] > a.q_budget) counts_out[q] = ~0ull;  // over budget: unknown
-  res->balg = ws->h_ctr[C_BALG];
-  res->balgc = ws->h_ctr[C_BALGC];
-  res->emitted = ws->h_ctr[C_EMIT];
-  if (ws->h_ctr[C_ERR] & ERR_OVERFLOW) return set_error(MG_E_CUDA, "device table overflow");
+  const unsigned long long *cnt = ws->h_res + C_NUM, *lvl = cnt + nq, *qel = lvl + MAXK + 1;
+  std::vector<unsigned long long> all;
+  if (batch) {
+    all.resize(res_words(nq) - C_NUM);
+    MG_CK(cudaMemcpyAsync(all.data(), ws->res + C_NUM, all.size() * 8, cudaMemcpyDeviceToHost, st));
+    MG_CK(cudaStreamSynchronize(st));
+    cnt = all.data();
+    lvl = cnt + nq;
+    qel = lvl + uint64_t(nq) * (MAXK + 1);
+  }
+  for (uint32_t q = 0; q < nq; ++q)  // over budget: unknown
+    counts_out[q] = a.q_budget && qel[q] > a.q_budget ? ~0ull : cnt[q];
+  if (lvl_rows_out)
+    for (uint64_t x = 0; x < uint64_t(nq) * (MAXK + 1); ++x) lvl_rows_out[x] = lvl[x];
+  for (int x = 0; x <= MAXK; ++x) res->surv[x] = lvl[x];
   return MG_OK;
 }
 
@@ -2086,7 +2237,6 @@ struct Lane {
   unsigned long long* status = nullptr;  // look-back words of the work/scan kernel
   uint32_t* tile_row = nullptr;
   uint32_t* col[MAXK][MAXK] = {};
-  uint32_t* work[MAXK] = {};
   uint64_t* woff[MAXK] = {};
   uint32_t* dstart[MAXK] = {};
   uint8_t* dci[MAXK] = {};
@@ -2107,10 +2257,8 @@ struct LaneSet {
 };
 
 constexpr uint64_t kLaneCap = 1ull << 20;     // rows per lane level table
-constexpr uint64_t kLaneSegment = 1ull << 26; // elements per lane expand launch
+constexpr uint64_t kLaneSegment = 1ull << 30; // elements per lane expand launch
 constexpr uint32_t kLanes = 8;
-constexpr uint32_t kSpinLimit = 1u << 22;     // polls of a look-back wait (~0.3 s)
-constexpr uint32_t kEpochMax = (1u << 20) - 1;
 
 void free_lanes(LaneSet* ls) {
   if (!ls) return;
@@ -2165,23 +2313,12 @@ static int ensure_lanes(DevGraph* dg, uint32_t nl, uint64_t cap, uint32_t kmax) 
       const uint64_t rows = l == 0 ? 1 : cap;
       for (uint32_t j = 0; j < l; ++j)
         if ((rc = lane_alloc(ls, (void**)&L.col[l][j], rows * 4))) return rc;
-      if ((rc = lane_alloc(ls, (void**)&L.work[l], rows * 4))) return rc;
       if ((rc = lane_alloc(ls, (void**)&L.woff[l], (rows + 1) * 8))) return rc;
       if ((rc = lane_alloc(ls, (void**)&L.dstart[l], rows * 4))) return rc;
       if ((rc = lane_alloc(ls, (void**)&L.dci[l], rows))) return rc;
     }
   }
   return MG_OK;
-}
-
-// Last level a plan expands in count mode: k-1, or k-2 when the last
-// position is closed in place, or k-3 when a pendant tail is closed from
-// dense aggregates.
-static int last_level(const PlanDev& P, bool dense, bool star) {
-  int l = int(P.k) - 1;
-  if (P.k >= 2 && P.last_o1) l = int(P.k) - 2;
-  if ((dense && P.tail2) || (star && P.star2)) l = int(P.k) - 3;
-  return l;
 }
 
 static int subiso_batch_lanes(DevGraph* dg, std::vector<PlanDev>& plans, const mg_opts& o,
@@ -2238,19 +2375,25 @@ static int subiso_batch_lanes(DevGraph* dg, std::vector<PlanDev>& plans, const m
   a.root_step = 1;
   a.probe_min = o.probe_min ? o.probe_min : kProbeMin;
   a.q_budget = o.max_elements;
-  a.lane = 1;
+  a.lane = a.dev = 1;
   a.cap_rows = cap;
   a.seg_cap = ls->seg_cap;
+  a.t_limit = ls->seg_cap;
   a.spin_limit = kSpinLimit;
-  a.nq = 1;
-  for (Lane& L : ls->lanes) {
+  a.nq = a.R = 1;
+  // Level-0 candidates of every query: the elements its budget is charged
+  // with before the lane starts.
+  std::vector<uint64_t> t0(nq);
+  std::vector<uint32_t> first(nq);
+  for (uint32_t j = 0; j < nq; ++j) t0[j] = root_range(dg, plans[j], a, &first[j]);
+  for (uint32_t l = 0; l < nl; ++l) {
+    Lane& L = ls->lanes[l];
     MG_CK(cudaStreamWaitEvent(L.st, ls->ev_start, 0));
     MG_CK(cudaMemsetAsync(L.ctr, 0, C_NUM * 8, L.st));
     MG_CK(cudaMemsetAsync(L.counts, 0, 8, L.st));
     MG_CK(cudaMemsetAsync(L.lvl, 0, (MAXK + 1) * 8, L.st));
-    MG_CK(cudaMemsetAsync(L.qel, 0, 8, L.st));
+    k_set_u64<<<1, 1, 0, L.st>>>(L.qel, l < nq ? t0[l] : 0ull);
   }
-  const unsigned g_ws = sms * 2, g_tr = sms * 2, g_ex = sms * 4;
   for (uint32_t j = 0; j < nq; ++j) {
     Lane& L = ls->lanes[j % nl];
     const PlanDev& P = plans[j];
@@ -2261,36 +2404,46 @@ static int subiso_batch_lanes(DevGraph* dg, std::vector<PlanDev>& plans, const m
     a.q_elems = L.qel;
     a.scan_status = L.status;
     a.tile_row = L.tile_row;
-    const int last = P.zero ? -1 : last_level(P, a.tail_dense != 0, a.star != 0);
+    int last = P.zero ? -1 : last_level(P, a.tail_dense != 0, a.star != 0);
+    if (o.max_elements && t0[j] > o.max_elements) last = -1;
+    a.T0 = t0[j];
+    a.root_first = first[j];
+    uint64_t rows = 1;
     for (int l = 0; l <= last; ++l) {
       a.level = uint32_t(l);
       TabPtrs t{};
       for (int c = 0; c < l; ++c) t.col[c] = L.col[l][c];
       a.in = t;
-      a.work = L.work[l];
       a.woff = L.woff[l];
       a.dstart = L.dstart[l];
       a.dci = L.dci[l];
-      if (++L.epoch > kEpochMax) {
-        MG_CK(cudaMemsetAsync(L.status, 0, (cap / WS_ROWS + 2) * 8, L.st));
-        L.epoch = 1;
+      if (l > 0) {
+        if (++L.epoch > kEpochMax) {
+          MG_CK(cudaMemsetAsync(L.status, 0, (cap / WS_ROWS + 2) * 8, L.st));
+          L.epoch = 1;
+        }
+        k_work_scan<<<grid_for(rows, WS_ROWS, sms * 2), 256, 0, L.st>>>(a, L.epoch);
+        res->launches++;
       }
-      k_work_scan<<<g_ws, 256, 0, L.st>>>(a, L.epoch);
-      k_tile_rows_lane<<<g_tr, 256, 0, L.st>>>(a);
       const bool writes = l < last;
       TabPtrs out{};
       if (writes)
         for (int c = 0; c <= l; ++c) out.col[c] = L.col[l + 1][c];
       a.out = out;
       a.out_cap = writes ? cap : 0;
-      a.out_slot = C_LOUT + l;
-      a.tile_slot = C_LTILE + l;
-      launch_expand(a, &P, 1, true, writes, g_ex, L.st);
-      res->launches += 3;
+      a.out_slot = lvl_slot(l, L_OUT);
+      a.tile_slot = lvl_slot(l, L_TILE);
+      const uint64_t bound =
+          l == 0 ? t0[j] : bounded_product(rows, row_bound(dg, &P, 1, l));
+      launch_expand(a, expand_mode(a, uint32_t(l), &P, 1, true, writes),
+                    grid_for(bound, 256, sms * 4), L.st);
+      rows = std::min(bound, cap);
+      res->launches++;
       res->expand_launches++;
     }
     k_lane_done<<<1, 32, 0, L.st>>>(L.ctr, L.counts, L.lvl, L.qel, o.max_elements, j,
-                                   ls->r_counts, ls->r_lvl, ls->r_err, ls->r_balg);
+                                   j + nl < nq ? t0[j + nl] : 0ull, ls->r_counts, ls->r_lvl,
+                                   ls->r_err, ls->r_balg);
     res->launches++;
   }
   MG_CK(cudaGetLastError());
@@ -2311,13 +2464,19 @@ static int subiso_batch_lanes(DevGraph* dg, std::vector<PlanDev>& plans, const m
   res->ms = ms;
   for (uint32_t j = 0; j < nq; ++j) {
     if (err[j]) continue;  // charged by its re-run below
-    res->balg += balg[2ull * j];
-    res->balgc += balg[2ull * j + 1];
+    res->balg += balg[2ull * j] + t0[j] * root_charge(dg);
+    res->balgc += balg[2ull * j + 1] + t0[j] * root_charge(dg);
   }
   for (uint32_t j = 0; j < nq; ++j) {
     if (err[j] & ERR_TIMEOUT)
       return set_error(MG_E_TIMEOUT, "query %u: a lane's device wait gave up", j);
     if (err[j] & ERR_OVERFLOW) {
+      if (o.max_elements && cnt[j] == ~0ull) {
+        // The elements that did run already pass its budget.
+        for (uint32_t i = 0; i <= MAXK; ++i) lv[uint64_t(j) * (MAXK + 1) + i] = 0;
+        res->reruns++;
+        continue;
+      }
       // Did not fit its lane: count it again on the chunked path.
       std::vector<PlanDev> one(1, plans[j]);
       RunResult r1;
@@ -2374,8 +2533,8 @@ static int selftest_wait(DevGraph* dg, const mg_csr_view* q, uint32_t spin_limit
   cudaStream_t st = L.st;
   const uint64_t rows = 2 * WS_ROWS;
   std::vector<unsigned long long> ctr(C_NUM, 0);
-  ctr[C_LOUT + 0] = rows;  // level-1 table holds `rows` rows
-  ctr[C_LSCAN + 1] = 1;    // tile 0 of level 1 is never handed out
+  ctr[lvl_slot(0, L_OUT)] = rows;  // level-1 table holds `rows` rows
+  ctr[lvl_slot(1, L_SCAN)] = 1;    // tile 0 of level 1 is never handed out
   MG_CK(cudaMemcpyAsync(ls->plans, &P, sizeof(PlanDev), cudaMemcpyHostToDevice, st));
   MG_CK(cudaMemcpyAsync(L.ctr, ctr.data(), C_NUM * 8, cudaMemcpyHostToDevice, st));
   // every row holds the first vertex of the bucket of position 0
@@ -2392,13 +2551,13 @@ static int selftest_wait(DevGraph* dg, const mg_csr_view* q, uint32_t spin_limit
   a.q_elems = L.qel;
   a.level = 1;
   a.in.col[0] = L.col[1][0];
-  a.work = L.work[1];
   a.woff = L.woff[1];
   a.dstart = L.dstart[1];
   a.dci = L.dci[1];
-  a.lane = 1;
+  a.lane = a.dev = 1;
   a.cap_rows = ls->cap;
-  a.seg_cap = ls->seg_cap;
+  a.seg_cap = a.t_limit = ls->seg_cap;
+  a.tile_row = L.tile_row;
   a.scan_status = L.status;
   a.spin_limit = spin_limit;
   a.root_step = 1;
@@ -2659,17 +2818,13 @@ int noalloc_scratch(int device, unsigned char** out) {
   return MG_OK;
 }
 
-// Carves the level tables of a single-query count out of `base`; returns the
-// bytes used (a size above MG_NOALLOC_SCRATCH_BYTES means it does not fit).
+// Level tables of a single-query count, carved out of `base`.
 struct NoallocLayout {
-  unsigned long long* ctr;
-  unsigned long long* counts;
-  unsigned long long* lvl_rows;
+  unsigned long long* res;
   PlanDev* plan;
-  uint64_t* bsum;
+  unsigned long long* status;
   uint32_t* tile_row;
   uint32_t* col[MAXK][MAXK];
-  uint32_t* work[MAXK];
   uint64_t* woff[MAXK];
   uint32_t* dstart[MAXK];
   uint8_t* dci[MAXK];
@@ -2678,24 +2833,46 @@ struct NoallocLayout {
 // Elements per expand launch of a level whose survivors are not stored.
 constexpr uint64_t kNoallocSegment = 1ull << 24;
 
+// Look-back words of tables of `cap` rows (a single vertex needs none).
+uint64_t noalloc_status_bytes(uint64_t cap, uint32_t k) {
+  return (k > 1 ? cap / WS_ROWS + 2 : 1) * 8;
+}
+
+// Bytes that tables of `cap` rows are charged with.  A fixed formula that
+// bounds the layout below, so that the chunk_rows that fit the scratch do not
+// change with it.
+uint64_t noalloc_charge(uint64_t cap, uint32_t k) {
+  uint64_t off = 0;
+  auto take = [&](uint64_t bytes) { off = ((off + 255) & ~uint64_t(255)) + bytes; };
+  for (uint64_t bytes : {uint64_t(72 * 8), uint64_t(8), uint64_t((MAXK + 1) * 8),
+                         uint64_t(sizeof(PlanDev)), (cap / 4096 + 2) * 8,
+                         (kNoallocSegment / 256 + 2) * 4})
+    take(bytes);
+  for (uint32_t l = 0; l < k; ++l) {
+    const uint64_t rows = l == 0 ? 1 : cap;
+    for (uint32_t j = 0; j <= l; ++j) take(rows * 4);
+    take((rows + 1) * 8);
+    take(rows * 4);
+    take(rows);
+  }
+  return off;
+}
+
 uint64_t noalloc_carve(unsigned char* base, uint64_t cap, uint32_t k, NoallocLayout* L) {
   uint64_t off = 0;
   auto take = [&](uint64_t bytes) -> unsigned char* {
     off = (off + 255) & ~uint64_t(255);
-    unsigned char* p = base ? base + off : nullptr;
+    unsigned char* p = base + off;
     off += bytes;
     return p;
   };
-  L->ctr = reinterpret_cast<unsigned long long*>(take(C_NUM * 8));
-  L->counts = reinterpret_cast<unsigned long long*>(take(8));
-  L->lvl_rows = reinterpret_cast<unsigned long long*>(take((MAXK + 1) * 8));
+  L->res = reinterpret_cast<unsigned long long*>(take(res_words(1) * 8));
   L->plan = reinterpret_cast<PlanDev*>(take(sizeof(PlanDev)));
-  L->bsum = reinterpret_cast<uint64_t*>(take((cap / SCAN_TILE + 2) * 8));
+  L->status = reinterpret_cast<unsigned long long*>(take(noalloc_status_bytes(cap, k)));
   L->tile_row = reinterpret_cast<uint32_t*>(take((kNoallocSegment / EXPAND_TILE + 2) * 4));
   for (uint32_t l = 0; l < k; ++l) {
     const uint64_t rows = l == 0 ? 1 : cap;
     for (uint32_t j = 0; j < l; ++j) L->col[l][j] = reinterpret_cast<uint32_t*>(take(rows * 4));
-    L->work[l] = reinterpret_cast<uint32_t*>(take(rows * 4));
     L->woff[l] = reinterpret_cast<uint64_t*>(take((rows + 1) * 8));
     L->dstart[l] = reinterpret_cast<uint32_t*>(take(rows * 4));
     L->dci[l] = reinterpret_cast<uint8_t*>(take(rows));
@@ -2739,18 +2916,18 @@ int noalloc_count(DevGraph* dg, const mg_csr_view* q, const mg_opts* opts, uint6
   uint64_t cap = 0;
   if (o.chunk_rows) {
     if (o.chunk_rows > (1ull << 31) ||
-        noalloc_carve(nullptr, o.chunk_rows, k, &L) > MG_NOALLOC_SCRATCH_BYTES)
+        noalloc_charge(o.chunk_rows, k) > MG_NOALLOC_SCRATCH_BYTES)
       return set_error(MG_E_LIMIT,
                        "chunk_rows=%llu for a %u-vertex query needs %llu bytes of scratch; the "
                        "static scratch holds %llu bytes",
                        (unsigned long long)o.chunk_rows, k,
-                       (unsigned long long)noalloc_carve(nullptr, std::min<uint64_t>(
-                           o.chunk_rows, 1ull << 31), k, &L),
+                       (unsigned long long)noalloc_charge(
+                           std::min<uint64_t>(o.chunk_rows, 1ull << 31), k),
                        (unsigned long long)MG_NOALLOC_SCRATCH_BYTES);
     cap = o.chunk_rows;
   } else {
     for (uint64_t c = 1ull << 22; c >= 64; c >>= 1)
-      if (noalloc_carve(nullptr, c, k, &L) <= MG_NOALLOC_SCRATCH_BYTES) {
+      if (noalloc_charge(c, k) <= MG_NOALLOC_SCRATCH_BYTES) {
         cap = c;
         break;
       }
@@ -2760,119 +2937,52 @@ int noalloc_count(DevGraph* dg, const mg_csr_view* q, const mg_opts* opts, uint6
   }
   unsigned char* base = nullptr;
   if ((rc = noalloc_scratch(dg->device, &base))) return rc;
-  noalloc_carve(base, cap, k, &L);
+  if (noalloc_carve(base, cap, k, &L) > MG_NOALLOC_SCRATCH_BYTES)
+    return set_error(MG_E_LIMIT, "tables of %llu rows do not fit the static scratch",
+                     (unsigned long long)cap);
 
   cudaStream_t st = dg->stream;
   // The array keeps the previous call's contents: counters start at zero.
   MG_CK(cudaMemcpyAsync(L.plan, &P, sizeof(PlanDev), cudaMemcpyHostToDevice, st));
-  MG_CK(cudaMemsetAsync(L.counts, 0, 8, st));
-  MG_CK(cudaMemsetAsync(L.lvl_rows, 0, (MAXK + 1) * 8, st));
-  MG_CK(cudaMemsetAsync(L.ctr, 0, C_NUM * 8, st));
+  MG_CK(cudaMemsetAsync(L.res, 0, res_words(1) * 8, st));
+  MG_CK(cudaMemsetAsync(L.status, 0, noalloc_status_bytes(cap, k), st));
 
   StepArgs a;
   std::memset(&a, 0, sizeof(a));
   a.g = dg->g;
   a.plans = L.plan;
-  a.ctr = L.ctr;
-  a.counts = L.counts;
-  a.lvl_rows = L.lvl_rows;
   a.count_mode = 1;
   a.filters = o.filters & MG_FILTER_ALL;
   a.nq = 1;
   a.grab = o.grab;
-  a.tile_row = L.tile_row;
   a.root_step = o.root_step > 1 ? o.root_step : 1u;
   a.probe_min = o.probe_min ? o.probe_min : kProbeMin;
-  a.out_slot = C_OUT;
-  a.tile_slot = C_TILE;
   if (o.root_end || a.root_step > 1) {
     a.root_begin = o.root_begin;
     a.root_end = o.root_end ? o.root_end : ~0ull;
   }
-  bool writes[MAXK] = {};
-  for (uint32_t l = 0; l < k; ++l)
-    writes[l] = P.k > l + 1 && !(P.k == l + 2 && P.last_o1);
-  auto tab = [&](uint32_t l) {
-    TabPtrs t{};
-    for (uint32_t j = 0; j < l; ++j) t.col[j] = L.col[l][j];
-    return t;
-  };
-  const unsigned sms = dg->sms;
-  uint64_t T[MAXK] = {}, cur[MAXK] = {}, host_u64 = 0, elements = 0;
-  uint32_t R[MAXK] = {};
-  R[0] = 1;
-  int lvl = 0;
-  bool need_work = true;
-  while (true) {
-    a.level = uint32_t(lvl);
-    a.R = R[lvl];
-    a.in = tab(lvl);
-    a.work = L.work[lvl];
-    a.woff = L.woff[lvl];
-    a.dstart = L.dstart[lvl];
-    a.dci = L.dci[lvl];
-    if (need_work) {
-      k_work<<<grid_for(R[lvl], 256, sms * 16), 256, 0, st>>>(a);
-      const uint32_t nb = (R[lvl] + SCAN_TILE - 1) / SCAN_TILE;
-      k_scan_reduce<<<nb, 256, 0, st>>>(L.work[lvl], R[lvl], L.bsum);
-      k_scan_bsum<<<1, 1024, 0, st>>>(L.bsum, nb, L.woff[lvl] + R[lvl]);
-      k_scan_apply<<<nb, 256, 0, st>>>(L.work[lvl], R[lvl], L.bsum, L.woff[lvl]);
-      MG_CK(cudaMemcpyAsync(&host_u64, L.woff[lvl] + R[lvl], 8, cudaMemcpyDeviceToHost, st));
-      MG_CK(cudaStreamSynchronize(st));
-      T[lvl] = host_u64;
-      cur[lvl] = 0;
-      need_work = false;
-    }
-    if (cur[lvl] < T[lvl]) {
-      const uint64_t t0 = cur[lvl];
-      const uint64_t t1 = writes[lvl] ? std::min(T[lvl], t0 + cap) : T[lvl];
-      elements += t1 - t0;
-      if (o.max_elements && elements > o.max_elements) {
-        cudaStreamSynchronize(st);  // nothing of this call stays queued on the array
-        return set_error(MG_E_LIMIT, "work budget of %llu candidate elements exceeded",
-                         (unsigned long long)o.max_elements);
-      }
-      a.out = writes[lvl] ? tab(lvl + 1) : TabPtrs{};
-      a.out_cap = writes[lvl] ? cap : 0;
-      MG_CK(cudaMemsetAsync(L.ctr + C_OUT, 0, 8, st));
-      const uint64_t seg = writes[lvl] ? std::min<uint64_t>(cap, kNoallocSegment) : kNoallocSegment;
-      for (uint64_t s0 = t0; s0 < t1; s0 += seg) {
-        const uint64_t s1 = std::min(t1, s0 + seg);
-        const uint32_t ntiles = uint32_t((s1 - s0 + EXPAND_TILE - 1) / EXPAND_TILE);
-        a.t0 = s0;
-        a.t1 = s1;
-        k_tile_rows<<<grid_for(uint64_t(ntiles) + 1, 256, sms * 16), 256, 0, st>>>(
-            L.woff[lvl], R[lvl], s0, s1, ntiles, L.tile_row);
-        MG_CK(cudaMemsetAsync(L.ctr + C_TILE, 0, 8, st));
-        launch_expand(a, &P, 1, true, writes[lvl],
-                      grid_for(s1 - s0, 256, sms * 4), st);
-      }
-      MG_CK(cudaGetLastError());
-      cur[lvl] = t1;
-      if (writes[lvl]) {
-        MG_CK(cudaMemcpyAsync(&host_u64, L.ctr + C_OUT, 8, cudaMemcpyDeviceToHost, st));
-        MG_CK(cudaStreamSynchronize(st));
-        if (host_u64 > cap)
-          return set_error(MG_E_CUDA, "level table overflow (%llu > %llu)",
-                           (unsigned long long)host_u64, (unsigned long long)cap);
-        if (host_u64 > 0) {
-          R[lvl + 1] = uint32_t(host_u64);
-          ++lvl;
-          need_work = true;
-        }
-      }
-    } else {
-      if (lvl == 0) break;
-      --lvl;
-    }
+  unsigned long long h[res_words(1)];
+  uint32_t epoch = 0;
+  WalkBufs B;
+  B.cap = cap;
+  B.col = L.col;
+  B.woff = L.woff;
+  B.dstart = L.dstart;
+  B.dci = L.dci;
+  B.tile_row = L.tile_row;
+  B.seg = kNoallocSegment;
+  B.status = L.status;
+  B.status_bytes = noalloc_status_bytes(cap, k);
+  B.epoch = &epoch;
+  B.res = L.res;
+  B.h_res = h;
+  RunResult res;
+  o.kernel_events = 0;
+  if ((rc = walk_levels(dg, &P, 1, true, o, a, B, &res))) {
+    cudaStreamSynchronize(st);  // nothing of this call stays queued on the array
+    return rc;
   }
-  unsigned long long err = 0, c = 0;
-  MG_CK(cudaMemcpyAsync(&err, L.ctr + C_ERR, 8, cudaMemcpyDeviceToHost, st));
-  MG_CK(cudaMemcpyAsync(&c, L.counts, 8, cudaMemcpyDeviceToHost, st));
-  MG_CK(cudaStreamSynchronize(st));
-  MG_CK(cudaGetLastError());
-  if (err & ERR_OVERFLOW) return set_error(MG_E_CUDA, "device table overflow");
-  *count = c;
+  *count = h[C_NUM];
   return MG_OK;
 }
 
