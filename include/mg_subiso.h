@@ -290,6 +290,13 @@ int  mg_subiso_emit(void* dgraph, const mg_csr_view* q, const mg_opts* opts,
 int  mg_subiso_emit_ex(void* dgraph, const mg_csr_view* q,
                        const mg_opts* opts, uint32_t* rows, uint64_t cap_rows,
                        uint64_t* n_rows, mg_stats* st);
+/* The same with the rows' memory handed out by the caller once their number
+ * is known: alloc(ctx, n) returns room for n rows of k ids (NULL: the call
+ * fails with MG_E_OOM).  It is called at most once, on the calling thread,
+ * with the graph handle in use: it must not call into this library.        */
+typedef uint32_t* (*mg_rows_alloc)(void* ctx, uint64_t n_rows);
+int  mg_subiso_emit_alloc(void* dgraph, const mg_csr_view* q, const mg_opts* opts,
+                          mg_rows_alloc alloc, void* ctx, uint64_t* n_rows, mg_stats* st);
 /* Counts for nq queries in one batch against one resident data graph.
  * Replaces nq calls of SubIso::Run (core/task/gpu_task/subiso.cu:236-260). */
 int  mg_subiso_batch_count(void* dgraph, const mg_csr_view* const* qs,

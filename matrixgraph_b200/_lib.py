@@ -107,6 +107,8 @@ _VP = C.c_void_p
 _PVP = C.POINTER(C.c_void_p)
 _PV = C.POINTER(CsrView)
 _PU64 = C.POINTER(C.c_uint64)
+# mg_rows_alloc: memory for the rows of an emit call
+RowsAlloc = C.CFUNCTYPE(C.c_void_p, C.c_void_p, C.c_uint64)
 _SIGS = {
     "mg_last_error": (C.c_char_p, []),
     "mg_version": (C.c_char_p, []),
@@ -145,6 +147,8 @@ _SIGS = {
     "mg_subiso_emit": (C.c_int, [_VP, _PV, C.POINTER(Opts), P32, C.c_uint64, _PU64]),
     "mg_subiso_emit_ex": (C.c_int, [_VP, _PV, C.POINTER(Opts), P32, C.c_uint64, _PU64,
                                     C.POINTER(Stats)]),
+    "mg_subiso_emit_alloc": (C.c_int, [_VP, _PV, C.POINTER(Opts), RowsAlloc, _VP, _PU64,
+                                       C.POINTER(Stats)]),
     "mg_subiso_batch_count": (C.c_int, [_VP, C.POINTER(_PV), C.c_uint32, C.POINTER(Opts),
                                         _PU64]),
     "mg_subiso_batch_count_ex": (C.c_int, [_VP, C.POINTER(_PV), C.c_uint32, C.POINTER(Opts),

@@ -120,11 +120,14 @@ struct DevGraph {
   GraphDev g{};
   mg_graph_info info{};
   GraphStats stats;
+  uint32_t max_gid = 0;      // no global id is above it
   bool stats_full = false;   // degree / label-pair statistics computed
   std::vector<uint32_t> h_bucket_off;
   std::vector<void*> allocs;
   Workspace* ws = nullptr;
   LaneSet* lanes = nullptr;
+  unsigned char* emit_mem = nullptr;  // emit calls: rows and sort buffers
+  uint64_t emit_bytes = 0;
   std::mutex mu;
   ~DevGraph();
 };

@@ -45,6 +45,7 @@ DevGraph::~DevGraph() {
     cudaStreamSynchronize(stream);
     free_workspace(ws);
     free_lanes(lanes);
+    cudaFree(emit_mem);
     for (void* p : allocs) cudaFree(p);
     cudaStreamDestroy(stream);
     cudaSetDevice(prev);
@@ -677,6 +678,7 @@ static int upload(const mg_csr_view* v, int device, const mg_upload_opts& uo, De
   // Global ids -> local ids when the stored ids are not the identity.
   bool ident = true;
   for (uint32_t i = 0; i < n && ident; ++i) ident = v->globalid[i] == i;
+  dg->max_gid = ident ? n - 1 : v->max_vid;
   uint32_t* d_g2l = nullptr;
   if (ident) {
     MG_CK(cudaMemcpyAsync(d_gid, d_input, uint64_t(n) * 4, cudaMemcpyDeviceToDevice, st));

@@ -112,11 +112,20 @@ class DeviceGraph:
     def emit(self, q: CSRGraph, cap: int | None = None, stats: bool = False, **kw):
         """Sorted matches, one row of k global ids per match (query-id order)."""
         o, keep = make_opts(**kw)
-        if cap is None:
-            cap = self.count(q, **kw)
-        rows = np.zeros((max(cap, 1), q.n), dtype=np.uint32)
         n = C.c_uint64()
         st = L.Stats()
+        if cap is None:
+            got = []
+
+            def alloc(_, n_rows):
+                got.append(np.empty((n_rows, q.n), dtype=np.uint32))
+                return got[0].ctypes.data if n_rows else None
+
+            L.check(L.lib.mg_subiso_emit_alloc(self.handle, C.byref(q.view), C.byref(o),
+                                               L.RowsAlloc(alloc), None, C.byref(n),
+                                               C.byref(st)))
+            return (got[0], n.value, stats_dict(st)) if stats else got[0]
+        rows = np.zeros((max(cap, 1), q.n), dtype=np.uint32)
         rc = L.lib.mg_subiso_emit_ex(self.handle, C.byref(q.view), C.byref(o),
                                      rows.ctypes.data_as(L.P32), cap, C.byref(n), C.byref(st))
         if rc not in (L.MG_OK, L.MG_E_CAPACITY):
