@@ -98,15 +98,13 @@ struct PlanDev {
 };
 
 // Signature of a two-hop aggregate: A(y) = sum over the da-slice of y labelled
-// la of the db-slice lengths labelled lb.  Queries of one call sharing a
-// signature share the hub table of aggregates.
+// la of the db-slice lengths labelled lb, for the vertices y labelled lp.
+// Queries of one call sharing a signature share its table.
 struct TailKey {
   uint32_t da, la, db, lb;
-  uint32_t lp;     // label of m_p: only hubs with this label get aggregates
+  uint32_t lp;
   uint32_t b0;     // first vertex of label lp
-  uint64_t base;   // first entry of this key's hub table (~0: none)
-  uint64_t lazy;   // first entry of this key's lazily filled table over the
-                   // bucket of label lp (~0: none, sum in place)
+  uint64_t base;   // first entry of this key's table (~0: none, sum in place)
 };
 
 struct Workspace;  // enumeration scratch (mg_enum.cu)

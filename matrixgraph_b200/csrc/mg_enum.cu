@@ -41,15 +41,19 @@ const char* last_error_cstr();
 // ---------------------------------------------------------------------------
 // Workspace (per graph handle)
 // ---------------------------------------------------------------------------
-// Pendant-tail keys of a call and the two-hop aggregates of their hubs.
+// Pendant-tail keys of a call and their two-hop aggregates (A, AD).
 struct TailStore {
-  unsigned long long* A = nullptr;
-  unsigned long long* AD = nullptr;
+  ulonglong2* agg = nullptr;
   uint64_t cap = 0;
-  unsigned long long* lazy = nullptr;  // packed (AD << 32 | A), ~0 = not yet filled
-  uint64_t lazy_cap = 0;
   TailKey* keys = nullptr;
   uint32_t keys_cap = 0;
+  void free() {
+    cudaFree(agg);
+    cudaFree(keys);
+    agg = nullptr;
+    keys = nullptr;
+    cap = keys_cap = 0;
+  }
 };
 
 struct Workspace {
@@ -99,6 +103,7 @@ constexpr int lvl_slot(int l, int what) { return C_LVL + 4 * l + what; }
 void free_workspace(Workspace* ws) {
   if (!ws) return;
   for (void* p : ws->allocs) cudaFree(p);
+  ws->tails.free();
   if (ws->h_res) cudaFreeHost(ws->h_res);
   if (ws->h_plan) cudaFreeHost(ws->h_plan);
   if (ws->ev0) cudaEventDestroy(ws->ev0);
@@ -220,13 +225,11 @@ struct StepArgs {
   uint32_t grab;   // expand tiles taken per work-queue grab
   const TailKey* tkeys;
   // Two-position pendant tails (tail_dense): counted while expanding
-  // position k-3; the two-hop aggregates of a hub m_p are read at
-  // tkeys[kid].base + hub slot, those of other vertices summed in place.
+  // position k-3; the two-hop aggregates of m_p are read at
+  // tail_agg[tkeys[kid].base + m_p - tkeys[kid].b0].
   uint32_t tail_dense;
   uint32_t star;  // two-leaf star endings are counted in closed form (PlanDev::star2)
-  const unsigned long long* tdA;
-  const unsigned long long* tdAD;
-  unsigned long long* tdL;  // lazily filled aggregates of non-hub vertices
+  const ulonglong2* tail_agg;
   // Level 0 of a single query is one row that needs no table: its candidates
   // are root_first + e * root_step, e < T0.
   uint64_t T0;
@@ -379,83 +382,113 @@ __device__ __forceinline__ void acc_flush_warp(const StepArgs& a, uint32_t q, ui
   }
 }
 
-// Two-hop aggregates of one tail key for the hubs of direction da, warp per
-// hub: for y labelled lp,
+// Two-hop aggregates of the tail keys, for every vertex y of label lp:
 //   A(y)  = sum_{x in N^{da}_{la}(y)} (|N^{db}_{lb}(x)| - [x self-loop, la == lb]),
 //   AD(y) = sum_{x in N^{da}_{la}(y)} |N^{db}_{lb}(x)|
-// at tdA / tdAD[tk.base + hub slot] (hubs of other labels are skipped: no
-// prefix can match them at position p).
-__global__ void __launch_bounds__(256) k_tail_dense(GraphDev g, TailKey tk,
-                                                    unsigned long long* tdA,
-                                                    unsigned long long* tdAD) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint64_t warp = (blockIdx.x * uint64_t(blockDim.x) + threadIdx.x) >> 5;
-  const uint64_t nwarps = (uint64_t(gridDim.x) * blockDim.x) >> 5;
-  const uint32_t nh = g.n_hubs[tk.da];
-  const uint32_t b0 = __ldg(g.bucket_off + tk.lp), b1 = __ldg(g.bucket_off + tk.lp + 1);
-  for (uint64_t h = warp; h < nh; h += nwarps) {
-    const uint32_t y = __ldg(g.hub_vid[tk.da] + h);
-    if (y < b0 || y >= b1) continue;
-    uint32_t s, e;
-    slice_of(g, tk.da, y, tk.la, s, e);
-    unsigned long long sa = 0, sd = 0;
-    for (uint32_t q = s + lane; q < e; q += 32) {
+// A block takes TA_V vertices of one key's bucket: short slices by a thread
+// each, longer ones by a warp, the longest by the block (hubs come first in a
+// bucket).  The slices of a block are one range of adj and their lengths come
+// from one label's offsets, so a table costs a pass over the edges between two
+// labels.  Tables for hubs only, a key per launch and a warp per hub, took 27
+// launches and 2.4 ms in a batch of 64 queries, and the other vertices' sums
+// were filled in by whichever candidate came first.
+constexpr int TA_BLOCK = 256, TA_V = 256;
+constexpr uint32_t TA_WARP = 16, TA_ALL = 2048;  // slices above: a warp each, the block
+
+__global__ void __launch_bounds__(TA_BLOCK) k_tail_table(GraphDev g, const TailKey* keys,
+                                                         ulonglong2* agg) {
+  const TailKey tk = keys[blockIdx.y];
+  const uint32_t b1 = __ldg(g.bucket_off + tk.lp + 1), lane = threadIdx.x & 31;
+  const uint64_t v0 = tk.b0 + uint64_t(blockIdx.x) * TA_V;
+  if (tk.base == ~0ull || v0 >= b1) return;
+  const uint32_t nv = min(uint32_t(TA_V), uint32_t(b1 - v0));
+  ulonglong2* out = agg + tk.base + (v0 - tk.b0);
+  __shared__ uint32_t s_long[TA_V], s_all[TA_V], n_long, n_all;
+  __shared__ unsigned long long s_a, s_d;
+  if (threadIdx.x == 0) n_long = n_all = 0;
+  __syncthreads();
+  auto sum = [&](uint32_t s, uint32_t e, uint32_t at, uint32_t step, unsigned long long& a,
+                 unsigned long long& d) {
+    for (uint32_t q = s + at; q < e; q += step) {
       const uint32_t x = __ldg(g.adj[tk.da] + q);
       uint32_t xs, xe;
       slice_of(g, tk.db, x, tk.lb, xs, xe);
-      sd += xe - xs;
-      sa += xe - xs - ((tk.la == tk.lb && has_self(g, x)) ? 1u : 0u);
+      d += xe - xs;
+      a += xe - xs - ((tk.la == tk.lb && has_self(g, x)) ? 1u : 0u);
     }
-    sa = warp_sum(sa);
-    sd = warp_sum(sd);
+  };
+  uint32_t s = 0, e = 0;
+  if (threadIdx.x < nv) {
+    slice_of(g, tk.da, uint32_t(v0) + threadIdx.x, tk.la, s, e);
+    if (e - s <= TA_WARP) {
+      unsigned long long a = 0, d = 0;
+      sum(s, e, 0, 1, a, d);
+      out[threadIdx.x] = make_ulonglong2(a, d);
+    } else if (e - s <= TA_ALL) {
+      s_long[atomicAdd(&n_long, 1u)] = threadIdx.x;
+    } else {
+      s_all[atomicAdd(&n_all, 1u)] = threadIdx.x;
+    }
+  }
+  __syncthreads();
+  for (uint32_t j = threadIdx.x >> 5; j < n_long; j += TA_BLOCK / 32) {
+    unsigned long long a = 0, d = 0;
+    slice_of(g, tk.da, uint32_t(v0) + s_long[j], tk.la, s, e);
+    sum(s, e, lane, 32, a, d);
+    a = warp_sum(a);
+    d = warp_sum(d);
+    if (lane == 0) out[s_long[j]] = make_ulonglong2(a, d);
+  }
+  for (uint32_t j = 0; j < n_all; ++j) {
+    if (threadIdx.x == 0) s_a = s_d = 0;
+    __syncthreads();
+    unsigned long long a = 0, d = 0;
+    slice_of(g, tk.da, uint32_t(v0) + s_all[j], tk.la, s, e);
+    sum(s, e, threadIdx.x, TA_BLOCK, a, d);
+    a = warp_sum(a);
+    d = warp_sum(d);
     if (lane == 0) {
-      tdA[tk.base + h] = sa;
-      tdAD[tk.base + h] = sd;
+      atomicAdd(&s_a, a);
+      atomicAdd(&s_d, d);
     }
+    __syncthreads();
+    if (threadIdx.x == 0) out[s_all[j]] = make_ulonglong2(s_a, s_d);
+    __syncthreads();
   }
 }
 
-// Two-hop aggregates A(m_p), AD(m_p) of a tail (see k_tail_dense): from the
-// hub table when m_p is a hub; otherwise from the key's lazy table over the
-// bucket of label l_p, filled on first use by whichever thread needs the
-// entry (A and AD packed in one 64-bit word, so a reader sees an entry whole
-// or not at all; concurrent fillers store the same value), or summed over the
-// label-l_a slice [s, e) when the entry cannot be tabled.  Entries whose AD
-// does not fit 32 bits are never tabled.
+// Two-hop aggregates A(m_p), AD(m_p) of a tail (see k_tail_table): from the
+// key's table, or summed over the label-l_a slice [s, e) when it has none.
 __device__ __forceinline__ void tail_agg(const StepArgs& a, const PlanDev& P, uint32_t mp,
                                          uint32_t s, uint32_t e, long long& c, long long& d) {
   const GraphDev& g = a.g;
-  const uint32_t da = P.tail_da, db = P.tail_db;
   const TailKey& tk = a.tkeys[P.tail_kid];
-  if (tk.base != ~0ull && g.hub_slot[da]) {
-    const uint16_t h = __ldg(g.hub_slot[da] + mp);
-    if (h != NO_HUB) {
-      c = (long long)a.tdA[tk.base + h];
-      d = (long long)a.tdAD[tk.base + h];
-      return;
-    }
-  }
-  unsigned long long* slot = nullptr;
-  if (tk.lazy != ~0ull) {
-    slot = a.tdL + tk.lazy + (mp - tk.b0);
-    const unsigned long long w = *reinterpret_cast<volatile unsigned long long*>(slot);
-    if (w != ~0ull) {
-      c = (long long)(w & 0xFFFFFFFFull);
-      d = (long long)(w >> 32);
-      return;
-    }
+  const uint64_t base = tk.base;
+  if (base != ~0ull) {
+    const ulonglong2 w = __ldg(a.tail_agg + base + (mp - tk.b0));
+    c = (long long)w.x;
+    d = (long long)w.y;
+    return;
   }
   const uint32_t la = tk.la, lb = tk.lb;
   c = d = 0;
   for (uint32_t j = s; j < e; ++j) {
-    const uint32_t x = __ldg(g.adj[da] + j);
+    const uint32_t x = __ldg(g.adj[P.tail_da] + j);
     uint32_t xs, xe;
-    slice_of(g, db, x, lb, xs, xe);
+    slice_of(g, P.tail_db, x, lb, xs, xe);
     d += xe - xs;
     c += (long long)(xe - xs) - ((la == lb && has_self(g, x)) ? 1 : 0);
   }
-  if (slot && d < 0xFFFFFFFFll)
-    atomicExch(slot, (unsigned long long)(d) << 32 | (unsigned long long)(c));
+}
+
+// z in the slice [s, e) of y's d-adjacency (z carries that slice's label), where
+// y, of label ylab, is the candidate at hand (`cur`) or a vertex of its row and
+// z a vertex of the row.  In a symmetric graph the question is put to the row's
+// vertex, whose hub row or slice all candidates of the row share.
+__device__ __forceinline__ bool joined(const StepArgs& a, uint32_t d, uint32_t y, uint32_t ylab,
+                                       bool cur, uint32_t s, uint32_t e, uint32_t z) {
+  if (cur && z != y && a.g.symmetric) return in_slice(a.g, d, z, ylab, y, a.probe_min);
+  return in_slice_se(a.g, d, y, s, e, z, a.probe_min);
 }
 
 // Closed-form count of one prefix of length a = k-2 under a two-position
@@ -470,8 +503,8 @@ __device__ __forceinline__ void tail_agg(const StepArgs& a, const PlanDev& P, ui
 // position j < a.
 template <class Col>
 __device__ __forceinline__ void tail_close(const StepArgs& a, const PlanDev& P, Col col,
-                                           uint32_t mp, uint32_t s, uint32_t e, long long c,
-                                           long long d, unsigned long long& cnt,
+                                           uint32_t mp, bool cur, uint32_t s, uint32_t e,
+                                           long long c, long long d, unsigned long long& cnt,
                                            unsigned long long& pre, unsigned long long& dsum) {
   const GraphDev& g = a.g;
   const uint32_t ia = P.k - 2;
@@ -481,7 +514,7 @@ __device__ __forceinline__ void tail_close(const StepArgs& a, const PlanDev& P, 
   for (uint32_t mi = P.tail_Ia; mi; mi &= mi - 1) {
     const uint32_t i2 = __ffs(mi) - 1;
     const uint32_t x = col(i2);
-    if (!in_slice_se(g, da, mp, s, e, x, a.probe_min)) continue;
+    if (!joined(a, da, mp, P.label[P.tail_p], cur, s, e, x)) continue;
     inS += 1;
     uint32_t xs, xe;
     slice_of(g, db, x, lb, xs, xe);
@@ -511,7 +544,7 @@ __device__ __forceinline__ void tail_close(const StepArgs& a, const PlanDev& P, 
 // prefix of length k-1 (count-mode definition: 8 for the last position).
 // col(j) is the vertex matched at position j < k-2.
 template <class Col>
-__device__ __forceinline__ void star_close(const StepArgs& a, const PlanDev& P, Col col,
+__device__ __forceinline__ void star_close(const StepArgs& a, const PlanDev& P, Col col, bool cur,
                                            unsigned long long& cnt, unsigned long long& pre,
                                            unsigned long long& bal,
                                            unsigned long long& balc) {
@@ -522,7 +555,7 @@ __device__ __forceinline__ void star_close(const StepArgs& a, const PlanDev& P, 
   slice_of(g, d, mp, P.label[ia], sa, ea);
   unsigned long long A = ea - sa;
   for (uint32_t m = P.samelab[ia]; m; m &= m - 1)
-    if (in_slice_se(g, d, mp, sa, ea, col(__ffs(m) - 1), a.probe_min)) A -= 1;
+    if (joined(a, d, mp, P.label[P.star_p], cur, sa, ea, col(__ffs(m) - 1))) A -= 1;
   unsigned long long lb_len;
   if (P.label[ib] == P.label[ia]) {
     cnt = A ? A * (A - 1) : 0ull;
@@ -532,7 +565,7 @@ __device__ __forceinline__ void star_close(const StepArgs& a, const PlanDev& P, 
     slice_of(g, d, mp, P.label[ib], sb, eb);
     unsigned long long B = eb - sb;
     for (uint32_t m = P.samelab[ib]; m; m &= m - 1)
-      if (in_slice_se(g, d, mp, sb, eb, col(__ffs(m) - 1), a.probe_min)) B -= 1;
+      if (joined(a, d, mp, P.label[P.star_p], cur, sb, eb, col(__ffs(m) - 1))) B -= 1;
     cnt = A * B;
     lb_len = eb - sb;
   }
@@ -584,8 +617,8 @@ __device__ __forceinline__ uint32_t row_work(const StepArgs& a, const PlanDev& P
     }
     chc = (i + 1 == P.k && P.last_o1) ? 8ull : ch;
   }
-  if (a.q_budget && best) {
-    // Per-query budget: a query whose scheduled elements pass the budget
+  if (a.q_budget && best && a.in.qid) {
+    // Per-query budget (a batch's rows; one query's are charged by the tile): a query whose scheduled elements pass the budget
     // stops expanding (its count is reported as unknown).
     const unsigned long long before = atomicAdd(&a.q_elems[q], (unsigned long long)best);
     if (before + best > a.q_budget) best = 0;
@@ -827,8 +860,8 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
           // The prefix ending in x has length k-2 and the plan ends in two
           // leaves of one anchor: counted here, not stored.
           unsigned long long tc, tp, tb, tbc;
-          star_close(a, P, [&](uint32_t j) { return j == i ? x : a.in.col[j][rr]; }, tc, tp, tb,
-                     tbc);
+          star_close(a, P, [&](uint32_t j) { return j == i ? x : a.in.col[j][rr]; },
+                     P.star_p == i, tc, tp, tb, tbc);
           cnt += tc;
           sk += tc;
           s2 += tp;
@@ -843,8 +876,8 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
           long long ac, ad;
           tail_agg(a, P, mp, ts, ten, ac, ad);
           unsigned long long tc, tp, td;
-          tail_close(a, P, [&](uint32_t j) { return j == i ? x : a.in.col[j][rr]; }, mp, ts, ten,
-                     ac, ad, tc, tp, td);
+          tail_close(a, P, [&](uint32_t j) { return j == i ? x : a.in.col[j][rr]; }, mp,
+                     P.tail_p == i, ts, ten, ac, ad, tc, tp, td);
           cnt += tc;
           sk += tc;
           s2 += tp;
@@ -857,7 +890,7 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
           const uint32_t y = pos == i ? x : a.in.col[pos][rr];
           uint32_t s, en;
           slice_of(g, dir, y, P.label[kl], s, en);
-          unsigned long long c1 = en - s;
+          uint32_t c1 = en - s;
           bal += 8ull + 4ull * c1;
           balc += 8ull;
           for (uint32_t m = P.samelab[kl]; m; m &= m - 1) {
@@ -866,7 +899,7 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
               c1 -= 1;
             } else {
               const uint32_t mj = j == i ? x : a.in.col[j][rr];
-              c1 -= in_slice_se(g, dir, y, s, en, mj, a.probe_min) ? 1ull : 0ull;
+              c1 -= joined(a, dir, y, P.label[pos], pos == i, s, en, mj) ? 1u : 0u;
             }
           }
           sk += c1;
@@ -1245,7 +1278,18 @@ __global__ void __launch_bounds__(256) k_work_scan(StepArgs a, uint32_t epoch) {
       }
     }
     unsigned long long tot;
-    const unsigned long long ex = block_exclusive_scan(sum, &tot);
+    unsigned long long ex = block_exclusive_scan(sum, &tot);
+    if (a.q_budget && !a.in.qid) {
+      // One query: a tile whose elements pass its budget is not expanded (the
+      // count is reported as unknown).
+      if (threadIdx.x == 0) s_prefix = atomicAdd(&a.q_elems[0], tot);
+      __syncthreads();
+      if (s_prefix + tot > a.q_budget) {
+        tot = ex = 0;
+        for (int j = 0; j < 4; ++j) v[j] = 0;
+      }
+      __syncthreads();
+    }
     if (threadIdx.x < 32) {
       if (threadIdx.x == 0)
         atomicExch(a.scan_status + tile, lb_word(epoch, tile == 0 ? LB_INC : LB_AGG, tot));
@@ -1501,62 +1545,65 @@ static void launch_expand(const StepArgs& a, int mode, unsigned grid, cudaStream
 }
 
 // Tail keys (da, la, db, lb, lp) of the plans that end in a two-position
-// pendant tail, their hub aggregate tables (one entry per hub of direction
-// da; all keys of a call share one array of at most 2^27 entries), their lazy
-// tables over the bucket of l_p (cleared here; at most 2^30 entries in all)
-// and the tail fields of `a`.  A key past either limit sums in place.
-template <class Alloc>
-static int setup_tails(DevGraph* dg, std::vector<PlanDev>& plans, TailStore& ts, Alloc alloc,
-                       cudaStream_t st, StepArgs* a, uint64_t* launches) {
+// pendant tail, their tables of two-hop aggregates over the bucket of l_p (all
+// keys of a call share one array of at most kTailEntries entries; a key past it
+// sums in place) and the tail fields of `a`.
+constexpr uint64_t kTailEntries = 1ull << 29;  // 8 GiB
+
+static int setup_tails(DevGraph* dg, std::vector<PlanDev>& plans, TailStore& ts, cudaStream_t st,
+                       StepArgs* a, uint64_t* launches) {
   std::vector<TailKey> keys;
-  uint64_t entries = 0, lazy = 0;
+  uint64_t entries = 0;
+  uint32_t widest = 0;
   for (PlanDev& p : plans) {
     if (!p.tail2) continue;
-    TailKey tk{p.tail_da, p.label[p.k - 2], p.tail_db, p.label[p.k - 1], p.label[p.tail_p], 0, 0,
-               0};
+    TailKey tk{p.tail_da, p.label[p.k - 2], p.tail_db, p.label[p.k - 1], p.label[p.tail_p], 0, 0};
     uint32_t kid = 0;
     while (kid < keys.size() && std::memcmp(&keys[kid], &tk, 20) != 0) ++kid;
     if (kid == keys.size()) {
-      const uint64_t nh = dg->g.n_hubs[tk.da];
-      tk.base = (nh && entries + nh <= (1ull << 27)) ? entries : ~0ull;
-      if (tk.base != ~0ull) entries += nh;
-      const uint64_t nb = dg->h_bucket_off[tk.lp + 1] - dg->h_bucket_off[tk.lp];
+      const uint32_t nb = dg->h_bucket_off[tk.lp + 1] - dg->h_bucket_off[tk.lp];
       tk.b0 = dg->h_bucket_off[tk.lp];
-      tk.lazy = (lazy + nb <= (1ull << 30)) ? lazy : ~0ull;
-      if (tk.lazy != ~0ull) lazy += nb;
+      tk.base = entries + nb <= kTailEntries ? entries : ~0ull;
+      if (tk.base != ~0ull) {
+        entries += nb;
+        widest = std::max(widest, nb);
+      }
       keys.push_back(tk);
     }
     p.tail_kid = kid;
   }
   if (keys.empty()) return MG_OK;
-  int rc;
-  if (ts.cap < entries) {
-    if ((rc = alloc((void**)&ts.A, entries * 8))) return rc;
-    if ((rc = alloc((void**)&ts.AD, entries * 8))) return rc;
-    ts.cap = entries;
-  }
-  if (ts.lazy_cap < lazy) {
-    if ((rc = alloc((void**)&ts.lazy, lazy * 8))) return rc;
-    ts.lazy_cap = lazy;
-  }
-  if (lazy) MG_CK(cudaMemsetAsync(ts.lazy, 0xFF, lazy * 8, st));
-  if (ts.keys_cap < keys.size()) {
-    if ((rc = alloc((void**)&ts.keys, keys.size() * sizeof(TailKey)))) return rc;
-    ts.keys_cap = uint32_t(keys.size());
+  if (ts.cap < entries || ts.keys_cap < keys.size()) {
+    const uint64_t want = std::max<uint64_t>(entries, ts.cap);
+    const uint32_t nk = std::max<uint32_t>(uint32_t(keys.size()), ts.keys_cap);
+    MG_CK(cudaStreamSynchronize(st));
+    ts.free();
+    if (cudaMalloc((void**)&ts.keys, nk * sizeof(TailKey)) != cudaSuccess) {
+      cudaGetLastError();
+      ts.keys = nullptr;
+      return set_error(MG_E_OOM, "tail keys: cudaMalloc failed");
+    }
+    ts.keys_cap = nk;
+    if (cudaMalloc((void**)&ts.agg, want * sizeof(ulonglong2)) == cudaSuccess) {
+      ts.cap = want;
+    } else {  // no room for tables: every key sums in place
+      cudaGetLastError();
+      ts.agg = nullptr;
+      for (TailKey& tk : keys) tk.base = ~0ull;
+      widest = 0;
+    }
   }
   MG_CK(cudaMemcpyAsync(ts.keys, keys.data(), keys.size() * sizeof(TailKey),
                         cudaMemcpyHostToDevice, st));
-  for (const TailKey& tk : keys) {
-    if (tk.base == ~0ull) continue;
-    k_tail_dense<<<grid_for(uint64_t(dg->g.n_hubs[tk.da]) * 32, 256, dg->sms * 16), 256, 0, st>>>(
-        dg->g, tk, ts.A, ts.AD);
+  for (uint32_t k0 = 0; widest && k0 < keys.size(); k0 += 65535) {
+    const uint32_t nk = std::min<uint32_t>(uint32_t(keys.size()) - k0, 65535);
+    k_tail_table<<<dim3((widest + TA_V - 1) / TA_V, nk), TA_BLOCK, 0, st>>>(dg->g, ts.keys + k0,
+                                                                           ts.agg);
     ++*launches;
   }
   MG_CK(cudaGetLastError());
   a->tail_dense = 1;
-  a->tdA = ts.A;
-  a->tdAD = ts.AD;
-  a->tdL = ts.lazy;
+  a->tail_agg = ts.agg;
   a->tkeys = ts.keys;
   return MG_OK;
 }
@@ -1882,10 +1929,7 @@ static int run_levels(DevGraph* dg, std::vector<PlanDev> plans, bool count_mode,
   // Pendant tails counted in closed form (count mode): tail-key table and
   // memo table of two-hop aggregates, shared by every query of the call.
   if (count_mode && o.no_tail != 1) {
-    rc = setup_tails(dg, plans, ws->tails,
-                     [&](void** p, size_t bytes) { return ws_alloc(ws, p, bytes); }, st, &a,
-                     &res->launches);
-    if (rc) return rc;
+    if ((rc = setup_tails(dg, plans, ws->tails, st, &a, &res->launches))) return rc;
   }
   a.star = count_mode && o.no_tail != 1;
   if (batch) {
@@ -2145,6 +2189,7 @@ void free_lanes(LaneSet* ls) {
   for (Lane& l : ls->lanes)
     if (l.st) cudaStreamDestroy(l.st);
   for (void* p : ls->allocs) cudaFree(p);
+  ls->tails.free();
   if (ls->ev_start) cudaEventDestroy(ls->ev_start);
   if (ls->ev_end) cudaEventDestroy(ls->ev_end);
   delete ls;
@@ -2236,10 +2281,7 @@ static int subiso_batch_lanes(DevGraph* dg, std::vector<PlanDev>& plans, const m
   // Pendant tails closed from hub aggregates (their table is filled on the
   // graph's stream before the lanes start).
   if (o.no_tail != 1) {
-    rc = setup_tails(dg, plans, ls->tails,
-                     [&](void** p, size_t bytes) { return lane_alloc(ls, p, bytes); }, st, &a,
-                     &res->launches);
-    if (rc) return rc;
+    if ((rc = setup_tails(dg, plans, ls->tails, st, &a, &res->launches))) return rc;
   } else {
     for (PlanDev& p : plans) p.tail2 = 0;
   }
