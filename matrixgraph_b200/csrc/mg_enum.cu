@@ -57,10 +57,10 @@ struct TailStore {
 };
 
 struct Workspace {
-  int device = 0;
-  uint64_t cap = 0;       // rows per level table (and elements per chunk)
-  uint32_t rows0 = 0;     // capacity of the level-0 table (one row per query)
-  int levels = 0;         // level tables allocated: 0..levels-1
+  // Level tables: rows[l] rows of prefix length l, all arrays of a level in one
+  // block; they grow when a call needs more (ensure_level).
+  uint64_t rows[MAXK] = {};
+  void* block[MAXK] = {};
   uint32_t* col[MAXK][MAXK] = {};
   uint32_t* qid[MAXK] = {};
   uint64_t* woff[MAXK] = {};
@@ -76,14 +76,12 @@ struct Workspace {
   // Results of a call of nq queries, one block: counters (C_NUM), counts (nq),
   // rows per prefix length (nq * (MAXK + 1)), elements scheduled (nq).
   unsigned long long* res = nullptr;
-  uint32_t res_cap = 0;                  // queries
-  unsigned long long* h_res = nullptr;   // pinned mirror of one query's block
-  PlanDev* h_plan = nullptr;             // pinned, one plan
   PlanDev* plans = nullptr;
-  uint32_t plans_cap = 0;
+  uint32_t nq_cap = 0;                   // queries that res and plans hold
+  // Pinned: one plan, and a mirror of one query's result block.
+  PlanDev* h_plan = nullptr;
+  unsigned long long* h_res = nullptr;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr, ev2 = nullptr, ev3 = nullptr;
-  std::vector<void*> allocs;
-  uint64_t bytes = 0;
 };
 
 // Counter slots.  A level's slots lie together, so that clearing everything
@@ -102,29 +100,27 @@ constexpr int lvl_slot(int l, int what) { return C_LVL + 4 * l + what; }
 
 void free_workspace(Workspace* ws) {
   if (!ws) return;
-  for (void* p : ws->allocs) cudaFree(p);
+  for (void* p : ws->block) cudaFree(p);
+  for (void* p : {(void*)ws->tile_row, (void*)ws->status, (void*)ws->root_keep, (void*)ws->res,
+                  (void*)ws->plans})
+    cudaFree(p);
   ws->tails.free();
-  if (ws->h_res) cudaFreeHost(ws->h_res);
   if (ws->h_plan) cudaFreeHost(ws->h_plan);
-  if (ws->ev0) cudaEventDestroy(ws->ev0);
-  if (ws->ev1) cudaEventDestroy(ws->ev1);
-  if (ws->ev2) cudaEventDestroy(ws->ev2);
-  if (ws->ev3) cudaEventDestroy(ws->ev3);
+  for (cudaEvent_t e : {ws->ev0, ws->ev1, ws->ev2, ws->ev3})
+    if (e) cudaEventDestroy(e);
   delete ws;
 }
 
-static int ws_alloc(Workspace* ws, void** p, size_t bytes) {
+// Replaces *p by `bytes` of device memory (contents are lost).
+static int ws_alloc(void** p, size_t bytes) {
+  cudaFree(*p);
   *p = nullptr;
-  cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    *p = nullptr;
-    return set_error(MG_E_OOM, "enumeration scratch: cudaMalloc(%zu) failed: %s", bytes,
-                     cudaGetErrorString(e));
-  }
-  ws->allocs.push_back(*p);
-  ws->bytes += bytes;
-  return MG_OK;
+  const cudaError_t e = cudaMalloc(p, std::max<size_t>(bytes, 16));
+  if (e == cudaSuccess) return MG_OK;
+  cudaGetLastError();
+  *p = nullptr;
+  return set_error(MG_E_OOM, "enumeration scratch: cudaMalloc(%zu) failed: %s", bytes,
+                   cudaGetErrorString(e));
 }
 
 constexpr uint64_t kDefaultCap = 1ull << 24;
@@ -141,47 +137,59 @@ constexpr uint64_t res_words(uint64_t nq) { return C_NUM + nq * (MAXK + 3); }
 
 static uint64_t level_row_bytes(int l) { return uint64_t(l) * 4 + 4 + 4 + 8 + 4 + 1; }
 
-static int ensure_ws(DevGraph* dg, uint64_t cap, int levels, uint32_t nq) {
+// Rows that a level table starts with.  Tables for 2^24 rows at once (the most
+// a level holds by default) cost 2 GB and 12 ms of allocation in a graph's first
+// calls and 10 ms when it is freed; most queries need a small part of them.
+constexpr uint64_t kFirstRows = 1ull << 17;
+
+// Makes room for `rows` rows of prefix length l (the table's contents are lost).
+static int ensure_level(Workspace* ws, int l, uint64_t rows) {
+  if (ws->rows[l] >= rows) return MG_OK;
+  auto pad = [](uint64_t b) { return (b + 255) & ~uint64_t(255); };
+  const uint64_t words = pad(rows * 4), offs = pad((rows + 1) * 8);
+  ws->rows[l] = 0;
+  int rc = ws_alloc(&ws->block[l], words * (l + 2) + offs + pad(rows));
+  if (rc) return rc;
+  auto* p = static_cast<unsigned char*>(ws->block[l]);
+  auto take = [&](uint64_t bytes) {
+    unsigned char* q = p;
+    p += bytes;
+    return q;
+  };
+  for (int j = 0; j < l; ++j) ws->col[l][j] = reinterpret_cast<uint32_t*>(take(words));
+  ws->qid[l] = reinterpret_cast<uint32_t*>(take(words));
+  ws->dstart[l] = reinterpret_cast<uint32_t*>(take(words));
+  ws->woff[l] = reinterpret_cast<uint64_t*>(take(offs));
+  ws->dci[l] = take(pad(rows));
+  ws->rows[l] = rows;
+  return MG_OK;
+}
+
+// Scratch of a walk with level tables of at most `cap` rows for nq queries.
+static int ensure_ws(DevGraph* dg, uint64_t cap, uint32_t nq) {
   Workspace*& ws = dg->ws;
-  if (ws && (ws->cap != cap || ws->rows0 < nq)) {
-    cudaStreamSynchronize(dg->stream);
-    free_workspace(ws);
-    ws = nullptr;
-  }
+  int rc;
   if (!ws) {
     ws = new Workspace();
-    ws->device = dg->device;
-    ws->cap = cap;
-    ws->rows0 = std::max<uint32_t>(nq, 1024);
-    int rc;
-    MG_CK(cudaMallocHost((void**)&ws->h_res, res_words(1) * 8));
-    MG_CK(cudaMallocHost((void**)&ws->h_plan, sizeof(PlanDev)));
-    MG_CK(cudaEventCreate(&ws->ev0));
-    MG_CK(cudaEventCreate(&ws->ev1));
-    MG_CK(cudaEventCreate(&ws->ev2));
-    MG_CK(cudaEventCreate(&ws->ev3));
-    const uint64_t status = (std::max<uint64_t>(cap, ws->rows0) / WS_ROWS + 2) * 8;
-    if ((rc = ws_alloc(ws, (void**)&ws->status, status))) return rc;
-    ws->status_bytes = status;
+    static_assert(sizeof(PlanDev) % 8 == 0, "the result block follows the plan");
+    MG_CK(cudaMallocHost((void**)&ws->h_plan, sizeof(PlanDev) + res_words(1) * 8));
+    ws->h_res = reinterpret_cast<unsigned long long*>(ws->h_plan + 1);
+    for (cudaEvent_t* e : {&ws->ev0, &ws->ev1, &ws->ev2, &ws->ev3}) MG_CK(cudaEventCreate(e));
+    if ((rc = ws_alloc((void**)&ws->tile_row, (kSegment / EXPAND_TILE + 2) * 4))) return rc;
+  }
+  const uint64_t status = (std::max<uint64_t>(cap, nq) / WS_ROWS + 2) * 8;
+  if (ws->status_bytes < status) {
+    ws->status_bytes = 0;
+    if ((rc = ws_alloc((void**)&ws->status, status))) return rc;
     MG_CK(cudaMemsetAsync(ws->status, 0, status, dg->stream));
-    if ((rc = ws_alloc(ws, (void**)&ws->tile_row, (kSegment / EXPAND_TILE + 2) * 4))) return rc;
+    ws->status_bytes = status;
+    ws->epoch = 0;
   }
-  if (ws->res_cap < nq) {
-    int rc;
-    if ((rc = ws_alloc(ws, (void**)&ws->res, res_words(nq) * 8))) return rc;
-    if ((rc = ws_alloc(ws, (void**)&ws->plans, uint64_t(nq) * sizeof(PlanDev)))) return rc;
-    ws->res_cap = ws->plans_cap = nq;
-  }
-  for (int l = ws->levels; l < levels; ++l) {
-    const uint64_t rows = l == 0 ? ws->rows0 : cap;
-    int rc;
-    for (int j = 0; j < l; ++j)
-      if ((rc = ws_alloc(ws, (void**)&ws->col[l][j], rows * 4))) return rc;
-    if ((rc = ws_alloc(ws, (void**)&ws->qid[l], rows * 4))) return rc;
-    if ((rc = ws_alloc(ws, (void**)&ws->woff[l], (rows + 1) * 8))) return rc;
-    if ((rc = ws_alloc(ws, (void**)&ws->dstart[l], rows * 4))) return rc;
-    if ((rc = ws_alloc(ws, (void**)&ws->dci[l], rows))) return rc;
-    ws->levels = l + 1;
+  if (ws->nq_cap < nq) {
+    ws->nq_cap = 0;
+    if ((rc = ws_alloc((void**)&ws->res, res_words(nq) * 8))) return rc;
+    if ((rc = ws_alloc((void**)&ws->plans, uint64_t(nq) * sizeof(PlanDev)))) return rc;
+    ws->nq_cap = nq;
   }
   return MG_OK;
 }
@@ -1648,7 +1656,9 @@ static uint64_t bounded_product(uint64_t a, uint64_t b) {
 
 // Scratch of a walk over the levels.
 struct WalkBufs {
-  uint64_t cap = 0;  // rows per level table
+  uint64_t cap = 0;  // rows per level table, at most
+  const uint64_t* rows = nullptr;  // rows that each table holds now (nullptr: cap)
+  Workspace* grow = nullptr;       // whose tables can grow up to cap
   uint32_t* (*col)[MAXK] = nullptr;
   uint32_t** qid = nullptr;  // nullptr: single queries only
   uint64_t** woff = nullptr;
@@ -1703,7 +1713,6 @@ static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool cou
   a.counts = B.res + C_NUM;
   a.lvl_rows = a.counts + nq;
   a.q_elems = a.lvl_rows + uint64_t(nq) * (MAXK + 1);
-  a.cap_rows = B.cap;
   a.seg_cap = B.seg;
   a.tile_row = B.tile_row;
   a.scan_status = B.status;
@@ -1715,8 +1724,10 @@ static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool cou
   R[0] = nq;
   int rc;
 
+  auto held = [&](int l) { return B.rows ? std::min(B.rows[l], B.cap) : B.cap; };
   auto set_level = [&](int l) {
     a.level = uint32_t(l);
+    a.cap_rows = l == 0 ? nq : held(l);
     auto tab = [&](int x) {
       TabPtrs t{};
       for (int j = 0; j < x; ++j) t.col[j] = B.col[x][j];
@@ -1728,7 +1739,7 @@ static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool cou
     a.dstart = B.dstart[l];
     a.dci = B.dci[l];
     a.out = writes[l] ? tab(l + 1) : TabPtrs{};
-    a.out_cap = writes[l] ? B.cap : 0;
+    a.out_cap = writes[l] ? held(l + 1) : 0;
     a.out_slot = lvl_slot(l, L_OUT);
     a.tile_slot = lvl_slot(l, L_TILE);
   };
@@ -1756,7 +1767,7 @@ static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool cou
     a.dev = 1;
     for (int l = l0; l <= last; ++l) {
       set_level(l);
-      a.t_limit = writes[l] ? std::min(B.cap, B.seg) : B.seg;
+      a.t_limit = writes[l] ? std::min(held(l + 1), B.seg) : B.seg;
       if (one && o.max_elements) a.t_limit = std::min(a.t_limit, o.max_elements - elements);
       if (++*B.epoch > kEpochMax) {
         MG_CK(cudaMemsetAsync(B.status, 0, B.status_bytes, st));
@@ -1766,7 +1777,7 @@ static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool cou
       res->launches++;
       const uint64_t bound = std::min(bounded_product(rows, widest[l]), a.t_limit);
       if (int r = expand(l, bound)) return r;
-      rows = std::min(bound, B.cap);
+      rows = bound;
     }
     return MG_OK;
   };
@@ -1803,6 +1814,12 @@ static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool cou
 
   int top = -1;
   bool waited = false;
+  if (B.grow) {
+    if (!one && (rc = ensure_level(B.grow, 0, nq))) return rc;
+    for (int l = 1; l <= last; ++l)
+      if ((rc = ensure_level(B.grow, l, std::min(B.cap, kFirstRows)))) return rc;
+  }
+  if (!one) k_iota<<<grid_for(nq, 256, 1024), 256, 0, st>>>(B.qid[0], nq);
   if (one && last >= 0) {
     T[0] = a.T0 = root_range(dg, plans[0], a, &a.root_first);
     res->balg += T[0] * root_charge(dg);
@@ -1819,7 +1836,18 @@ static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool cou
       continue;
     }
     const uint64_t t0 = cur[top];
-    const uint64_t t1 = writes[top] ? std::min(T[top], t0 + B.cap) : T[top];
+    if (writes[top] && B.grow && held(top + 1) < std::min(T[top] - t0, B.cap)) {
+      // The next table grows to what this level needs (nothing below this level
+      // is in use, the stream is idle); without memory the level is chunked.
+      uint64_t want = kFirstRows;
+      while (want < T[top] - t0 && want < B.cap) want <<= 1;
+      want = std::min(want, B.cap);
+      if (ensure_level(B.grow, top + 1, want) &&
+          (rc = ensure_level(B.grow, top + 1, std::min(B.cap, kFirstRows))))
+        return rc;
+      clear_error();
+    }
+    const uint64_t t1 = writes[top] ? std::min(T[top], t0 + held(top + 1)) : T[top];
     if (one && o.max_elements && t1 - t0 > o.max_elements - elements) return refuse();
     elements += t1 - t0;
     if (waited)  // the slots of this level and below
@@ -1840,7 +1868,7 @@ static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool cou
     }
     res->chunks++;
     cur[top] = t1;
-    if ((rc = descend(top + 1, std::min(t1 - t0, B.cap)))) return rc;
+    if ((rc = descend(top + 1, t1 - t0))) return rc;
     int stop;
     if ((rc = settle(top + 1, &stop))) return rc;
     waited = true;
@@ -1880,9 +1908,19 @@ static int run_levels(DevGraph* dg, std::vector<PlanDev> plans, bool count_mode,
       if (cap == 0) return set_error(MG_E_OOM, "memory budget below one row per level");
     }
   }
-  int rc = ensure_ws(dg, cap, int(kmax), nq);
+  int rc = ensure_ws(dg, cap, nq);
   if (rc) return rc;
   Workspace* ws = dg->ws;
+  if (o.mem_budget_bytes) {  // tables of earlier calls count too
+    uint64_t held = 0;
+    for (int l = 0; l < MAXK; ++l) held += ws->rows[l] * level_row_bytes(l);
+    if (held > o.mem_budget_bytes)
+      for (int l = 0; l < MAXK; ++l) {
+        cudaFree(ws->block[l]);
+        ws->block[l] = nullptr;
+        ws->rows[l] = 0;
+      }
+  }
   cudaStream_t st = dg->stream;
   const bool batch = nq > 1;
   MG_CK(cudaEventRecord(ws->ev0, st));
@@ -1910,14 +1948,11 @@ static int run_levels(DevGraph* dg, std::vector<PlanDev> plans, bool count_mode,
     a.root_begin = o.root_begin;
     a.root_end = o.root_end ? o.root_end : ~0ull;
   }
-  if (batch) {
-    k_iota<<<grid_for(nq, 256, 1024), 256, 0, st>>>(ws->qid[0], nq);
-    res->launches++;
-  }
   if (o.matrix_filter && !batch && !plans[0].zero) {
     const uint64_t words = (uint64_t(dg->g.n) + 31) / 32;
     if (ws->root_keep_words < words) {
-      if ((rc = ws_alloc(ws, (void**)&ws->root_keep, words * 4))) return rc;
+      ws->root_keep_words = 0;
+      if ((rc = ws_alloc((void**)&ws->root_keep, words * 4))) return rc;
       ws->root_keep_words = words;
     }
     if ((rc = matrix_filter_roots(o.matrix_filter, dg, plans[0].perm[0], plans[0].label[0],
@@ -1942,6 +1977,8 @@ static int run_levels(DevGraph* dg, std::vector<PlanDev> plans, bool count_mode,
 
   WalkBufs B;
   B.cap = cap;
+  B.rows = ws->rows;
+  B.grow = ws;
   B.col = ws->col;
   B.qid = ws->qid;
   B.woff = ws->woff;
@@ -2226,22 +2263,31 @@ static int ensure_lanes(DevGraph* dg, uint32_t nl, uint64_t cap, uint32_t kmax) 
   int rc;
   for (Lane& L : ls->lanes) {
     MG_CK(cudaStreamCreateWithFlags(&L.st, cudaStreamNonBlocking));
-    if ((rc = lane_alloc(ls, (void**)&L.ctr, C_NUM * 8))) return rc;
-    if ((rc = lane_alloc(ls, (void**)&L.counts, 8))) return rc;
-    if ((rc = lane_alloc(ls, (void**)&L.lvl, (MAXK + 1) * 8))) return rc;
-    if ((rc = lane_alloc(ls, (void**)&L.qel, 8))) return rc;
     const uint64_t ntiles = cap / WS_ROWS + 2;
-    if ((rc = lane_alloc(ls, (void**)&L.status, ntiles * 8))) return rc;
-    MG_CK(cudaMemset(L.status, 0, ntiles * 8));
-    if ((rc = lane_alloc(ls, (void**)&L.tile_row, (ls->seg_cap / EXPAND_TILE + 2) * 4))) return rc;
-    for (uint32_t l = 0; l < ls->kmax; ++l) {
-      const uint64_t rows = l == 0 ? 1 : cap;
-      for (uint32_t j = 0; j < l; ++j)
-        if ((rc = lane_alloc(ls, (void**)&L.col[l][j], rows * 4))) return rc;
-      if ((rc = lane_alloc(ls, (void**)&L.woff[l], (rows + 1) * 8))) return rc;
-      if ((rc = lane_alloc(ls, (void**)&L.dstart[l], rows * 4))) return rc;
-      if ((rc = lane_alloc(ls, (void**)&L.dci[l], rows))) return rc;
+    // All arrays of a lane in one block: measured first, then carved.
+    unsigned char* p = nullptr;
+    for (int pass = 0; pass < 2; ++pass) {
+      uint64_t off = 0;
+      auto take = [&](auto** array, uint64_t bytes) {
+        if (p) *array = reinterpret_cast<std::remove_reference_t<decltype(**array)>*>(p + off);
+        off += (bytes + 255) & ~uint64_t(255);
+      };
+      take(&L.ctr, C_NUM * 8);
+      take(&L.counts, 8);
+      take(&L.lvl, (MAXK + 1) * 8);
+      take(&L.qel, 8);
+      take(&L.status, ntiles * 8);
+      take(&L.tile_row, (ls->seg_cap / EXPAND_TILE + 2) * 4);
+      for (uint32_t l = 0; l < ls->kmax; ++l) {
+        const uint64_t rows = l == 0 ? 1 : cap;
+        for (uint32_t j = 0; j < l; ++j) take(&L.col[l][j], rows * 4);
+        take(&L.woff[l], (rows + 1) * 8);
+        take(&L.dstart[l], rows * 4);
+        take(&L.dci[l], rows);
+      }
+      if (pass == 0 && (rc = lane_alloc(ls, (void**)&p, off))) return rc;
     }
+    MG_CK(cudaMemset(L.status, 0, ntiles * 8));
   }
   return MG_OK;
 }
@@ -2273,7 +2319,7 @@ static int subiso_batch_lanes(DevGraph* dg, std::vector<PlanDev>& plans, const m
     ls->r_cap = nq;
   }
   Workspace* ws = dg->ws;  // timing events live with the graph's workspace
-  if (!ws && (rc = ensure_ws(dg, 1ull << 16, 1, 1))) return rc;
+  if (!ws && (rc = ensure_ws(dg, 1ull << 16, 1))) return rc;
   ws = dg->ws;
   MG_CK(cudaEventRecord(ws->ev0, st));
   StepArgs a;
