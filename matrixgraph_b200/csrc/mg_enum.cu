@@ -684,7 +684,21 @@ enum : int {
   X_FUSED = 4,  // the last position (one backward slice) is closed in place
   X_TAIL = 8,   // a two-position pendant tail is closed from dense aggregates
   X_ONE = 16,   // one query, no row query ids: its plan is staged in shared memory
+  X_DIRECT = 32,  // with X_ONE and X_FUSED or X_TAIL: nearly every candidate survives
+                  // and is closed where it is found (see direct_sides)
 };
+
+// Positions of a row whose matches may lie in the slice that closes a candidate
+// at position i (FUSED: of the last position, TAIL: of position k-2), and that
+// have to be looked up per candidate: the slice is the candidate's own (anchor
+// i), or the candidate itself may lie in an earlier vertex's slice.
+__host__ __device__ __forceinline__ uint32_t direct_sides(const PlanDev& P, uint32_t i, bool tail) {
+  const uint32_t earlier = (1u << i) - 1;
+  if (tail) return P.tail_Ia & earlier;
+  const uint32_t kl = P.k - 1, pos = P.cons[kl][0] & 0xFF, open = P.samelab[kl] & ~P.guar[kl];
+  if (pos == i) return open & earlier;
+  return (open >> i) & 1u ? 1u << pos : 0u;
+}
 
 // One set-up row of an expand task (shared memory, a row per slot).  A further
 // constraint is probed at p: the hub bitmap row of its vertex (len HUB_LEN), or
@@ -699,7 +713,9 @@ struct alignas(16) XRow {
   uint32_t len1, m1;
   uint32_t q, ci, v0;    // query; driving constraint; bucket row: element e is
   uint32_t end;          // vertex v0 + e * root_step
-  uint32_t pad[4];
+  uint32_t raw, free;    // X_DIRECT, slice of an earlier vertex: its entries, and
+                         // those that no earlier match takes
+  uint32_t pad[2];
 };
 constexpr uint32_t HUB_LEN = FULL;
 
@@ -733,6 +749,7 @@ __device__ __forceinline__ void probe_all(const uint32_t* const (&p)[U], const u
 #pragma unroll
   for (int u = 0; u < U; ++u) {
     w[u] = __ldg(p[u] + (len[u] == HUB_LEN ? x[u] >> 5 : 0u));
+    ok[u] = ok[u] && len[u];  // nothing lies in an empty slice
     if (len[u] != HUB_LEN && ok[u]) longest = max(longest, len[u]);
   }
   longest = __reduce_max_sync(FULL, longest);
@@ -757,7 +774,7 @@ __device__ __forceinline__ void probe_all(const uint32_t* const (&p)[U], const u
 #pragma unroll
     for (int u = 0; u < U; ++u) {
       const uint32_t v = __ldg(p[u] + at[u]);
-      if (len[u] != HUB_LEN) ok[u] = ok[u] && len[u] && v == x[u];
+      if (len[u] != HUB_LEN) ok[u] = ok[u] && v == x[u];
     }
   }
 #pragma unroll
@@ -788,11 +805,18 @@ __device__ __forceinline__ void probe_all(const uint32_t* const (&p)[U], const u
 // blocks per SM (64 registers) were the best of 1-4 and 3-6: more candidates
 // spill, fewer expose the probe latency.  Walking each row by its own, 32-128
 // candidates at a time, was no better (11.3-12.5 ms for the 4-cycle).
+//
+// X_DIRECT leaves the staging out where nearly every candidate survives and is
+// closed at once, with its look-ups done like the probes of the others:
+// instructions per candidate were what bounded those launches (275 per 32
+// candidates, 71% issue).  R-MAT scale 18, 5-paths whose ends share a label:
+// 90 -> 184 and 47 -> 191 G candidates/s; scale 22, 5-path: 6.5 -> 5.5 ms.
 template <int MODE>
 __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
   constexpr bool ONE = (MODE & X_ONE) != 0;
   // Launches that only count complete matches keep nothing of a survivor.
-  constexpr bool STAGE = (MODE & (X_WRITE | X_EMIT | X_FUSED | X_TAIL)) != 0 || !ONE;
+  constexpr bool DIRECT = (MODE & X_DIRECT) != 0;
+  constexpr bool STAGE = ((MODE & (X_WRITE | X_EMIT | X_FUSED | X_TAIL)) != 0 || !ONE) && !DIRECT;
   constexpr int XU = 2;
   const uint32_t i = a.level;
   const GraphDev& g = a.g;
@@ -827,6 +851,16 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
   const uint32_t others = ONE ? plan(0).ncons[i] - (plan(0).ncons[i] ? 1u : 0u) : 3u;
   const uint32_t sames = ONE ? __popc(plan(0).samelab[i]) : 3u;
   const bool extra = (i == 0 && a.root_keep) || ((plan(0).selfloop_mask >> i) & 1u);
+
+  // X_DIRECT: up to two vertices of a row whose adjacency candidates are looked
+  // up in, in the slots of the further constraints (this shape has none).
+  const uint32_t sides = DIRECT ? direct_sides(plan(0), i, (MODE & X_TAIL) != 0) : 0u;
+  const uint32_t side0 = __ffs(sides) - 1, side1 = __ffs(sides & (sides - 1)) - 1;
+  const uint32_t nsides = __popc(sides);
+  const uint32_t kl = plan(0).k - 1;
+  const bool own = (plan(0).cons[kl][0] & 0xFF) == i;  // FUSED: the slice is the candidate's
+  unsigned long long d_c = 0, d_raw = 0, d_d = 0;      // sums over closed candidates
+  uint32_t d_in = 0;
 
   unsigned long long cnt = 0, bal = 0, balc = 0, s1 = 0, sk = 0, s2 = 0;
   uint32_t cnt_q = 0;
@@ -1042,11 +1076,27 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
           }
           R.p0 = R.p1 = nullptr;
           R.len0 = R.len1 = 0;
-          uint32_t c = ci == 0 ? 1u : 0u;
-          if (c < nc) {
-            probe_of(a, P.cons[i][c], lab, row, R.p0, R.len0);
-            if (++c == ci) ++c;
-            if (c < nc) probe_of(a, P.cons[i][c], lab, row, R.p1, R.len1);
+          if constexpr (DIRECT) {
+            if (nsides > 0) probe_of(a, side0, lab, row, R.p0, R.len0);
+            if (nsides > 1) probe_of(a, side1, lab, row, R.p1, R.len1);
+            if ((MODE & X_FUSED) && !own) {
+              const uint32_t y = a.in.col[P.cons[kl][0] & 0xFF][row];
+              uint32_t s, e;
+              slice_of(g, P.cons[kl][0] >> 8, y, P.label[kl], s, e);
+              R.raw = R.free = e - s;
+              for (uint32_t m2 = P.samelab[kl] & ((1u << i) - 1); m2; m2 &= m2 - 1) {
+                const uint32_t j = __ffs(m2) - 1;
+                R.free -= ((P.guar[kl] >> j) & 1u) ||
+                          in_slice_se(g, P.cons[kl][0] >> 8, y, s, e, a.in.col[j][row], a.probe_min);
+              }
+            }
+          } else {
+            uint32_t c = ci == 0 ? 1u : 0u;
+            if (c < nc) {
+              probe_of(a, P.cons[i][c], lab, row, R.p0, R.len0);
+              if (++c == ci) ++c;
+              if (c < nc) probe_of(a, P.cons[i][c], lab, row, R.p1, R.len1);
+            }
           }
           rows[__popc(act & lanemask_lt())] = R;
         }
@@ -1107,7 +1157,7 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
             for (int u = 0; u < XU; ++u)
               ok[u] = ok[u] && x[u] != rows[h[u]].m0 && x[u] != rows[h[u]].m1;
           }
-          if (others > 0 || !ONE) {
+          if (!DIRECT && (others > 0 || !ONE)) {
             const uint32_t* p[XU];
             uint32_t len[XU];
 #pragma unroll
@@ -1117,7 +1167,7 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
             }
             probe_some(p, len);
           }
-          if (others > 1 || !ONE) {
+          if (!DIRECT && (others > 1 || !ONE)) {
             const uint32_t* p[XU];
             uint32_t len[XU];
 #pragma unroll
@@ -1152,7 +1202,75 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
               if (ok[u] && ((P.selfloop_mask >> i) & 1u)) ok[u] = has_self(g, x[u]);
             }
           }
-          if constexpr (STAGE) {
+          if constexpr (DIRECT) {
+            // membership of the candidate in the sides' adjacency
+            bool in0[XU], in1[XU];
+#pragma unroll
+            for (int u = 0; u < XU; ++u) in0[u] = in1[u] = false;
+            auto look = [&](bool second, bool (&in)[XU]) {
+              const uint32_t* p[XU];
+              uint32_t len[XU];
+#pragma unroll
+              for (int u = 0; u < XU; ++u) {
+                p[u] = second ? rows[h[u]].p1 : rows[h[u]].p0;
+                len[u] = second ? rows[h[u]].len1 : rows[h[u]].len0;
+                in[u] = ok[u];
+              }
+              probe_all<XU>(p, len, x, in);
+            };
+            if (nsides > 0) look(false, in0);
+            if (nsides > 1) look(true, in1);
+            const PlanDev& P = s_plan;
+            if constexpr ((MODE & X_FUSED) != 0) {
+              const uint32_t* off = g.loff[P.cons[kl][0] >> 8] + uint64_t(P.label[kl]) * g.n;
+              const uint32_t sure = __popc(P.samelab[kl] & P.guar[kl]);
+              const bool self = own && ((P.samelab[kl] & ~P.guar[kl]) >> i & 1u);
+              uint32_t raw[XU], free[XU];
+#pragma unroll
+              for (int u = 0; u < XU; ++u) {
+                if (own) {
+                  raw[u] = __ldg(off + x[u] + 1) - __ldg(off + x[u]);
+                  free[u] = raw[u] - sure;
+                } else {
+                  raw[u] = rows[h[u]].raw;
+                  free[u] = rows[h[u]].free - ((P.samelab[kl] & P.guar[kl]) >> i & 1u);
+                }
+              }
+#pragma unroll
+              for (int u = 0; u < XU; ++u)
+                if (ok[u]) {
+                  s1 += 1;
+                  d_raw += raw[u];
+                  d_c += free[u] - (in0[u] ? 1u : 0u) - (in1[u] ? 1u : 0u) -
+                         (self && has_self(g, x[u]) ? 1u : 0u);
+                }
+            } else {
+              const uint32_t* off = g.loff[P.tail_da] + uint64_t(P.label[P.k - 2]) * g.n;
+              const uint32_t nJ = __popc(P.tail_J);
+#pragma unroll
+              for (int u = 0; u < XU; ++u) {
+                if (ok[u] && a.filters) ok[u] = pass_filters(g, P, i, x[u], a.filters);
+                if (!ok[u]) continue;
+                const uint32_t ts = __ldg(off + x[u]), te2 = __ldg(off + x[u] + 1);
+                long long ac, ad;
+                tail_agg(a, P, x[u], ts, te2, ac, ad);
+                s1 += 1;
+                d_raw += te2 - ts;
+                if (in0[u] || in1[u] || ((P.tail_Ia >> i & 1u) && has_self(g, x[u]))) {
+                  const uint32_t rr = rows[h[u]].row;
+                  unsigned long long tc, tp, td;
+                  tail_close(a, P, [&](uint32_t j) { return j == i ? x[u] : a.in.col[j][rr]; },
+                             x[u], true, ts, te2, ac, ad, tc, tp, td);
+                  d_c += tc;
+                  d_d += td;
+                  d_in += te2 - ts - uint32_t(tp);
+                } else {
+                  d_c += (unsigned long long)(ac - (long long)nJ * (te2 - ts));
+                  d_d += (unsigned long long)ad;
+                }
+              }
+            }
+          } else if constexpr (STAGE) {
 #pragma unroll
             for (int u = 0; u < XU; ++u) {
               const uint32_t km = __ballot_sync(FULL, ok[u]);
@@ -1184,6 +1302,17 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
     gbase = __shfl_sync(FULL, gbase, 0) + uint64_t(nwarps) * grab;
   }
   if (ONE && a.count_mode && s_plan.k == i + 1) cnt = s1;  // complete matches
+  if constexpr (DIRECT) {
+    cnt = sk = d_c;
+    if constexpr ((MODE & X_TAIL) != 0) {
+      s2 = d_raw - d_in;
+      balc = 8 * s1 + 4 * d_raw + 8 * s2;
+      bal = balc + 4 * d_d;
+    } else {
+      balc = 8 * s1;
+      bal = 8 * s1 + 4 * d_raw;
+    }
+  }
   acc_flush_warp(a, cnt_q, i, cnt, s1, sk, s2, true);
   bal = warp_sum(bal);
   balc = warp_sum(balc);
@@ -1535,6 +1664,14 @@ static int expand_mode(const StepArgs& a, uint32_t i, const PlanDev* plans, uint
     if (((a.tail_dense && p.tail2) || (a.star && p.star2)) && p.k == i + 3) tail = true;
     if (!count_mode && p.k == i + 1) emit = true;
   }
+  // Closed where they are found: a single query's candidates with no further
+  // constraint, when at most two vertices of a row need a look-up.  (Candidates
+  // with further constraints survive rarely and are staged first; a tail is
+  // direct when it hangs off the candidate.)
+  if (nplans == 1 && !writes && !emit && fused != tail && a.g.symmetric &&
+      plans[0].ncons[i] <= 1 && (fused || (plans[0].tail2 && plans[0].tail_p == i)) &&
+      __builtin_popcount(direct_sides(plans[0], i, tail)) <= 2)
+    return X_DIRECT | X_ONE | (fused ? X_FUSED : X_TAIL);
   return (writes ? X_WRITE : 0) | (emit ? X_EMIT : 0) | (fused ? X_FUSED : 0) |
          (tail ? X_TAIL : 0) | (nplans == 1 ? X_ONE : 0);
 }
@@ -1548,6 +1685,7 @@ static void launch_expand(const StepArgs& a, int mode, unsigned grid, cudaStream
     // emit runs hold one query, whose level either writes or emits
     MG_X(0) MG_X(1) MG_X(4) MG_X(5) MG_X(8) MG_X(9) MG_X(12) MG_X(13)
     MG_X(16) MG_X(17) MG_X(18) MG_X(20) MG_X(21) MG_X(24) MG_X(25) MG_X(28) MG_X(29)
+    MG_X(52) MG_X(56)
 #undef MG_X
   }
 }
