@@ -26,6 +26,8 @@
 #include <cmath>
 #include <cstring>
 #include <fstream>
+#include <initializer_list>
+#include <mutex>
 #include <random>
 #include <sstream>
 
@@ -76,6 +78,11 @@ struct OrderModel {
   __nv_bfloat16* params_bf16 = nullptr;
   bool bf16_stale = true;
   uint64_t step = 0;
+  // Inputs and outputs of a call (queries, samples, loss, predictions): one
+  // block that grows and stays.
+  void* io = nullptr;
+  size_t io_bytes = 0;
+  std::mutex mu;  // held by a call that uses io
   ~OrderModel() {
     if (stream) {
       int prev = 0;
@@ -87,6 +94,7 @@ struct OrderModel {
       cudaFree(adam_m);
       cudaFree(adam_v);
       cudaFree(params_bf16);
+      cudaFree(io);
       cudaStreamDestroy(stream);
       cudaSetDevice(prev);
     }
@@ -186,91 +194,306 @@ __device__ float mpnn_forward(const W* P, const QFeat& Q, uint32_t mask, FwdSmem
   return y;
 }
 
-// Forward (+ backward) over samples [0, ns): every block walks a contiguous
-// range, accumulates parameter gradients of scale*(y - t)^2 in shared memory
-// (thread j owns row j of every matrix) and flushes them with atomics.
-// out (optional) receives y per sample.
-__global__ void __launch_bounds__(MH) k_mpnn_train(const float* __restrict__ P,
+// ---- training -------------------------------------------------------------------
+// Forward (+ backward) over samples [0, ns).  A block takes a contiguous range
+// and works on tiles of up to TR nodes of up to TS samples, so that the layers
+// are matrix products over the nodes of many samples, in FP32.
+//
+// What bounds it: shared-memory reads and FMA issue.  Weights are staged once
+// per block with rows padded to TL words (16-byte reads of neighbouring rows
+// fall into different banks); every thread owns a 4x4 part of each 64x64 weight
+// gradient in registers over all its tiles, and the block adds them to global
+// memory once at the end.  One 64-thread block per sample, weights read from
+// global memory a row per lane and gradients summed in shared memory with all
+// lanes on one bank, took 1,750 us for 4,096 samples; the whole call with its
+// copies took 2,400 us and takes 365.
+constexpr int TB = 256, TR = 64, TS = 32, TL = 68, TF = MF + MF + 1;
+
+struct TrainSmem {
+  float w2h[MH * TL], w2m[MH * TL], wr[MH * TL];
+  float w1[MH * TF];  // W1x | W1m per unit
+  float b1[MH], b2[MH], br[MH], wo[MH];
+  float x[TR * TF];  // node features | a1
+  float h1[TR * TL], a2[TR * TL], h2[TR * TL], u[TR * TL], v[TR * TL];
+  float z[TS * TL], r[TS * TL], dr[TS * TL], dz[TS * TL];
+  float y[TS], dy[TS];
+  unsigned long long adj[TR];  // neighbours among the tile's rows
+  int node[TR], owner[TR];     // query vertex, sample of the tile
+  int base[TS + 1];            // first row of every sample
+  int ns;
+};
+
+// acc[i][c] += sum_k A[4 * ty + i][k] * W[tx + 16 * c][k] over 64 columns k.
+__device__ __forceinline__ void mul_rows(const float* A, const float* W, int ty, int tx,
+                                         float (&acc)[4][4]) {
+  for (int k = 0; k < MH; k += 4) {
+    float4 a[4], w[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(A + (4 * ty + i) * TL + k);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) w[c] = *reinterpret_cast<const float4*>(W + (tx + 16 * c) * TL + k);
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < 4; ++c)
+        acc[i][c] += a[i].x * w[c].x + a[i].y * w[c].y + a[i].z * w[c].z + a[i].w * w[c].w;
+  }
+}
+
+// acc[i][c] += sum_k A[4 * ty + i][k] * W[k][tx + 16 * c].
+__device__ __forceinline__ void mul_cols(const float* A, const float* W, int ty, int tx,
+                                         float (&acc)[4][4]) {
+  for (int k = 0; k < MH; k += 4) {
+    float4 a[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) a[i] = *reinterpret_cast<const float4*>(A + (4 * ty + i) * TL + k);
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const float* w = W + k * TL + tx + 16 * c;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        acc[i][c] += a[i].x * w[0] + a[i].y * w[TL] + a[i].z * w[2 * TL] + a[i].w * w[3 * TL];
+    }
+  }
+}
+
+// g[i][c] += sum_{r < n} D[r][ty + 16 * i] * H[r][tx + 16 * c].
+__device__ __forceinline__ void outer(const float* D, const float* H, int n, int ty, int tx,
+                                      float (&g)[4][4]) {
+  for (int r = 0; r < n; ++r) {
+    float d[4], h[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) d[i] = D[r * TL + ty + 16 * i];
+#pragma unroll
+    for (int c = 0; c < 4; ++c) h[c] = H[r * TL + tx + 16 * c];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) g[i][c] += d[i] * h[c];
+  }
+}
+
+__global__ void __launch_bounds__(TB) k_mpnn_train(const float* __restrict__ P,
                                                    const QFeat* __restrict__ qf,
                                                    const Sample* __restrict__ smp, uint32_t ns,
                                                    float scale, int backward, float* grad,
                                                    float* loss, float* out) {
-  extern __shared__ float g[];  // NPARAM gradient accumulators
-  __shared__ FwdSmem s;
-  __shared__ float dz[MH], dr[MH];
-  __shared__ float dpre2[MQ][MH], gw[MQ][MH], dh1a[MQ][MH], dpre1[MQ][MH];
-  const int j = threadIdx.x;
-  if (backward)
-    for (int t = j; t < NPARAM; t += MH) g[t] = 0.f;
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  TrainSmem& s = *reinterpret_cast<TrainSmem*>(smem_raw);
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4, j = t & 63, q4 = t >> 6;
+  for (int x = t; x < MH * MH; x += TB) {
+    const int at = (x >> 6) * TL + (x & 63);
+    s.w2h[at] = P[OFF_W2h + x];
+    s.w2m[at] = P[OFF_W2m + x];
+    s.wr[at] = P[OFF_Wr + x];
+  }
+  for (int x = t; x < MH * TF; x += TB) {
+    const int u = x / TF, f = x % TF;
+    s.w1[x] = f < MF ? P[OFF_W1x + u * MF + f] : P[OFF_W1m + u * (MF + 1) + f - MF];
+  }
+  if (t < MH) {
+    s.b1[t] = P[OFF_b1 + t];
+    s.b2[t] = P[OFF_b2 + t];
+    s.br[t] = P[OFF_br + t];
+    s.wo[t] = P[OFF_wo + t];
+  }
+  const float bo = P[OFF_bo];
+  float g2h[4][4] = {}, g2m[4][4] = {}, gr[4][4] = {}, g1[5] = {};
+  float gb1 = 0.f, gb2 = 0.f, gbr = 0.f, gwo = 0.f, gbo = 0.f, lsum = 0.f;
   const uint32_t per = (ns + gridDim.x - 1) / gridDim.x;
-  const uint32_t s0 = blockIdx.x * per, s1 = min(ns, s0 + per);
-  float lsum = 0.f;
-  for (uint32_t si = s0; si < s1; ++si) {
-    const Sample sm = smp[si];
-    const QFeat& Q = qf[sm.q];
-    const float y = mpnn_forward(P, Q, sm.mask, s);
-    if (out && j == 0) out[si] = y;
-    const float diff = y - sm.target;
-    lsum += diff * diff;
+  const uint32_t s1 = min(ns, (blockIdx.x + 1) * per);
+  for (uint32_t s0 = blockIdx.x * per; s0 < s1; s0 += s.ns) {
+    __syncthreads();  // the previous tile is no longer read
+    // ---- rows of this tile
+    if (t < 32) {
+      const uint32_t si = s0 + t;
+      const int nn = si < s1 ? __popc(smp[si].mask & ((1u << qf[smp[si].q].k) - 1)) : TR + 1;
+      int incl = nn;
+      for (int d = 1; d < 32; d <<= 1) {
+        const int o = __shfl_up_sync(FULL, incl, d);
+        if (t >= d) incl += o;
+      }
+      s.base[t + 1] = incl;
+      if (t == 0) s.base[0] = 0;
+      const uint32_t fit = __ballot_sync(FULL, incl <= TR);
+      if (t == 0) s.ns = __popc(fit);
+    }
+    __syncthreads();
+    const int nsm = s.ns, M = s.base[nsm];
+    for (int x = t; x < nsm * MQ; x += TB) {
+      const int si = x / MQ, u = x % MQ;
+      const Sample sm = smp[s0 + si];
+      const QFeat& Q = qf[sm.q];
+      const uint32_t mask = sm.mask & ((1u << Q.k) - 1);
+      if (!((mask >> u) & 1u)) continue;
+      const int row = s.base[si] + __popc(mask & ((1u << u) - 1));
+      s.node[row] = u;
+      s.owner[row] = si;
+      unsigned long long nb = 0;
+      for (uint32_t m = Q.adj[u] & mask; m; m &= m - 1)
+        nb |= 1ull << (s.base[si] + __popc(mask & ((1u << (__ffs(m) - 1)) - 1)));
+      s.adj[row] = nb;
+      for (int f = 0; f < MF; ++f)
+        s.x[row * TF + f] = f == 5 ? float(__popc(Q.adj[u] & mask)) * 0.125f : Q.x[u][f];
+    }
+    __syncthreads();
+    for (int x = t; x < M * (MF + 1); x += TB) {
+      const int row = x / (MF + 1), f = x % (MF + 1);
+      float acc = 0.f;
+      for (unsigned long long m = s.adj[row]; m; m &= m - 1) {
+        const int b = __ffsll(m) - 1;
+        acc += f < MF ? s.x[b * TF + f] : qf[smp[s0 + s.owner[row]].q].e[s.node[row]][s.node[b]];
+      }
+      s.x[row * TF + MF + f] = acc;
+    }
+    __syncthreads();
+    // ---- layer 1
+    for (int row = q4; row < M; row += 4) {
+      float v = s.b1[j];
+      for (int f = 0; f < TF; ++f) v += s.w1[j * TF + f] * s.x[row * TF + f];
+      s.h1[row * TL + j] = fmaxf(v, 0.f);
+    }
+    __syncthreads();
+    for (int row = q4; row < M; row += 4) {
+      float acc = 0.f;
+      for (unsigned long long m = s.adj[row]; m; m &= m - 1) acc += s.h1[(__ffsll(m) - 1) * TL + j];
+      s.a2[row * TL + j] = acc;
+    }
+    __syncthreads();
+    // ---- layer 2
+    if (4 * ty < M) {
+      float acc[4][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[i][c] = s.b2[tx + 16 * c];
+      mul_rows(s.h1, s.w2h, ty, tx, acc);
+      mul_rows(s.a2, s.w2m, ty, tx, acc);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) s.h2[(4 * ty + i) * TL + tx + 16 * c] = fmaxf(acc[i][c], 0.f);
+    }
+    __syncthreads();
+    // ---- readout
+    for (int si = q4; si < nsm; si += 4) {
+      float zj = 0.f;
+      for (int row = s.base[si]; row < s.base[si + 1]; ++row) zj += s.h2[row * TL + j];
+      s.z[si * TL + j] = zj;
+    }
+    __syncthreads();
+    for (int si = q4; si < nsm; si += 4) {
+      float v = s.br[j];
+      for (int l = 0; l < MH; l += 4) {
+        const float4 w = *reinterpret_cast<const float4*>(s.wr + j * TL + l);
+        const float4 z = *reinterpret_cast<const float4*>(s.z + si * TL + l);
+        v += w.x * z.x + w.y * z.y + w.z * z.z + w.w * z.w;
+      }
+      s.r[si * TL + j] = fmaxf(v, 0.f);
+    }
+    __syncthreads();
+    for (int si = t >> 5; si < nsm; si += TB / 32) {
+      const int l = t & 31;
+      float v = s.wo[l] * s.r[si * TL + l] + s.wo[l + 32] * s.r[si * TL + l + 32];
+      for (int d = 16; d > 0; d >>= 1) v += __shfl_down_sync(FULL, v, d);
+      if (l == 0) {
+        v += bo;
+        s.y[si] = v;
+        s.dy[si] = 2.f * scale * (v - smp[s0 + si].target);
+        if (out) out[s0 + si] = v;
+      }
+    }
+    __syncthreads();
+    if (t == 0)
+      for (int si = 0; si < nsm; ++si) {
+        const float diff = s.y[si] - smp[s0 + si].target;
+        lsum += diff * diff;
+        gbo += s.dy[si];
+      }
     if (!backward) continue;
-    const int nn = s.nn;
-    const float dy = 2.f * scale * diff;
-    // readout
-    if (j == 0) g[OFF_bo] += dy;
-    g[OFF_wo + j] += dy * s.r[j];
-    const float drj = s.r[j] > 0.f ? dy * P[OFF_wo + j] : 0.f;
-    dr[j] = drj;
-    g[OFF_br + j] += drj;
-    for (int l = 0; l < MH; ++l) g[OFF_Wr + j * MH + l] += drj * s.z[l];
+    // ---- backward: readout
+    for (int si = q4; si < nsm; si += 4)
+      s.dr[si * TL + j] = s.r[si * TL + j] > 0.f ? s.dy[si] * s.wo[j] : 0.f;
+    if (t < MH)
+      for (int si = 0; si < nsm; ++si) gwo += s.dy[si] * s.r[si * TL + t];
     __syncthreads();
-    float dzj = 0.f;
-    for (int i = 0; i < MH; ++i) dzj += P[OFF_Wr + i * MH + j] * dr[i];
-    dz[j] = dzj;
+    if (t < MH)
+      for (int si = 0; si < nsm; ++si) gbr += s.dr[si * TL + t];
+    outer(s.dr, s.z, nsm, ty, tx, gr);
+    for (int si = q4; si < nsm; si += 4) {
+      float v = 0.f;
+      for (int i = 0; i < MH; ++i) v += s.wr[i * TL + j] * s.dr[si * TL + i];
+      s.dz[si * TL + j] = v;
+    }
     __syncthreads();
-    // layer 2
-    for (int a = 0; a < nn; ++a) {
-      const float d = s.h2[a][j] > 0.f ? dz[j] : 0.f;
-      dpre2[a][j] = d;
-      g[OFF_b2 + j] += d;
-      for (int l = 0; l < MH; ++l) {
-        g[OFF_W2h + j * MH + l] += d * s.h1[a][l];
-        g[OFF_W2m + j * MH + l] += d * s.a2[a][l];
+    // ---- layer 2: h2 becomes its gradient before the activation
+    for (int row = q4; row < TR; row += 4)
+      s.h2[row * TL + j] =
+          row < M && s.h2[row * TL + j] > 0.f ? s.dz[s.owner[row] * TL + j] : 0.f;
+    __syncthreads();
+    if (t < MH)
+      for (int row = 0; row < M; ++row) gb2 += s.h2[row * TL + t];
+    outer(s.h2, s.h1, M, ty, tx, g2h);
+    outer(s.h2, s.a2, M, ty, tx, g2m);
+    if (4 * ty < M) {
+      float au[4][4] = {}, av[4][4] = {};
+      mul_cols(s.h2, s.w2h, ty, tx, au);
+      mul_cols(s.h2, s.w2m, ty, tx, av);
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          s.u[(4 * ty + i) * TL + tx + 16 * c] = au[i][c];
+          s.v[(4 * ty + i) * TL + tx + 16 * c] = av[i][c];
+        }
+    }
+    __syncthreads();
+    // ---- layer 1
+    for (int row = q4; row < M; row += 4) {
+      float dh = s.u[row * TL + j];
+      for (unsigned long long m = s.adj[row]; m; m &= m - 1) dh += s.v[(__ffsll(m) - 1) * TL + j];
+      s.a2[row * TL + j] = s.h1[row * TL + j] > 0.f ? dh : 0.f;
+    }
+    __syncthreads();
+    if (t < MH)
+      for (int row = 0; row < M; ++row) gb1 += s.a2[row * TL + t];
+#pragma unroll
+    for (int x = 0; x < 5; ++x) {
+      const int at = t + x * TB;
+      if (at < MH * TF) {
+        const int u = at / TF, f = at % TF;
+        float v = 0.f;
+        for (int row = 0; row < M; ++row) v += s.a2[row * TL + u] * s.x[row * TF + f];
+        g1[x] += v;
       }
     }
-    __syncthreads();
-    for (int a = 0; a < nn; ++a) {
-      float v = 0.f, w2 = 0.f;
-      for (int i = 0; i < MH; ++i) {
-        v += P[OFF_W2m + i * MH + j] * dpre2[a][i];
-        w2 += P[OFF_W2h + i * MH + j] * dpre2[a][i];
-      }
-      gw[a][j] = v;
-      dh1a[a][j] = w2;
-    }
-    __syncthreads();
-    // layer 1
-    for (int a = 0; a < nn; ++a) {
-      const int u = s.nodes[a];
-      float dh = dh1a[a][j];
-      for (int b = 0; b < nn; ++b)
-        if ((Q.adj[u] >> s.nodes[b]) & 1u) dh += gw[b][j];
-      dpre1[a][j] = s.h1[a][j] > 0.f ? dh : 0.f;
-    }
-    __syncthreads();
-    for (int a = 0; a < nn; ++a) {
-      const float d = dpre1[a][j];
-      g[OFF_b1 + j] += d;
-      for (int f = 0; f < MF; ++f) g[OFF_W1x + j * MF + f] += d * s.x[a][f];
-      for (int f = 0; f < MF + 1; ++f) g[OFF_W1m + j * (MF + 1) + f] += d * s.a1[a][f];
-    }
-    __syncthreads();
   }
-  if (j == 0 && loss) atomicAdd(loss, lsum * scale);
-  if (backward) {
-    __syncthreads();
-    for (int t = j; t < NPARAM; t += MH)
-      if (g[t] != 0.f) atomicAdd(&grad[t], g[t]);
+  if (t == 0 && loss) atomicAdd(loss, lsum * scale);
+  if (!backward) return;
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int at = (ty + 16 * i) * MH + tx + 16 * c;
+      atomicAdd(&grad[OFF_W2h + at], g2h[i][c]);
+      atomicAdd(&grad[OFF_W2m + at], g2m[i][c]);
+      atomicAdd(&grad[OFF_Wr + at], gr[i][c]);
+    }
+#pragma unroll
+  for (int x = 0; x < 5; ++x) {
+    const int at = t + x * TB;
+    if (at < MH * TF) {
+      const int u = at / TF, f = at % TF;
+      atomicAdd(&grad[f < MF ? OFF_W1x + u * MF + f : OFF_W1m + u * (MF + 1) + f - MF], g1[x]);
+    }
   }
+  if (t < MH) {
+    atomicAdd(&grad[OFF_b1 + t], gb1);
+    atomicAdd(&grad[OFF_b2 + t], gb2);
+    atomicAdd(&grad[OFF_br + t], gbr);
+    atomicAdd(&grad[OFF_wo + t], gwo);
+  }
+  if (t == 0) atomicAdd(&grad[OFF_bo], gbo);
 }
 
 // BF16 inference: one sample per block.
@@ -309,7 +532,7 @@ __global__ void k_to_bf16(const float* p, __nv_bfloat16* o, int n) {
 // ---------------------------------------------------------------------------
 namespace {
 
-const size_t kTrainSmem = size_t(NPARAM) * 4;
+const size_t kTrainSmem = sizeof(TrainSmem);
 
 int model_init(OrderModel* M, int device) {
   M->device = device;
@@ -381,6 +604,36 @@ bool connected(uint32_t mask, const QFeat& f) {
   return seen == mask;
 }
 
+// Device memory for the arrays of a call, each on a 256-byte boundary (io_trim
+// gives a large block back after it).
+constexpr size_t kIoKeep = size_t(64) << 20;
+
+int io_block(OrderModel* M, std::initializer_list<std::pair<void**, size_t>> arrays) {
+  size_t bytes = 0;
+  for (auto& a : arrays) bytes += (a.second + 255) & ~size_t(255);
+  if (M->io_bytes < bytes) {
+    MG_CK(cudaStreamSynchronize(M->stream));
+    cudaFree(M->io);
+    M->io = nullptr;
+    M->io_bytes = 0;
+    MG_CK(cudaMalloc(&M->io, bytes));
+    M->io_bytes = bytes;
+  }
+  auto* p = static_cast<unsigned char*>(M->io);
+  for (auto& a : arrays) {
+    *a.first = p;
+    p += (a.second + 255) & ~size_t(255);
+  }
+  return MG_OK;
+}
+
+void io_trim(OrderModel* M) {
+  if (M->io_bytes <= kIoKeep) return;
+  cudaFree(M->io);
+  M->io = nullptr;
+  M->io_bytes = 0;
+}
+
 int refresh_bf16(OrderModel* M) {
   if (!M->bf16_stale) return MG_OK;
   k_to_bf16<<<64, 256, 0, M->stream>>>(M->params, M->params_bf16, NPARAM);
@@ -394,6 +647,7 @@ int infer(OrderModel* M, const std::vector<QFeat>& qf, const std::vector<Sample>
           std::vector<float>& out) {
   out.assign(smp.size(), 0.f);
   if (smp.empty()) return MG_OK;
+  std::lock_guard<std::mutex> lock(M->mu);
   int prev = 0;
   cudaGetDevice(&prev);
   MG_CK(cudaSetDevice(M->device));
@@ -403,19 +657,18 @@ int infer(OrderModel* M, const std::vector<QFeat>& qf, const std::vector<Sample>
   Sample* ds;
   float* dout;
   cudaStream_t st = M->stream;
-  MG_CK(cudaMallocAsync((void**)&dq, qf.size() * sizeof(QFeat), st));
-  MG_CK(cudaMallocAsync((void**)&ds, smp.size() * sizeof(Sample), st));
-  MG_CK(cudaMallocAsync((void**)&dout, smp.size() * 4, st));
+  if ((rc = io_block(M, {{(void**)&dq, qf.size() * sizeof(QFeat)},
+                         {(void**)&ds, smp.size() * sizeof(Sample)},
+                         {(void**)&dout, smp.size() * 4}})))
+    return rc;
   MG_CK(cudaMemcpyAsync(dq, qf.data(), qf.size() * sizeof(QFeat), cudaMemcpyHostToDevice, st));
   MG_CK(cudaMemcpyAsync(ds, smp.data(), smp.size() * sizeof(Sample), cudaMemcpyHostToDevice, st));
   const unsigned blocks = unsigned(std::min<size_t>(smp.size(), size_t(M->sms) * 32));
   k_mpnn_infer_bf16<<<blocks, MH, 0, st>>>(M->params_bf16, dq, ds, uint32_t(smp.size()), dout);
   MG_CK(cudaMemcpyAsync(out.data(), dout, smp.size() * 4, cudaMemcpyDeviceToHost, st));
-  cudaFreeAsync(dq, st);
-  cudaFreeAsync(ds, st);
-  cudaFreeAsync(dout, st);
   MG_CK(cudaStreamSynchronize(st));
   MG_CK(cudaGetLastError());
+  io_trim(M);
   cudaSetDevice(prev);
   return MG_OK;
 }
@@ -586,9 +839,11 @@ static int gather(DevGraph* dg, const mg_csr_view* const* qs, uint32_t nq,
 
 static int train_pass(OrderModel* M, const QFeat* dq, const Sample* ds, uint32_t ns, float scale,
                       bool backward, float* dloss, float* dout) {
-  const unsigned blocks = std::max(1u, std::min<unsigned>(ns, M->sms * 2));
+  // A block per SM, and at least eight samples for each: a block pays the
+  // staging of the weights and the adding up of their gradients.
+  const unsigned blocks = std::max(1u, std::min<unsigned>((ns + 7) / 8, M->sms));
   if (backward) MG_CK(cudaMemsetAsync(M->grad, 0, NPARAM * 4, M->stream));
-  k_mpnn_train<<<blocks, MH, kTrainSmem, M->stream>>>(M->params, dq, ds, ns, scale,
+  k_mpnn_train<<<blocks, TB, kTrainSmem, M->stream>>>(M->params, dq, ds, ns, scale,
                                                        backward ? 1 : 0, M->grad, dloss, dout);
   MG_CK(cudaGetLastError());
   return MG_OK;
@@ -744,27 +999,27 @@ int mg_order_model_grad(void* model, void* dgraph, const mg_csr_view* const* qs,
   mg::QFeat* dq;
   mg::Sample* ds;
   float *dl, *dout = nullptr;
-  MG_CK(cudaMallocAsync((void**)&dq, feats.size() * sizeof(mg::QFeat), st));
-  MG_CK(cudaMallocAsync((void**)&ds, smp.size() * sizeof(mg::Sample), st));
-  MG_CK(cudaMallocAsync((void**)&dl, 4, st));
-  if (pred_out) MG_CK(cudaMallocAsync((void**)&dout, ns * 4ull, st));
+  std::lock_guard<std::mutex> mlock(M->mu);
+  if ((rc = mg::io_block(M, {{(void**)&dq, feats.size() * sizeof(mg::QFeat)},
+                             {(void**)&ds, smp.size() * sizeof(mg::Sample)},
+                             {(void**)&dl, 4},
+                             {(void**)&dout, pred_out ? ns * 4ull : 0}})))
+    return rc;
   MG_CK(cudaMemcpyAsync(dq, feats.data(), feats.size() * sizeof(mg::QFeat),
                         cudaMemcpyHostToDevice, st));
   MG_CK(cudaMemcpyAsync(ds, smp.data(), smp.size() * sizeof(mg::Sample), cudaMemcpyHostToDevice,
                         st));
   MG_CK(cudaMemsetAsync(dl, 0, 4, st));
-  rc = mg::train_pass(M, dq, ds, ns, 1.f / float(ns), grad_out != nullptr, dl, dout);
+  rc = mg::train_pass(M, dq, ds, ns, 1.f / float(ns), grad_out != nullptr, dl,
+                      pred_out ? dout : nullptr);
   if (rc == MG_OK) {
     if (grad_out)
       MG_CK(cudaMemcpyAsync(grad_out, M->grad, mg::NPARAM * 4, cudaMemcpyDeviceToHost, st));
     if (loss_out) MG_CK(cudaMemcpyAsync(loss_out, dl, 4, cudaMemcpyDeviceToHost, st));
     if (pred_out) MG_CK(cudaMemcpyAsync(pred_out, dout, ns * 4ull, cudaMemcpyDeviceToHost, st));
   }
-  cudaFreeAsync(dq, st);
-  cudaFreeAsync(ds, st);
-  cudaFreeAsync(dl, st);
-  if (dout) cudaFreeAsync(dout, st);
   MG_CK(cudaStreamSynchronize(st));
+  mg::io_trim(M);
   cudaSetDevice(prev);
   return rc;
 }
