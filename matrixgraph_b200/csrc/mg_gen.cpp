@@ -166,22 +166,15 @@ static int gen_labels(uint32_t n, uint32_t kind, uint32_t L, double s,
 // Maps a global id of the data graph to its local id (identity fast path).
 struct G2L {
   const mg_csr_view* g;
-  std::vector<uint32_t> map;
-  bool ident = true;
-  explicit G2L(const mg_csr_view* gv) : g(gv) {
-    for (uint32_t i = 0; i < g->n; ++i)
-      if (g->globalid[i] != i) {
-        ident = false;
-        break;
-      }
-    if (!ident) {
+  std::vector<uint32_t> map;  // made for the first id that is not its own local id
+  explicit G2L(const mg_csr_view* gv) : g(gv) {}
+  uint32_t operator()(uint32_t gid) {
+    if (gid < g->n && g->globalid[gid] == gid) return gid;
+    if (map.empty()) {
       map.assign(uint64_t(g->max_vid) + 1, 0xFFFFFFFFu);
       for (uint32_t i = 0; i < g->n; ++i)
         if (g->globalid[i] <= g->max_vid) map[g->globalid[i]] = i;
     }
-  }
-  uint32_t operator()(uint32_t gid) const {
-    if (ident) return gid;
     return gid < map.size() ? map[gid] : 0xFFFFFFFFu;
   }
 };
