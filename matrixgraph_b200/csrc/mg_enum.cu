@@ -41,9 +41,9 @@ const char* last_error_cstr();
 // ---------------------------------------------------------------------------
 // Workspace (per graph handle)
 // ---------------------------------------------------------------------------
-// Pendant-tail keys of a call and their two-hop aggregates (A, AD).
+// Pendant-tail keys of a call and their tables of two-hop aggregates.
 struct TailStore {
-  ulonglong2* agg = nullptr;
+  uint4* agg = nullptr;
   uint64_t cap = 0;
   TailKey* keys = nullptr;
   uint32_t keys_cap = 0;
@@ -237,7 +237,7 @@ struct StepArgs {
   // tail_agg[tkeys[kid].base + m_p - tkeys[kid].b0].
   uint32_t tail_dense;
   uint32_t star;  // two-leaf star endings are counted in closed form (PlanDev::star2)
-  const ulonglong2* tail_agg;
+  const uint4* tail_agg;
   // Level 0 of a single query is one row that needs no table: its candidates
   // are root_first + e * root_step, e < T0.
   uint64_t T0;
@@ -393,6 +393,9 @@ __device__ __forceinline__ void acc_flush_warp(const StepArgs& a, uint32_t q, ui
 // Two-hop aggregates of the tail keys, for every vertex y of label lp:
 //   A(y)  = sum_{x in N^{da}_{la}(y)} (|N^{db}_{lb}(x)| - [x self-loop, la == lb]),
 //   AD(y) = sum_{x in N^{da}_{la}(y)} |N^{db}_{lb}(x)|
+// as {A, AD, |N^{da}_{la}(y)|, degree of y}: all that closing a tail at y reads is
+// one 16-byte load.  (The x of a sum are distinct vertices, so sums are below the
+// number of adjacency entries, 2^32.)
 // A block takes TA_V vertices of one key's bucket: short slices by a thread
 // each, longer ones by a warp, the longest by the block (hubs come first in a
 // bucket).  The slices of a block are one range of adj and their lengths come
@@ -404,13 +407,16 @@ constexpr int TA_BLOCK = 256, TA_V = 256;
 constexpr uint32_t TA_WARP = 16, TA_ALL = 2048;  // slices above: a warp each, the block
 
 __global__ void __launch_bounds__(TA_BLOCK) k_tail_table(GraphDev g, const TailKey* keys,
-                                                         ulonglong2* agg) {
+                                                         uint4* agg) {
   const TailKey tk = keys[blockIdx.y];
   const uint32_t b1 = __ldg(g.bucket_off + tk.lp + 1), lane = threadIdx.x & 31;
   const uint64_t v0 = tk.b0 + uint64_t(blockIdx.x) * TA_V;
   if (tk.base == ~0ull || v0 >= b1) return;
   const uint32_t nv = min(uint32_t(TA_V), uint32_t(b1 - v0));
-  ulonglong2* out = agg + tk.base + (v0 - tk.b0);
+  uint4* out = agg + tk.base + (v0 - tk.b0);
+  auto put = [&](uint32_t at, unsigned long long a, unsigned long long d, uint32_t len) {
+    out[at] = make_uint4(uint32_t(a), uint32_t(d), len, __ldg(g.deg[0] + v0 + at));
+  };
   __shared__ uint32_t s_long[TA_V], s_all[TA_V], n_long, n_all;
   __shared__ unsigned long long s_a, s_d;
   if (threadIdx.x == 0) n_long = n_all = 0;
@@ -431,7 +437,7 @@ __global__ void __launch_bounds__(TA_BLOCK) k_tail_table(GraphDev g, const TailK
     if (e - s <= TA_WARP) {
       unsigned long long a = 0, d = 0;
       sum(s, e, 0, 1, a, d);
-      out[threadIdx.x] = make_ulonglong2(a, d);
+      put(threadIdx.x, a, d, e - s);
     } else if (e - s <= TA_ALL) {
       s_long[atomicAdd(&n_long, 1u)] = threadIdx.x;
     } else {
@@ -445,7 +451,7 @@ __global__ void __launch_bounds__(TA_BLOCK) k_tail_table(GraphDev g, const TailK
     sum(s, e, lane, 32, a, d);
     a = warp_sum(a);
     d = warp_sum(d);
-    if (lane == 0) out[s_long[j]] = make_ulonglong2(a, d);
+    if (lane == 0) put(s_long[j], a, d, e - s);
   }
   for (uint32_t j = 0; j < n_all; ++j) {
     if (threadIdx.x == 0) s_a = s_d = 0;
@@ -460,33 +466,29 @@ __global__ void __launch_bounds__(TA_BLOCK) k_tail_table(GraphDev g, const TailK
       atomicAdd(&s_d, d);
     }
     __syncthreads();
-    if (threadIdx.x == 0) out[s_all[j]] = make_ulonglong2(s_a, s_d);
+    if (threadIdx.x == 0) put(s_all[j], s_a, s_d, e - s);
     __syncthreads();
   }
 }
 
-// Two-hop aggregates A(m_p), AD(m_p) of a tail (see k_tail_table): from the
-// key's table, or summed over the label-l_a slice [s, e) when it has none.
-__device__ __forceinline__ void tail_agg(const StepArgs& a, const PlanDev& P, uint32_t mp,
-                                         uint32_t s, uint32_t e, long long& c, long long& d) {
+// Table entry of m_p (see k_tail_table): read from the key's table, or summed
+// over the label-l_a slice of m_p when the key has none.
+__device__ __forceinline__ uint4 tail_entry(const StepArgs& a, const PlanDev& P, uint32_t mp) {
   const GraphDev& g = a.g;
   const TailKey& tk = a.tkeys[P.tail_kid];
   const uint64_t base = tk.base;
-  if (base != ~0ull) {
-    const ulonglong2 w = __ldg(a.tail_agg + base + (mp - tk.b0));
-    c = (long long)w.x;
-    d = (long long)w.y;
-    return;
-  }
+  if (base != ~0ull) return __ldg(a.tail_agg + base + (mp - tk.b0));
   const uint32_t la = tk.la, lb = tk.lb;
-  c = d = 0;
+  uint32_t s, e, c = 0, d = 0;
+  slice_of(g, P.tail_da, mp, la, s, e);
   for (uint32_t j = s; j < e; ++j) {
     const uint32_t x = __ldg(g.adj[P.tail_da] + j);
     uint32_t xs, xe;
     slice_of(g, P.tail_db, x, lb, xs, xe);
     d += xe - xs;
-    c += (long long)(xe - xs) - ((la == lb && has_self(g, x)) ? 1 : 0);
+    c += xe - xs - ((la == lb && has_self(g, x)) ? 1u : 0u);
   }
+  return make_uint4(c, d, e - s, __ldg(g.deg[0] + mp));
 }
 
 // z in the slice [s, e) of y's d-adjacency (z carries that slice's label), where
@@ -511,18 +513,25 @@ __device__ __forceinline__ bool joined(const StepArgs& a, uint32_t d, uint32_t y
 // position j < a.
 template <class Col>
 __device__ __forceinline__ void tail_close(const StepArgs& a, const PlanDev& P, Col col,
-                                           uint32_t mp, bool cur, uint32_t s, uint32_t e,
-                                           long long c, long long d, unsigned long long& cnt,
+                                           uint32_t mp, bool cur, const uint4& entry,
+                                           unsigned long long& cnt,
                                            unsigned long long& pre, unsigned long long& dsum) {
   const GraphDev& g = a.g;
   const uint32_t ia = P.k - 2;
   const uint32_t la = P.label[ia], lb = P.label[ia + 1];
   const uint32_t da = P.tail_da, db = P.tail_db;
+  long long c = entry.x, d = entry.y;
   unsigned long long inS = 0;
   for (uint32_t mi = P.tail_Ia; mi; mi &= mi - 1) {
     const uint32_t i2 = __ffs(mi) - 1;
     const uint32_t x = col(i2);
-    if (!joined(a, da, mp, P.label[P.tail_p], cur, s, e, x)) continue;
+    bool in;
+    if (cur && x != mp && g.symmetric) {  // asked of the row's vertex (see joined)
+      in = in_slice(g, da, x, P.label[P.tail_p], mp, a.probe_min);
+    } else {
+      in = in_slice(g, da, mp, la, x, a.probe_min);
+    }
+    if (!in) continue;
     inS += 1;
     uint32_t xs, xe;
     slice_of(g, db, x, lb, xs, xe);
@@ -535,9 +544,9 @@ __device__ __forceinline__ void tail_close(const StepArgs& a, const PlanDev& P, 
     }
     c -= cx;
   }
-  c -= (long long)__popc(P.tail_J) * (long long)(e - s);
+  c -= (long long)__popc(P.tail_J) * (long long)entry.z;
   cnt = (unsigned long long)c;
-  pre = (unsigned long long)(e - s) - inS;
+  pre = (unsigned long long)entry.z - inS;
   dsum = (unsigned long long)d;
 }
 
@@ -810,9 +819,11 @@ __device__ __forceinline__ void probe_all(const uint32_t* const (&p)[U], const u
 // closed at once, with its look-ups done like the probes of the others:
 // instructions per candidate were what bounded those launches (275 per 32
 // candidates, 71% issue).  R-MAT scale 18, 5-paths whose ends share a label:
-// 90 -> 184 and 47 -> 191 G candidates/s; scale 22, 5-path: 6.5 -> 5.5 ms.
+// 90 -> 184 and 47 -> 191 G candidates/s; scale 22, 5-path: 6.5 -> 5.5 ms, and
+// 2.6 ms with all a tail needs in one 16-byte table entry instead of six loads
+// (3.6 ms at four blocks per SM, whose 64 registers spill: tails get 80).
 template <int MODE>
-__global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
+__global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expand(StepArgs a) {
   constexpr bool ONE = (MODE & X_ONE) != 0;
   // Launches that only count complete matches keep nothing of a survivor.
   constexpr bool DIRECT = (MODE & X_DIRECT) != 0;
@@ -913,18 +924,15 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
           // The prefix ending in x has length k-2: its two-position pendant
           // tail is counted here from the dense aggregates, not stored.
           const uint32_t mp = P.tail_p == i ? x : a.in.col[P.tail_p][rr];
-          uint32_t ts, ten;
-          slice_of(g, P.tail_da, mp, P.label[P.k - 2], ts, ten);
-          long long ac, ad;
-          tail_agg(a, P, mp, ts, ten, ac, ad);
+          const uint4 te = tail_entry(a, P, mp);
           unsigned long long tc, tp, td;
           tail_close(a, P, [&](uint32_t j) { return j == i ? x : a.in.col[j][rr]; }, mp,
-                     P.tail_p == i, ts, ten, ac, ad, tc, tp, td);
+                     P.tail_p == i, te, tc, tp, td);
           cnt += tc;
           sk += tc;
           s2 += tp;
-          bal += 8ull + 4ull * (ten - ts) + 8ull * tp + 4ull * td;
-          balc += 8ull + 4ull * (ten - ts) + 8ull * tp;
+          bal += 8ull + 4ull * te.z + 8ull * tp + 4ull * td;
+          balc += 8ull + 4ull * te.z + 8ull * tp;
         } else if ((MODE & X_FUSED) && fused) {
           const uint32_t kl = P.k - 1;
           const uint32_t cs = P.cons[kl][0];
@@ -1245,28 +1253,31 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, 4) k_expand(StepArgs a) {
                          (self && has_self(g, x[u]) ? 1u : 0u);
                 }
             } else {
-              const uint32_t* off = g.loff[P.tail_da] + uint64_t(P.label[P.k - 2]) * g.n;
+              // The filter of position i: its query neighbours are its backward
+              // ones, whose labels the candidate meets by its slices, and
+              // position k-2, whose label it meets when that slice has entries.
               const uint32_t nJ = __popc(P.tail_J);
+              const uint32_t min_len = (a.filters & MG_FILTER_NLB) ? 1u : 0u;
+              const uint32_t min_deg = (a.filters & MG_FILTER_DEGREE) ? P.req[0][i] : 0u;
+              uint4 te[XU];
+#pragma unroll
+              for (int u = 0; u < XU; ++u) te[u] = tail_entry(a, P, x[u]);
 #pragma unroll
               for (int u = 0; u < XU; ++u) {
-                if (ok[u] && a.filters) ok[u] = pass_filters(g, P, i, x[u], a.filters);
-                if (!ok[u]) continue;
-                const uint32_t ts = __ldg(off + x[u]), te2 = __ldg(off + x[u] + 1);
-                long long ac, ad;
-                tail_agg(a, P, x[u], ts, te2, ac, ad);
+                if (!ok[u] || te[u].z < min_len || te[u].w < min_deg) continue;
                 s1 += 1;
-                d_raw += te2 - ts;
+                d_raw += te[u].z;
                 if (in0[u] || in1[u] || ((P.tail_Ia >> i & 1u) && has_self(g, x[u]))) {
                   const uint32_t rr = rows[h[u]].row;
                   unsigned long long tc, tp, td;
                   tail_close(a, P, [&](uint32_t j) { return j == i ? x[u] : a.in.col[j][rr]; },
-                             x[u], true, ts, te2, ac, ad, tc, tp, td);
+                             x[u], true, te[u], tc, tp, td);
                   d_c += tc;
                   d_d += td;
-                  d_in += te2 - ts - uint32_t(tp);
+                  d_in += te[u].z - uint32_t(tp);
                 } else {
-                  d_c += (unsigned long long)(ac - (long long)nJ * (te2 - ts));
-                  d_d += (unsigned long long)ad;
+                  d_c += (unsigned long long)((long long)te[u].x - (long long)nJ * te[u].z);
+                  d_d += te[u].y;
                 }
               }
             }
@@ -1730,7 +1741,7 @@ static int setup_tails(DevGraph* dg, std::vector<PlanDev>& plans, TailStore& ts,
       return set_error(MG_E_OOM, "tail keys: cudaMalloc failed");
     }
     ts.keys_cap = nk;
-    if (cudaMalloc((void**)&ts.agg, want * sizeof(ulonglong2)) == cudaSuccess) {
+    if (cudaMalloc((void**)&ts.agg, want * sizeof(uint4)) == cudaSuccess) {
       ts.cap = want;
     } else {  // no room for tables: every key sums in place
       cudaGetLastError();
