@@ -635,8 +635,9 @@ __device__ __forceinline__ uint32_t row_work(const StepArgs& a, const PlanDev& P
     chc = (i + 1 == P.k && P.last_o1) ? 8ull : ch;
   }
   if (a.q_budget && best && a.in.qid) {
-    // Per-query budget (a batch's rows; one query's are charged by the tile): a query whose scheduled elements pass the budget
-    // stops expanding (its count is reported as unknown).
+    // Per-query budget of a batch's rows (one query's are charged by the tile):
+    // a query whose scheduled elements pass the budget stops expanding (its
+    // count is reported as unknown).
     const unsigned long long before = atomicAdd(&a.q_elems[q], (unsigned long long)best);
     if (before + best > a.q_budget) best = 0;
   }
@@ -1400,6 +1401,10 @@ __global__ void __launch_bounds__(256) k_work_scan(StepArgs a, uint32_t epoch) {
   __shared__ uint32_t s_tile;
   __shared__ unsigned long long s_prefix;
   __shared__ unsigned long long s_off[WS_ROWS];
+  const PlanDev& P0 = a.plans[0];
+  const uint32_t nc = P0.ncons[i];
+  const bool o1 = i + 1 == P0.k && P0.last_o1;
+  const bool fast = !a.in.qid && i > 0 && nc > 0 && !P0.zero;
   for (;;) {
     if (threadIdx.x == 0)
       s_tile = uint32_t(atomicAdd(&a.ctr[lvl_slot(int(i), L_SCAN)], 1ull));
@@ -1408,11 +1413,45 @@ __global__ void __launch_bounds__(256) k_work_scan(StepArgs a, uint32_t epoch) {
     __syncthreads();
     if (tile >= ntiles) break;
     const uint64_t base = tile * WS_ROWS + uint64_t(threadIdx.x) * 4;
-    unsigned long long v[4], sum = 0;
-    for (int j = 0; j < 4; ++j) {
-      const uint64_t r = base + j;
-      v[j] = 0;
-      if (r < R) {
+    unsigned long long v[4] = {}, sum = 0;
+    if (fast && base + 4 <= R) {
+      // Four rows of one query at once: their columns are one 16-byte read, and
+      // the reads of their slices overlap.
+      uint32_t best[4], bs[4], ci[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        best[j] = FULL;
+        bs[j] = ci[j] = 0;
+      }
+      unsigned long long ch = 0;
+      const uint32_t lab = P0.label[i];
+      for (uint32_t c = 0; c < nc; ++c) {
+        const uint32_t cs = P0.cons[i][c];
+        const uint4 y4 = *reinterpret_cast<const uint4*>(a.in.col[cs & 0xFF] + base);
+        const uint32_t y[4] = {y4.x, y4.y, y4.z, y4.w};
+        uint32_t s[4], e[4];
+#pragma unroll
+        for (int j = 0; j < 4; ++j) slice_of(a.g, cs >> 8, y[j], lab, s[j], e[j]);
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          ch += e[j] - s[j];
+          if (e[j] - s[j] < best[j]) {
+            best[j] = e[j] - s[j];
+            bs[j] = s[j];
+            ci[j] = c;
+          }
+        }
+      }
+      bal += 32ull * nc + 4 * ch;
+      balc += o1 ? 32ull : 32ull * nc + 4 * ch;
+      *reinterpret_cast<uint4*>(a.dstart + base) = make_uint4(bs[0], bs[1], bs[2], bs[3]);
+      *reinterpret_cast<uchar4*>(a.dci + base) = make_uchar4(ci[0], ci[1], ci[2], ci[3]);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) sum += v[j] = best[j];
+    } else {
+      for (int j = 0; j < 4; ++j) {
+        const uint64_t r = base + j;
+        if (r >= R) break;
         const uint32_t q = a.in.qid ? a.in.qid[r] : 0u;
         uint32_t bs;
         uint8_t bci;
