@@ -513,8 +513,8 @@ __device__ __forceinline__ bool joined(const StepArgs& a, uint32_t d, uint32_t y
 // position j < a.
 template <class Col>
 __device__ __forceinline__ void tail_close(const StepArgs& a, const PlanDev& P, Col col,
-                                           uint32_t mp, bool cur, const uint4& entry,
-                                           unsigned long long& cnt,
+                                           uint32_t Ia, uint32_t mp, bool cur,
+                                           const uint4& entry, unsigned long long& cnt,
                                            unsigned long long& pre, unsigned long long& dsum) {
   const GraphDev& g = a.g;
   const uint32_t ia = P.k - 2;
@@ -522,7 +522,7 @@ __device__ __forceinline__ void tail_close(const StepArgs& a, const PlanDev& P, 
   const uint32_t da = P.tail_da, db = P.tail_db;
   long long c = entry.x, d = entry.y;
   unsigned long long inS = 0;
-  for (uint32_t mi = P.tail_Ia; mi; mi &= mi - 1) {
+  for (uint32_t mi = Ia; mi; mi &= mi - 1) {
     const uint32_t i2 = __ffs(mi) - 1;
     const uint32_t x = col(i2);
     bool in;
@@ -694,20 +694,20 @@ enum : int {
   X_FUSED = 4,  // the last position (one backward slice) is closed in place
   X_TAIL = 8,   // a two-position pendant tail is closed from dense aggregates
   X_ONE = 16,   // one query, no row query ids: its plan is staged in shared memory
-  X_DIRECT = 32,  // with X_ONE and X_FUSED or X_TAIL: nearly every candidate survives
-                  // and is closed where it is found (see direct_sides)
+  X_DIRECT = 32,  // with X_ONE and X_FUSED or X_TAIL: candidates are closed where they
+                  // are found (see direct_sides)
 };
 
-// Positions of a row whose matches may lie in the slice that closes a candidate
-// at position i (FUSED: of the last position, TAIL: of position k-2), and that
-// have to be looked up per candidate: the slice is the candidate's own (anchor
-// i), or the candidate itself may lie in an earlier vertex's slice.
+// Positions of a row whose adjacency each candidate of position i is looked up
+// in to be closed.  The slice that closes it (FUSED: of the last position, TAIL:
+// of position k-2) is the candidate's own, and then earlier matches with that
+// slice's label may lie in it, or that of an earlier vertex, and then the
+// candidate itself may; what earlier matches take from it is a matter of the row.
 __host__ __device__ __forceinline__ uint32_t direct_sides(const PlanDev& P, uint32_t i, bool tail) {
-  const uint32_t earlier = (1u << i) - 1;
-  if (tail) return P.tail_Ia & earlier;
-  const uint32_t kl = P.k - 1, pos = P.cons[kl][0] & 0xFF, open = P.samelab[kl] & ~P.guar[kl];
-  if (pos == i) return open & earlier;
-  return (open >> i) & 1u ? 1u << pos : 0u;
+  const uint32_t anchor = tail ? P.tail_p : P.cons[P.k - 1][0] & 0xFF;
+  const uint32_t open = tail ? P.tail_Ia : P.samelab[P.k - 1] & ~P.guar[P.k - 1];
+  if (anchor == i) return open & ((1u << i) - 1);
+  return (open >> i) & 1u ? 1u << anchor : 0u;
 }
 
 // One set-up row of an expand task (shared memory, a row per slot).  A further
@@ -723,9 +723,9 @@ struct alignas(16) XRow {
   uint32_t len1, m1;
   uint32_t q, ci, v0;    // query; driving constraint; bucket row: element e is
   uint32_t end;          // vertex v0 + e * root_step
-  uint32_t raw, free;    // X_DIRECT, slice of an earlier vertex: its entries, and
-                         // those that no earlier match takes
-  uint32_t pad[2];
+  // X_DIRECT, slice of an earlier vertex: its entries, those that no earlier
+  // match takes, and a tail's matches and second-slice entries over them.
+  uint32_t raw, free, c0, d0;
 };
 constexpr uint32_t HUB_LEN = FULL;
 
@@ -864,13 +864,13 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
   const uint32_t sames = ONE ? __popc(plan(0).samelab[i]) : 3u;
   const bool extra = (i == 0 && a.root_keep) || ((plan(0).selfloop_mask >> i) & 1u);
 
-  // X_DIRECT: up to two vertices of a row whose adjacency candidates are looked
-  // up in, in the slots of the further constraints (this shape has none).
+  // X_DIRECT: the vertices of a row that candidates are looked up in, in the
+  // slots that further constraints leave.
   const uint32_t sides = DIRECT ? direct_sides(plan(0), i, (MODE & X_TAIL) != 0) : 0u;
-  const uint32_t side0 = __ffs(sides) - 1, side1 = __ffs(sides & (sides - 1)) - 1;
   const uint32_t nsides = __popc(sides);
   const uint32_t kl = plan(0).k - 1;
-  const bool own = (plan(0).cons[kl][0] & 0xFF) == i;  // FUSED: the slice is the candidate's
+  const uint32_t anchor = (MODE & X_TAIL) ? plan(0).tail_p : plan(0).cons[kl][0] & 0xFF;
+  const bool own = anchor == i;  // the closing slice is the candidate's
   unsigned long long d_c = 0, d_raw = 0, d_d = 0;      // sums over closed candidates
   uint32_t d_in = 0;
 
@@ -927,7 +927,7 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
           const uint32_t mp = P.tail_p == i ? x : a.in.col[P.tail_p][rr];
           const uint4 te = tail_entry(a, P, mp);
           unsigned long long tc, tp, td;
-          tail_close(a, P, [&](uint32_t j) { return j == i ? x : a.in.col[j][rr]; }, mp,
+          tail_close(a, P, [&](uint32_t j) { return j == i ? x : a.in.col[j][rr]; }, P.tail_Ia, mp,
                      P.tail_p == i, te, tc, tp, td);
           cnt += tc;
           sk += tc;
@@ -1085,26 +1085,38 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
           }
           R.p0 = R.p1 = nullptr;
           R.len0 = R.len1 = 0;
+          uint32_t c = ci == 0 ? 1u : 0u;
+          if (c < nc) {
+            probe_of(a, P.cons[i][c], lab, row, R.p0, R.len0);
+            if (++c == ci) ++c;
+            if (c < nc) probe_of(a, P.cons[i][c], lab, row, R.p1, R.len1);
+          }
           if constexpr (DIRECT) {
-            if (nsides > 0) probe_of(a, side0, lab, row, R.p0, R.len0);
-            if (nsides > 1) probe_of(a, side1, lab, row, R.p1, R.len1);
-            if ((MODE & X_FUSED) && !own) {
-              const uint32_t y = a.in.col[P.cons[kl][0] & 0xFF][row];
-              uint32_t s, e;
-              slice_of(g, P.cons[kl][0] >> 8, y, P.label[kl], s, e);
-              R.raw = R.free = e - s;
-              for (uint32_t m2 = P.samelab[kl] & ((1u << i) - 1); m2; m2 &= m2 - 1) {
-                const uint32_t j = __ffs(m2) - 1;
-                R.free -= ((P.guar[kl] >> j) & 1u) ||
-                          in_slice_se(g, P.cons[kl][0] >> 8, y, s, e, a.in.col[j][row], a.probe_min);
+            uint32_t slot = others;
+            for (uint32_t m2 = sides; m2; m2 &= m2 - 1, ++slot)
+              probe_of(a, __ffs(m2) - 1, lab, row, slot ? R.p1 : R.p0, slot ? R.len1 : R.len0);
+            if (!own) {
+              const uint32_t y = a.in.col[anchor][row];
+              if constexpr ((MODE & X_TAIL) != 0) {
+                const uint4 te = tail_entry(a, P, y);
+                unsigned long long tc, tp, td;
+                tail_close(a, P, [&](uint32_t j) { return a.in.col[j][row]; },
+                           P.tail_Ia & ((1u << i) - 1), y, false, te, tc, tp, td);
+                R.raw = te.z;
+                R.free = uint32_t(tp);
+                R.c0 = uint32_t(tc);
+                R.d0 = uint32_t(td);
+              } else {
+                uint32_t s, e;
+                slice_of(g, P.cons[kl][0] >> 8, y, P.label[kl], s, e);
+                R.raw = R.free = e - s;
+                for (uint32_t m2 = P.samelab[kl] & ((1u << i) - 1); m2; m2 &= m2 - 1) {
+                  const uint32_t j = __ffs(m2) - 1;
+                  R.free -= ((P.guar[kl] >> j) & 1u) ||
+                            in_slice_se(g, P.cons[kl][0] >> 8, y, s, e, a.in.col[j][row],
+                                        a.probe_min);
+                }
               }
-            }
-          } else {
-            uint32_t c = ci == 0 ? 1u : 0u;
-            if (c < nc) {
-              probe_of(a, P.cons[i][c], lab, row, R.p0, R.len0);
-              if (++c == ci) ++c;
-              if (c < nc) probe_of(a, P.cons[i][c], lab, row, R.p1, R.len1);
             }
           }
           rows[__popc(act & lanemask_lt())] = R;
@@ -1166,7 +1178,7 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
             for (int u = 0; u < XU; ++u)
               ok[u] = ok[u] && x[u] != rows[h[u]].m0 && x[u] != rows[h[u]].m1;
           }
-          if (!DIRECT && (others > 0 || !ONE)) {
+          if (others > 0 || !ONE) {
             const uint32_t* p[XU];
             uint32_t len[XU];
 #pragma unroll
@@ -1176,7 +1188,7 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
             }
             probe_some(p, len);
           }
-          if (!DIRECT && (others > 1 || !ONE)) {
+          if (others > 1 || !ONE) {
             const uint32_t* p[XU];
             uint32_t len[XU];
 #pragma unroll
@@ -1227,7 +1239,7 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
               }
               probe_all<XU>(p, len, x, in);
             };
-            if (nsides > 0) look(false, in0);
+            if (nsides > 0) look(others > 0, in0);
             if (nsides > 1) look(true, in1);
             const PlanDev& P = s_plan;
             if constexpr ((MODE & X_FUSED) != 0) {
@@ -1237,8 +1249,9 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
               uint32_t raw[XU], free[XU];
 #pragma unroll
               for (int u = 0; u < XU; ++u) {
+                raw[u] = free[u] = 0;
                 if (own) {
-                  raw[u] = __ldg(off + x[u] + 1) - __ldg(off + x[u]);
+                  if (others == 0 || ok[u]) raw[u] = __ldg(off + x[u] + 1) - __ldg(off + x[u]);
                   free[u] = raw[u] - sure;
                 } else {
                   raw[u] = rows[h[u]].raw;
@@ -1255,30 +1268,45 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
                 }
             } else {
               // The filter of position i: its query neighbours are its backward
-              // ones, whose labels the candidate meets by its slices, and
-              // position k-2, whose label it meets when that slice has entries.
+              // ones, which satisfy it by themselves, and, when the tail hangs
+              // off the candidate, position k-2: its label is met when that
+              // slice has entries.
               const uint32_t nJ = __popc(P.tail_J);
-              const uint32_t min_len = (a.filters & MG_FILTER_NLB) ? 1u : 0u;
-              const uint32_t min_deg = (a.filters & MG_FILTER_DEGREE) ? P.req[0][i] : 0u;
+              const uint32_t min_len = own && (a.filters & MG_FILTER_NLB) ? 1u : 0u;
+              const uint32_t min_deg = own && (a.filters & MG_FILTER_DEGREE) ? P.req[0][i] : 0u;
+              const bool self = own && (P.tail_Ia >> i & 1u);
               uint4 te[XU];
+              if (own) {
 #pragma unroll
-              for (int u = 0; u < XU; ++u) te[u] = tail_entry(a, P, x[u]);
+                for (int u = 0; u < XU; ++u) {
+                  te[u] = make_uint4(0, 0, 0, 0);
+                  if (others == 0 || ok[u]) te[u] = tail_entry(a, P, x[u]);
+                }
+              }
 #pragma unroll
               for (int u = 0; u < XU; ++u) {
-                if (!ok[u] || te[u].z < min_len || te[u].w < min_deg) continue;
+                if (!ok[u] || (own && (te[u].z < min_len || te[u].w < min_deg))) continue;
+                const XRow& R = rows[h[u]];
                 s1 += 1;
-                d_raw += te[u].z;
-                if (in0[u] || in1[u] || ((P.tail_Ia >> i & 1u) && has_self(g, x[u]))) {
-                  const uint32_t rr = rows[h[u]].row;
+                if (in0[u] || in1[u] || (self && has_self(g, x[u]))) {
+                  const uint32_t mp = own ? x[u] : a.in.col[anchor][R.row];
+                  const uint4 t4 = own ? te[u] : tail_entry(a, P, mp);
                   unsigned long long tc, tp, td;
-                  tail_close(a, P, [&](uint32_t j) { return j == i ? x[u] : a.in.col[j][rr]; },
-                             x[u], true, te[u], tc, tp, td);
+                  tail_close(a, P, [&](uint32_t j) { return j == i ? x[u] : a.in.col[j][R.row]; },
+                             P.tail_Ia, mp, own, t4, tc, tp, td);
+                  d_raw += t4.z;
                   d_c += tc;
                   d_d += td;
-                  d_in += te[u].z - uint32_t(tp);
-                } else {
+                  d_in += t4.z - uint32_t(tp);
+                } else if (own) {
+                  d_raw += te[u].z;
                   d_c += (unsigned long long)((long long)te[u].x - (long long)nJ * te[u].z);
                   d_d += te[u].y;
+                } else {
+                  d_raw += R.raw;
+                  d_c += R.c0;
+                  d_d += R.d0;
+                  d_in += R.raw - R.free;
                 }
               }
             }
@@ -1714,14 +1742,21 @@ static int expand_mode(const StepArgs& a, uint32_t i, const PlanDev* plans, uint
     if (((a.tail_dense && p.tail2) || (a.star && p.star2)) && p.k == i + 3) tail = true;
     if (!count_mode && p.k == i + 1) emit = true;
   }
-  // Closed where they are found: a single query's candidates with no further
-  // constraint, when at most two vertices of a row need a look-up.  (Candidates
-  // with further constraints survive rarely and are staged first; a tail is
-  // direct when it hangs off the candidate.)
+  // Closed where they are found: a single query's candidates, when the probes
+  // that this takes (further constraints and look-ups) fit a row's two slots.
+  // Not a tail whose anchor is joined to the candidate and whose position k-2
+  // has its label: every candidate would take the slow path there (5.1 ms
+  // against 2.9 ms staged over such queries of a batch on R-MAT scale 22).
   if (nplans == 1 && !writes && !emit && fused != tail && a.g.symmetric &&
-      plans[0].ncons[i] <= 1 && (fused || (plans[0].tail2 && plans[0].tail_p == i)) &&
-      __builtin_popcount(direct_sides(plans[0], i, tail)) <= 2)
-    return X_DIRECT | X_ONE | (fused ? X_FUSED : X_TAIL);
+      (fused || plans[0].tail2)) {
+    const PlanDev& p = plans[0];
+    const int others = std::max(0, int(p.ncons[i]) - 1);
+    bool sure = false;
+    if (tail && p.tail_p != i && (p.tail_Ia >> i & 1u))
+      for (uint32_t c = 0; c < p.ncons[i]; ++c) sure |= (p.cons[i][c] & 0xFF) == p.tail_p;
+    if (!sure && others + __builtin_popcount(direct_sides(p, i, tail)) <= 2)
+      return X_DIRECT | X_ONE | (fused ? X_FUSED : X_TAIL);
+  }
   return (writes ? X_WRITE : 0) | (emit ? X_EMIT : 0) | (fused ? X_FUSED : 0) |
          (tail ? X_TAIL : 0) | (nplans == 1 ? X_ONE : 0);
 }
