@@ -256,6 +256,14 @@ struct StepArgs {
                                  // (bit per vertex; nullptr: no filter)
 };
 
+// Kernels of a chain are launched as programmatic dependents: one may begin
+// before the kernel ahead of it has ended, and waits here before it reads
+// anything of it.
+__device__ __forceinline__ void chain_begin() {
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+}
+__device__ __forceinline__ void chain_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Rows of the input table of a launch with sizes on the device.
 __device__ __forceinline__ uint64_t dev_rows(const StepArgs& a) {
   if (a.level == 0) return a.R;
@@ -833,29 +841,28 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
   const uint32_t i = a.level;
   const GraphDev& g = a.g;
   const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  uint64_t t0 = a.t0, t1 = a.t1;
-  if (a.dev) {
-    if (a.ctr[C_STOP]) return;
-    t0 = 0;
-    t1 = ONE && i == 0 ? a.T0 : a.ctr[lvl_slot(int(i), L_T)];
-    if (t1 > a.seg_cap) return;  // flagged by the work/scan kernel
-  }
-  const uint64_t span = t1 - t0;
-  const uint32_t ntiles = uint32_t((span + EXPAND_TILE - 1) / EXPAND_TILE);
   __shared__ XRow s_rows[EXPAND_BLOCK / 32][32];
   __shared__ uint32_t s_x[STAGE ? EXPAND_BLOCK / 32 : 1][STAGE ? XSTAGE : 1];
   __shared__ uint32_t s_r[STAGE ? EXPAND_BLOCK / 32 : 1][STAGE ? XSTAGE : 1];
   // A single query's plan is read by every row: staged once per block.
   __shared__ PlanDev s_plan;
+  chain_begin();
   if constexpr (ONE) {
     const uint32_t* src = reinterpret_cast<const uint32_t*>(a.plans);
     uint32_t* dst = reinterpret_cast<uint32_t*>(&s_plan);
     for (uint32_t w = threadIdx.x; w < sizeof(PlanDev) / 4; w += EXPAND_BLOCK) dst[w] = src[w];
     __syncthreads();
   }
-  // A lane whose tables overflowed stops: its query is counted again on the
-  // chunked path.
-  if (a.lane && a.ctr[C_ERR]) return;
+  chain_wait();
+  uint64_t t0 = a.t0, t1 = a.t1;
+  if (a.dev) {
+    // (a lane whose tables overflowed stops: its query is counted again)
+    t0 = 0;
+    t1 = ONE && i == 0 ? a.T0 : a.ctr[lvl_slot(int(i), L_T)];
+    if (a.ctr[C_STOP] || (a.lane && a.ctr[C_ERR]) || t1 > a.seg_cap) return;
+  }
+  const uint64_t span = t1 - t0;
+  const uint32_t ntiles = uint32_t((span + EXPAND_TILE - 1) / EXPAND_TILE);
   auto plan = [&](uint32_t q) -> const PlanDev& { return ONE ? s_plan : a.plans[q]; };
   auto query = [&](uint32_t r) -> uint32_t { return !ONE && a.in.qid ? a.in.qid[r] : 0u; };
   // What candidates of this level are checked for (one query; a batch looks at
@@ -1338,6 +1345,7 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
       // In a batch: fold the per-thread counts of a warp that holds one query.
       if (!ONE && a.in.qid) acc_flush_warp(a, cnt_q, i, cnt, s1, sk, s2, false);
     }
+    if (uint64_t(nwarps) * grab >= ntasks) break;  // the first grabs were all
     if (lane == 0) gbase = atomicAdd(&a.ctr[a.tile_slot], (unsigned long long)grab);
     gbase = __shfl_sync(FULL, gbase, 0) + uint64_t(nwarps) * grab;
   }
@@ -1422,6 +1430,8 @@ __device__ __forceinline__ unsigned long long look_back(const StepArgs& a, uint3
 // kernels and a tile-row search, with no size returned to the host.
 __global__ void __launch_bounds__(256) k_work_scan(StepArgs a, uint32_t epoch) {
   const uint32_t i = a.level;
+  chain_begin();
+  chain_wait();
   if (a.ctr[C_STOP] || a.ctr[C_ERR]) return;
   const uint64_t R = dev_rows(a);
   const uint64_t ntiles = (R + WS_ROWS - 1) / WS_ROWS;
@@ -1548,7 +1558,8 @@ __global__ void __launch_bounds__(256) k_work_scan(StepArgs a, uint32_t epoch) {
         if (s_off[lo + d] <= t) lo += d;
       a.tile_row[j] = uint32_t(min(tile * WS_ROWS + lo, R - 1));
     }
-    __syncthreads();  // s_off and s_prefix are written again
+    if (ntiles <= gridDim.x) break;  // no block takes a second tile
+    __syncthreads();                 // s_off and s_prefix are written again
   }
   bal = warp_sum(bal);
   balc = warp_sum(balc);
@@ -1761,11 +1772,30 @@ static int expand_mode(const StepArgs& a, uint32_t i, const PlanDev* plans, uint
          (tail ? X_TAIL : 0) | (nplans == 1 ? X_ONE : 0);
 }
 
-static void launch_expand(const StepArgs& a, int mode, unsigned grid, cudaStream_t st) {
+// Launches a kernel that begins with chain_begin / chain_wait behind the kernel
+// ahead of it in the stream; `chained`: it need not wait for that one's end to
+// be launched.
+template <class... Args>
+static cudaError_t launch_chained(void (*kernel)(Args...), unsigned grid, unsigned block,
+                                  cudaStream_t st, bool chained, Args... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(block);
+  cfg.stream = st;
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+static void launch_expand(const StepArgs& a, int mode, unsigned grid, cudaStream_t st,
+                          bool chained) {
   switch (mode) {
 #define MG_X(m) \
   case m:       \
-    k_expand<m><<<grid, EXPAND_BLOCK, 0, st>>>(a); \
+    launch_chained(k_expand<m>, grid, EXPAND_BLOCK, st, chained, a); \
     break;
     // emit runs hold one query, whose level either writes or emits
     MG_X(0) MG_X(1) MG_X(4) MG_X(5) MG_X(8) MG_X(9) MG_X(12) MG_X(13)
@@ -1968,7 +1998,7 @@ static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool cou
   };
   auto expand = [&](int l, uint64_t bound) -> int {
     if (o.kernel_events && B.ev2) MG_CK(cudaEventRecord(B.ev2, st));
-    launch_expand(a, mode[l], grid_for(bound, 256, sms * 4), st);
+    launch_expand(a, mode[l], grid_for(bound, 256, sms * 4), st, one && a.dev);
     if (o.kernel_events && B.ev2) {
       MG_CK(cudaEventRecord(B.ev3, st));
       MG_CK(cudaEventSynchronize(B.ev3));
@@ -1996,7 +2026,8 @@ static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool cou
         MG_CK(cudaMemsetAsync(B.status, 0, B.status_bytes, st));
         *B.epoch = 1;
       }
-      k_work_scan<<<grid_for(rows, WS_ROWS, sms * 4), 256, 0, st>>>(a, *B.epoch);
+      launch_chained(k_work_scan, grid_for(rows, WS_ROWS, sms * 4), 256u, st, one && l > l0, a,
+                     *B.epoch);
       res->launches++;
       const uint64_t bound = std::min(bounded_product(rows, widest[l]), a.t_limit);
       if (int r = expand(l, bound)) return r;
@@ -2627,7 +2658,7 @@ static int subiso_batch_lanes(DevGraph* dg, std::vector<PlanDev>& plans, const m
       const uint64_t bound =
           l == 0 ? t0[j] : bounded_product(rows, row_bound(dg, &P, 1, l));
       launch_expand(a, expand_mode(a, uint32_t(l), &P, 1, true, writes),
-                    grid_for(bound, 256, sms * 4), L.st);
+                    grid_for(bound, 256, sms * 4), L.st, false);
       rows = std::min(bound, cap);
       res->launches++;
       res->expand_launches++;
