@@ -704,6 +704,7 @@ enum : int {
   X_ONE = 16,   // one query, no row query ids: its plan is staged in shared memory
   X_DIRECT = 32,  // with X_ONE and X_FUSED or X_TAIL: candidates are closed where they
                   // are found (see direct_sides)
+  X_ALONE = 64,   // with X_DIRECT: the position has no further constraint
 };
 
 // Positions of a row whose adjacency each candidate of position i is looked up
@@ -867,7 +868,8 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
   auto query = [&](uint32_t r) -> uint32_t { return !ONE && a.in.qid ? a.in.qid[r] : 0u; };
   // What candidates of this level are checked for (one query; a batch looks at
   // every row's plan): further constraints, equal labels, and the rare checks.
-  const uint32_t others = ONE ? plan(0).ncons[i] - (plan(0).ncons[i] ? 1u : 0u) : 3u;
+  constexpr bool ALONE = (MODE & X_ALONE) != 0;
+  const uint32_t others = ALONE ? 0u : ONE ? plan(0).ncons[i] - (plan(0).ncons[i] ? 1u : 0u) : 3u;
   const uint32_t sames = ONE ? __popc(plan(0).samelab[i]) : 3u;
   const bool extra = (i == 0 && a.root_keep) || ((plan(0).selfloop_mask >> i) & 1u);
 
@@ -1766,7 +1768,7 @@ static int expand_mode(const StepArgs& a, uint32_t i, const PlanDev* plans, uint
     if (tail && p.tail_p != i && (p.tail_Ia >> i & 1u))
       for (uint32_t c = 0; c < p.ncons[i]; ++c) sure |= (p.cons[i][c] & 0xFF) == p.tail_p;
     if (!sure && others + __builtin_popcount(direct_sides(p, i, tail)) <= 2)
-      return X_DIRECT | X_ONE | (fused ? X_FUSED : X_TAIL);
+      return X_DIRECT | X_ONE | (fused ? X_FUSED : X_TAIL) | (others == 0 ? X_ALONE : 0);
   }
   return (writes ? X_WRITE : 0) | (emit ? X_EMIT : 0) | (fused ? X_FUSED : 0) |
          (tail ? X_TAIL : 0) | (nplans == 1 ? X_ONE : 0);
@@ -1800,7 +1802,7 @@ static void launch_expand(const StepArgs& a, int mode, unsigned grid, cudaStream
     // emit runs hold one query, whose level either writes or emits
     MG_X(0) MG_X(1) MG_X(4) MG_X(5) MG_X(8) MG_X(9) MG_X(12) MG_X(13)
     MG_X(16) MG_X(17) MG_X(18) MG_X(20) MG_X(21) MG_X(24) MG_X(25) MG_X(28) MG_X(29)
-    MG_X(52) MG_X(56)
+    MG_X(52) MG_X(56) MG_X(116) MG_X(120)
 #undef MG_X
   }
 }
