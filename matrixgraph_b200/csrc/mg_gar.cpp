@@ -22,6 +22,8 @@
 #include <cstdlib>
 #include <cstring>
 #include <memory>
+#include <new>
+#include <thread>
 #include <tuple>
 #include <vector>
 
@@ -144,23 +146,60 @@ int build_instance(const GarInputs& in, GarInstance* I) {
   // Usable data edges, and per triple whether a self-loop (bit 0) or a
   // non-loop edge (bit 1) was seen: a pattern self-loop maps only onto a
   // data self-loop, any other pattern edge only onto a non-loop edge.
-  std::vector<std::tuple<uint32_t, uint32_t, uint32_t>> kept;
-  std::vector<uint8_t> seen(usable.size(), 0);
-  for (int e = 0; e < in.m; ++e) {
-    const uint32_t s = in.src[e], d = in.dst[e];
-    if (s >= n || d >= n) continue;
-    const uint32_t cs = vlab[s], cd = vlab[d];
-    if (cs == Lp || cd == Lp) continue;
-    uint32_t el = 0;
-    if (use_elab) {
-      auto it = std::find(elabels.begin(), elabels.end(), in.elab[e]);
-      if (it == elabels.end()) continue;
-      el = uint32_t(it - elabels.begin());
+  // The edges are scanned in consecutive parts by several threads, whose finds
+  // are joined in order (1.8M edges: 13 ms of a 41 ms call by one thread).
+  using Edge = std::tuple<uint32_t, uint32_t, uint32_t>;
+  struct Part {
+    std::vector<Edge> kept;
+    std::vector<uint8_t> seen;
+    bool failed = false;
+  };
+  const uint64_t m = uint64_t(in.m);
+  const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
+  std::vector<Part> parts(std::max<uint64_t>(1, std::min<uint64_t>(std::min(hw, 16u), m >> 16)));
+  auto scan = [&](size_t t) noexcept {
+    Part& p = parts[t];
+    try {
+      p.seen.assign(usable.size(), 0);
+      const uint64_t lo = m * t / parts.size(), hi = m * (t + 1) / parts.size();
+      for (uint64_t e = lo; e < hi; ++e) {
+        const uint32_t s = in.src[e], d = in.dst[e];
+        if (s >= n || d >= n) continue;
+        const uint32_t cs = vlab[s], cd = vlab[d];
+        if (cs == Lp || cd == Lp) continue;
+        uint32_t el = 0;
+        if (use_elab) {
+          auto it = std::find(elabels.begin(), elabels.end(), in.elab[e]);
+          if (it == elabels.end()) continue;
+          el = uint32_t(it - elabels.begin());
+        }
+        const uint64_t kk = key(cs, cd, el);
+        if (!usable[kk]) continue;
+        p.seen[kk] |= s == d ? 1 : 2;
+        p.kept.emplace_back(s, d, el);
+      }
+    } catch (const std::bad_alloc&) {
+      p.failed = true;
     }
-    const uint64_t kk = key(cs, cd, el);
-    if (!usable[kk]) continue;
-    seen[kk] |= s == d ? 1 : 2;
-    kept.emplace_back(s, d, el);
+  };
+  {
+    std::vector<std::thread> threads;
+    threads.reserve(parts.size());
+    size_t t = 1;
+    try {
+      for (; t < parts.size(); ++t) threads.emplace_back(scan, t);
+    } catch (...) {  // no more threads: this one takes the rest
+    }
+    scan(0);
+    for (size_t r = t; r < parts.size(); ++r) scan(r);
+    for (auto& th : threads) th.join();
+  }
+  std::vector<Edge> kept;
+  std::vector<uint8_t> seen(usable.size(), 0);
+  for (const Part& p : parts) {
+    if (p.failed) throw std::bad_alloc();
+    kept.insert(kept.end(), p.kept.begin(), p.kept.end());
+    for (size_t x = 0; x < seen.size(); ++x) seen[x] |= p.seen[x];
   }
   // A pattern edge without a usable data edge, or a node on no pattern edge,
   // leaves every partial match incomplete: empty result.
@@ -244,7 +283,7 @@ struct PosValues {
   size_t sorted = 0;
   void compact() {
     if (sorted == v.size()) return;
-    std::sort(v.begin(), v.end());
+    if (!std::is_sorted(v.begin(), v.end())) std::sort(v.begin(), v.end());
     v.erase(std::unique(v.begin(), v.end()), v.end());
     sorted = v.size();
   }
@@ -257,7 +296,8 @@ void add_rows(std::vector<PosValues>& pv, const uint32_t* rows, uint64_t n_rows,
   for (uint64_t i = 0; i < n_rows; ++i) {
     const uint32_t* row = rows + i * row_width;
     const uint64_t pivot = uint64_t(row[0]) << 32;
-    for (uint32_t u = 0; u < k; ++u) pv[u].v.push_back(pivot | row[u]);
+    for (uint32_t u = 0; u < k; ++u)  // (rows come sorted: repeats are often neighbours)
+      if (pv[u].v.empty() || pv[u].v.back() != (pivot | row[u])) pv[u].v.push_back(pivot | row[u]);
   }
   for (auto& p : pv)
     if (p.v.size() > 2 * p.sorted + (uint64_t(1) << 20)) p.compact();
