@@ -707,6 +707,7 @@ enum : int {
   X_ALONE = 64,   // with X_DIRECT: the position has no further constraint
   X_PAIR = 128,   // with X_ONE: exactly one further constraint, at most two equal
                   // labels before, no self-loop, no matrix filter
+  X_TRIO = 256,   // the same with two further constraints
 };
 
 // Positions of a row whose adjacency each candidate of position i is looked up
@@ -838,7 +839,9 @@ __device__ __forceinline__ void probe_all(const uint32_t* const (&p)[U], const u
 // X_PAIR, the commonest shape (two lists intersected), leaves out what the
 // others may need and has the registers for three candidates a lane: 4-cycle
 // 8.9 -> 7.9 ms, triangle 1.62 -> 1.40 ms on scale 22 (two candidates 8.3 ms,
-// four 8.5; five blocks per SM 9.2, three 8.6-8.9).
+// four 8.5; five blocks per SM 9.2, three 8.6-8.9).  X_TRIO is the same for three
+// lists: 4-cliques of six labellings on scale 22, 4.57 -> 4.35 ms a call (three
+// candidates 4.39).
 template <int MODE>
 __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expand(StepArgs a) {
   constexpr bool ONE = (MODE & X_ONE) != 0;
@@ -876,10 +879,15 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
   // What candidates of this level are checked for (one query; a batch looks at
   // every row's plan): further constraints, equal labels, and the rare checks.
   constexpr bool ALONE = (MODE & X_ALONE) != 0;
-  constexpr bool PAIR = (MODE & X_PAIR) != 0;
-  const uint32_t others = ALONE ? 0u : PAIR ? 1u : ONE ? plan(0).ncons[i] - (plan(0).ncons[i] ? 1u : 0u) : 3u;
+  constexpr bool PAIR = (MODE & X_PAIR) != 0, TRIO = (MODE & X_TRIO) != 0;
+  const uint32_t others = ALONE  ? 0u
+                          : PAIR ? 1u
+                          : TRIO ? 2u
+                          : ONE  ? plan(0).ncons[i] - (plan(0).ncons[i] ? 1u : 0u)
+                                 : 3u;
   const uint32_t sames = ONE ? __popc(plan(0).samelab[i]) : 3u;
-  const bool extra = PAIR ? false : (i == 0 && a.root_keep) || ((plan(0).selfloop_mask >> i) & 1u);
+  const bool extra =
+      PAIR || TRIO ? false : (i == 0 && a.root_keep) || ((plan(0).selfloop_mask >> i) & 1u);
 
   // X_DIRECT: the vertices of a row that candidates are looked up in, in the
   // slots that further constraints leave.
@@ -1217,7 +1225,7 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
           }
           // constraints and equal labels past the two that a row keeps, and the
           // rare checks
-          if (!PAIR && (others > 2 || sames > 2 || extra)) {
+          if (!PAIR && !TRIO && (others > 2 || sames > 2 || extra)) {
 #pragma unroll
             for (int u = 0; u < XU; ++u) {
               if (!ok[u]) continue;
@@ -1778,11 +1786,13 @@ static int expand_mode(const StepArgs& a, uint32_t i, const PlanDev* plans, uint
     if (!sure && others + __builtin_popcount(direct_sides(p, i, tail)) <= 2)
       return X_DIRECT | X_ONE | (fused ? X_FUSED : X_TAIL) | (others == 0 ? X_ALONE : 0);
   }
-  const bool pair = nplans == 1 && !emit && !fused && !tail && plans[0].ncons[i] == 2 &&
-                    __builtin_popcount(plans[0].samelab[i]) <= 2 &&
-                    !((plans[0].selfloop_mask >> i) & 1u) && !(i == 0 && a.root_keep);
+  const bool plain = nplans == 1 && !emit && !fused && !tail &&
+                     __builtin_popcount(plans[0].samelab[i]) <= 2 &&
+                     !((plans[0].selfloop_mask >> i) & 1u) && !(i == 0 && a.root_keep);
+  const uint32_t nc = plans[0].ncons[i];
   return (writes ? X_WRITE : 0) | (emit ? X_EMIT : 0) | (fused ? X_FUSED : 0) |
-         (tail ? X_TAIL : 0) | (nplans == 1 ? X_ONE : 0) | (pair ? X_PAIR : 0);
+         (tail ? X_TAIL : 0) | (nplans == 1 ? X_ONE : 0) | (plain && nc == 2 ? X_PAIR : 0) |
+         (plain && nc == 3 ? X_TRIO : 0);
 }
 
 // Launches a kernel that begins with chain_begin / chain_wait behind the kernel
@@ -1813,7 +1823,7 @@ static void launch_expand(const StepArgs& a, int mode, unsigned grid, cudaStream
     // emit runs hold one query, whose level either writes or emits
     MG_X(0) MG_X(1) MG_X(4) MG_X(5) MG_X(8) MG_X(9) MG_X(12) MG_X(13)
     MG_X(16) MG_X(17) MG_X(18) MG_X(20) MG_X(21) MG_X(24) MG_X(25) MG_X(28) MG_X(29)
-    MG_X(52) MG_X(56) MG_X(116) MG_X(120) MG_X(144) MG_X(145)
+    MG_X(52) MG_X(56) MG_X(116) MG_X(120) MG_X(144) MG_X(145) MG_X(272) MG_X(273)
 #undef MG_X
   }
 }

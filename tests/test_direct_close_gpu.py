@@ -1,7 +1,7 @@
 """Candidates closed where they are found (a last position, a pendant tail),
 against the oracle: own and earlier anchors, up to two further constraints, zero
 to three open look-ups, empty slices, self-loops, look-ups in hub bitmaps and in
-slices."""
+slices; and positions that intersect two or three lists."""
 import itertools
 
 import numpy as np
@@ -22,6 +22,10 @@ SHAPES = {
     "triangle-tail2": [(0, 1), (1, 2), (0, 2), (2, 3), (3, 4)],
     "square-tail2": [(0, 1), (1, 2), (2, 3), (0, 3), (1, 4), (4, 5)],
     "clique-tail1": [(0, 1), (0, 2), (0, 3), (1, 2), (1, 3), (2, 3), (1, 4)],
+    # two and three lists intersected, at a last position and before one
+    "square": [(0, 1), (1, 2), (2, 3), (0, 3)],
+    "clique": [(0, 1), (0, 2), (0, 3), (1, 2), (1, 3), (2, 3)],
+    "clique-roof": [(0, 1), (0, 2), (0, 3), (1, 2), (1, 3), (2, 3), (2, 4), (3, 4)],
 }
 
 
