@@ -18,14 +18,16 @@
 //     a hub, else by binary search, injectivity is checked against the row,
 //     and the survivors of a task are filtered (label, degree, neighbour
 //     labels) and appended with one atomic (__ballot_sync / __popc ranks);
-//   * a table chunk never holds more than `cap` rows: the host walks the
-//     levels depth-first, expanding at most `cap` elements of a level before
-//     descending, so intermediate results never exceed the scratch budget;
+//   * the levels of a call are queued at once with their sizes on the device; a
+//     level that does not fit its table stops the chain, and the host grows the
+//     table or walks on from there depth-first, expanding at most `cap` elements
+//     of a level before descending, so intermediate results never exceed the
+//     scratch budget;
 //   * in count mode the last position is never materialised: when it has a
 //     single backward neighbour its count is the slice length minus the
 //     injectivity collisions, added while expanding the position before it;
-//     a two-position pendant tail is counted from two-hop aggregates while
-//     expanding the position three before the end.
+//     a two-position pendant tail is counted from a table of two-hop aggregates
+//     while expanding the position three before the end.
 #include <algorithm>
 #include <cstring>
 #include <numeric>
