@@ -872,7 +872,11 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
     // (a lane whose tables overflowed stops: its query is counted again)
     t0 = 0;
     t1 = ONE && i == 0 ? a.T0 : a.ctr[lvl_slot(int(i), L_T)];
-    if (a.ctr[C_STOP] || (a.lane && a.ctr[C_ERR]) || t1 > a.seg_cap) return;
+    // Other warps of this launch may set C_ERR meanwhile: a warp leaves as a
+    // whole, on what its first lane saw, and no block barrier follows.  C_STOP
+    // and the sizes are left by kernels that have ended.
+    const bool stopped = a.ctr[C_STOP] || (a.lane && __ldcg(&a.ctr[C_ERR])) || t1 > a.seg_cap;
+    if (__shfl_sync(FULL, stopped ? 1 : 0, 0)) return;
   }
   const uint64_t span = t1 - t0;
   const uint32_t ntiles = uint32_t((span + EXPAND_TILE - 1) / EXPAND_TILE);
@@ -1452,7 +1456,6 @@ __global__ void __launch_bounds__(256) k_work_scan(StepArgs a, uint32_t epoch) {
   const uint32_t i = a.level;
   chain_begin();
   chain_wait();
-  if (a.ctr[C_STOP] || a.ctr[C_ERR]) return;
   const uint64_t R = dev_rows(a);
   const uint64_t ntiles = (R + WS_ROWS - 1) / WS_ROWS;
   unsigned long long bal = 0, balc = 0;
@@ -1464,13 +1467,19 @@ __global__ void __launch_bounds__(256) k_work_scan(StepArgs a, uint32_t epoch) {
   const bool o1 = i + 1 == P0.k && P0.last_o1;
   const bool fast = !a.in.qid && i > 0 && nc > 0 && !P0.zero;
   for (;;) {
-    if (threadIdx.x == 0)
-      s_tile = uint32_t(atomicAdd(&a.ctr[lvl_slot(int(i), L_SCAN)], 1ull));
+    // One thread looks at the flags, because this launch sets them too (the last
+    // tile's block C_STOP, any block C_ERR) while blocks without a tile are still
+    // starting: a block leaves or stays as a whole.
+    if (threadIdx.x == 0) {
+      const uint64_t claimed = atomicAdd(&a.ctr[lvl_slot(int(i), L_SCAN)], 1ull);
+      const bool stopped = __ldcg(&a.ctr[C_STOP]) || __ldcg(&a.ctr[C_ERR]);
+      s_tile = stopped || claimed >= ntiles ? FULL : uint32_t(claimed);
+    }
     __syncthreads();
-    const uint64_t tile = s_tile;
+    const uint32_t tile = s_tile;
     __syncthreads();
-    if (tile >= ntiles) break;
-    const uint64_t base = tile * WS_ROWS + uint64_t(threadIdx.x) * 4;
+    if (tile == FULL) break;
+    const uint64_t base = uint64_t(tile) * WS_ROWS + uint64_t(threadIdx.x) * 4;
     unsigned long long v[4] = {}, sum = 0;
     if (fast && base + 4 <= R) {
       // Four rows of one query at once: their columns are one 16-byte read, and
@@ -1564,7 +1573,7 @@ __global__ void __launch_bounds__(256) k_work_scan(StepArgs a, uint32_t epoch) {
     __syncthreads();
     const unsigned long long prefix = s_prefix;
     for (uint32_t x = threadIdx.x; x < WS_ROWS; x += 256) {
-      const uint64_t r = tile * WS_ROWS + x;
+      const uint64_t r = uint64_t(tile) * WS_ROWS + x;
       if (r < R) a.woff[r] = prefix + s_off[x];
     }
     // expand tiles that begin among these rows' elements: the last row that
@@ -1576,7 +1585,7 @@ __global__ void __launch_bounds__(256) k_work_scan(StepArgs a, uint32_t epoch) {
       uint32_t lo = 0;
       for (uint32_t d = WS_ROWS / 2; d > 0; d >>= 1)
         if (s_off[lo + d] <= t) lo += d;
-      a.tile_row[j] = uint32_t(min(tile * WS_ROWS + lo, R - 1));
+      a.tile_row[j] = uint32_t(min(uint64_t(tile) * WS_ROWS + lo, R - 1));
     }
     if (ntiles <= gridDim.x) break;  // no block takes a second tile
     __syncthreads();                 // s_off and s_prefix are written again

@@ -1,0 +1,35 @@
+"""The walk over the level tables where it stops and goes on: levels larger than
+their table, more blocks than tiles, and the limits of a call, against the oracle."""
+import numpy as np
+import pytest
+
+import matrixgraph_b200 as mg
+from helpers import oracle_count
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dense():
+    """R-MAT scale 12 with four labels: a 4-cycle has 11,119 rows at level 2, whose
+    candidate elements pass a table of 2^17 rows."""
+    g = mg.rmat(12, n_labels=4)
+    dg = mg.DeviceGraph(g)
+    yield g, dg
+    dg.free()
+
+
+@pytest.mark.parametrize("chunk_rows", [1000, 1 << 16, 1 << 17])
+@pytest.mark.parametrize("shape", ["4-cycle", "4-clique"])
+def test_stopped_levels_are_walked_again_alike(dense, shape, chunk_rows):
+    """A level that passes its table stops the chain from within the launch that
+    measures it, while most of that launch's blocks have no tile: every repetition
+    walks the same rows."""
+    g, dg = dense
+    q = mg.query_walk(g, shape, seed=3)
+    want = oracle_count(g, q, threads=4)
+    for _ in range(1 if chunk_rows < 4096 else 40):
+        got, st = dg.count(q, stats=True, chunk_rows=chunk_rows)
+        assert got == want["count"]
+        assert st["level_rows"] == want["level_rows"]
+        assert st["balg_bytes"] == want["balg"]
