@@ -260,7 +260,11 @@ struct StepArgs {
 
 // Kernels of a chain are launched as programmatic dependents: one may begin
 // before the kernel ahead of it has ended, and waits here before it reads
-// anything of it.
+// anything of it.  What a kernel of the chain writes (level tables, woff,
+// tile_row, counters) is read with ordinary loads only: the wait orders those,
+// while __ldg is for data that does not change while the kernel is resident,
+// which here are the graph's arrays and what was finished before the chain
+// began (tail tables, keep bits).
 __device__ __forceinline__ void chain_begin() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
@@ -358,8 +362,8 @@ __device__ __forceinline__ unsigned long long warp_sum(unsigned long long v) {
 }
 
 // Largest r in [lo, hi] with woff[r] <= t (woff non-decreasing, woff[lo] <= t).
-__device__ __forceinline__ uint32_t find_row(const uint64_t* __restrict__ woff, uint32_t lo,
-                                             uint32_t hi, uint64_t t) {
+__device__ __forceinline__ uint32_t find_row(const uint64_t* woff, uint32_t lo, uint32_t hi,
+                                             uint64_t t) {
   while (lo < hi) {
     uint32_t mid = (lo + hi + 1) >> 1;
     if (woff[mid] <= t) lo = mid;
@@ -1069,8 +1073,8 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
       uint64_t t = t0 + uint64_t(tile) * EXPAND_TILE + (task & ((1u << split) - 1)) * part;
       const uint64_t te = min(t + part, t1);
       if (t >= te) continue;
-      uint32_t r0 = root ? 0u : __ldg(a.tile_row + tile);
-      const uint32_t rhi = root ? 0u : __ldg(a.tile_row + tile + 1);
+      uint32_t r0 = root ? 0u : a.tile_row[tile];
+      const uint32_t rhi = root ? 0u : a.tile_row[tile + 1];
       while (t < te && !full) {
         if (r0 < rhi) r0 = find_row(a.woff, r0, rhi, t);
         // Set up 32 rows, one per lane: consecutive ones, or, where more rows

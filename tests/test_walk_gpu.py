@@ -33,3 +33,17 @@ def test_stopped_levels_are_walked_again_alike(dense, shape, chunk_rows):
         assert got == want["count"]
         assert st["level_rows"] == want["level_rows"]
         assert st["balg_bytes"] == want["balg"]
+
+
+def test_chained_levels_read_what_the_level_before_wrote(dense):
+    """Calls of many levels back to back, whose launches overlap and share one table
+    of tile rows: three queries of other sizes in turn, each the same every time."""
+    g, dg = dense
+    qs = [mg.query_walk(g, s, seed=7) for s in ("4-cycle", "4-clique", "tailed-triangle")]
+    want = [oracle_count(g, q, threads=4) for q in qs]
+    for q in qs:  # tables grow to what the queries need
+        dg.count(q, no_tail=1)
+    for _ in range(40):
+        for q, w in zip(qs, want):
+            got, st = dg.count(q, stats=True, no_tail=1)
+            assert got == w["count"] and st["level_rows"] == w["level_rows"]
