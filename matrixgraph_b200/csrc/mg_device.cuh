@@ -147,12 +147,15 @@ struct DeviceGuard {
 int matrix_filter_roots(void* filter, const DevGraph* dg, uint32_t u, uint32_t lab,
                         uint32_t* bits, cudaStream_t st);
 
+// (a failure that the context survives is not left for the next check to find)
 #define MG_CK(call)                                                          \
   do {                                                                       \
     cudaError_t _e = (call);                                                 \
-    if (_e != cudaSuccess)                                                   \
-      return ::mg::set_error(MG_E_CUDA, "%s:%d %s: %s", __FILE__, __LINE__, \
+    if (_e != cudaSuccess) {                                                 \
+      cudaGetLastError();                                                    \
+      return ::mg::set_error(MG_E_CUDA, "%s:%d %s: %s", __FILE__, __LINE__,  \
                              #call, cudaGetErrorString(_e));                 \
+    }                                                                        \
   } while (0)
 
 // cudaMalloc that records the allocation on the graph and maps failure to

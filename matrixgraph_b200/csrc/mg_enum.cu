@@ -30,6 +30,7 @@
 //     while expanding the position three before the end.
 #include <algorithm>
 #include <cstring>
+#include <memory>
 #include <numeric>
 #include <type_traits>
 
@@ -169,16 +170,19 @@ static int ensure_level(Workspace* ws, int l, uint64_t rows) {
 
 // Scratch of a walk with level tables of at most `cap` rows for nq queries.
 static int ensure_ws(DevGraph* dg, uint64_t cap, uint32_t nq) {
-  Workspace*& ws = dg->ws;
   int rc;
-  if (!ws) {
-    ws = new Workspace();
+  if (!dg->ws) {
+    // Built aside: the graph never keeps a workspace that is not complete.
+    std::unique_ptr<Workspace, void (*)(Workspace*)> made(new Workspace(), free_workspace);
     static_assert(sizeof(PlanDev) % 8 == 0, "the result block follows the plan");
-    MG_CK(cudaMallocHost((void**)&ws->h_plan, sizeof(PlanDev) + res_words(1) * 8));
-    ws->h_res = reinterpret_cast<unsigned long long*>(ws->h_plan + 1);
-    for (cudaEvent_t* e : {&ws->ev0, &ws->ev1, &ws->ev2, &ws->ev3}) MG_CK(cudaEventCreate(e));
-    if ((rc = ws_alloc((void**)&ws->tile_row, (kSegment / EXPAND_TILE + 2) * 4))) return rc;
+    MG_CK(cudaMallocHost((void**)&made->h_plan, sizeof(PlanDev) + res_words(1) * 8));
+    made->h_res = reinterpret_cast<unsigned long long*>(made->h_plan + 1);
+    for (cudaEvent_t* e : {&made->ev0, &made->ev1, &made->ev2, &made->ev3})
+      MG_CK(cudaEventCreate(e));
+    if ((rc = ws_alloc((void**)&made->tile_row, (kSegment / EXPAND_TILE + 2) * 4))) return rc;
+    dg->ws = made.release();
   }
+  Workspace* ws = dg->ws;
   const uint64_t status = (std::max<uint64_t>(cap, nq) / WS_ROWS + 2) * 8;
   if (ws->status_bytes < status) {
     ws->status_bytes = 0;
@@ -2502,9 +2506,8 @@ struct LaneSet {
   std::vector<Lane> lanes;
   std::vector<void*> allocs;
   unsigned long long *r_counts = nullptr, *r_lvl = nullptr, *r_err = nullptr, *r_balg = nullptr;
-  uint32_t r_cap = 0;
   PlanDev* plans = nullptr;
-  uint32_t plans_cap = 0;
+  uint32_t nq_cap = 0;  // queries that plans and the results hold
   TailStore tails;
   cudaEvent_t ev_start = nullptr, ev_end = nullptr;
 };
@@ -2518,6 +2521,9 @@ void free_lanes(LaneSet* ls) {
   for (Lane& l : ls->lanes)
     if (l.st) cudaStreamDestroy(l.st);
   for (void* p : ls->allocs) cudaFree(p);
+  for (void* p : {(void*)ls->plans, (void*)ls->r_counts, (void*)ls->r_lvl, (void*)ls->r_err,
+                  (void*)ls->r_balg})
+    cudaFree(p);
   ls->tails.free();
   if (ls->ev_start) cudaEventDestroy(ls->ev_start);
   if (ls->ev_end) cudaEventDestroy(ls->ev_end);
@@ -2538,14 +2544,16 @@ static int lane_alloc(LaneSet* ls, void** p, size_t bytes) {
 }
 
 static int ensure_lanes(DevGraph* dg, uint32_t nl, uint64_t cap, uint32_t kmax) {
-  LaneSet*& ls = dg->lanes;
-  if (ls && (ls->lanes.size() != nl || ls->cap != cap || ls->kmax < kmax)) {
+  if (dg->lanes &&
+      (dg->lanes->lanes.size() != nl || dg->lanes->cap != cap || dg->lanes->kmax < kmax)) {
     cudaDeviceSynchronize();
-    free_lanes(ls);
-    ls = nullptr;
+    free_lanes(dg->lanes);
+    dg->lanes = nullptr;
   }
-  if (ls) return MG_OK;
-  ls = new LaneSet();
+  if (dg->lanes) return MG_OK;
+  // Built aside: the graph never keeps a set of lanes that is not complete.
+  std::unique_ptr<LaneSet, void (*)(LaneSet*)> made(new LaneSet(), free_lanes);
+  LaneSet* ls = made.get();
   ls->cap = cap;
   ls->seg_cap = kLaneSegment;
   ls->kmax = std::max<uint32_t>(kmax, 8);
@@ -2579,8 +2587,23 @@ static int ensure_lanes(DevGraph* dg, uint32_t nl, uint64_t cap, uint32_t kmax) 
       }
       if (pass == 0 && (rc = lane_alloc(ls, (void**)&p, off))) return rc;
     }
-    MG_CK(cudaMemset(L.status, 0, ntiles * 8));
+    MG_CK(cudaMemsetAsync(L.status, 0, ntiles * 8, L.st));
   }
+  dg->lanes = made.release();
+  return MG_OK;
+}
+
+// Plans and results of nq queries of a batch.
+static int ensure_lane_queries(LaneSet* ls, uint32_t nq) {
+  int rc;
+  if (ls->nq_cap >= nq) return MG_OK;
+  ls->nq_cap = 0;
+  if ((rc = ws_alloc((void**)&ls->plans, uint64_t(nq) * sizeof(PlanDev)))) return rc;
+  if ((rc = ws_alloc((void**)&ls->r_counts, uint64_t(nq) * 8))) return rc;
+  if ((rc = ws_alloc((void**)&ls->r_lvl, uint64_t(nq) * (MAXK + 1) * 8))) return rc;
+  if ((rc = ws_alloc((void**)&ls->r_err, uint64_t(nq) * 8))) return rc;
+  if ((rc = ws_alloc((void**)&ls->r_balg, uint64_t(nq) * 16))) return rc;
+  ls->nq_cap = nq;
   return MG_OK;
 }
 
@@ -2599,17 +2622,7 @@ static int subiso_batch_lanes(DevGraph* dg, std::vector<PlanDev>& plans, const m
   cudaStream_t st = dg->stream;
   const unsigned sms = dg->sms;
 
-  if (ls->plans_cap < nq) {
-    if ((rc = lane_alloc(ls, (void**)&ls->plans, uint64_t(nq) * sizeof(PlanDev)))) return rc;
-    ls->plans_cap = nq;
-  }
-  if (ls->r_cap < nq) {
-    if ((rc = lane_alloc(ls, (void**)&ls->r_counts, uint64_t(nq) * 8))) return rc;
-    if ((rc = lane_alloc(ls, (void**)&ls->r_lvl, uint64_t(nq) * (MAXK + 1) * 8))) return rc;
-    if ((rc = lane_alloc(ls, (void**)&ls->r_err, uint64_t(nq) * 8))) return rc;
-    if ((rc = lane_alloc(ls, (void**)&ls->r_balg, uint64_t(nq) * 16))) return rc;
-    ls->r_cap = nq;
-  }
+  if ((rc = ensure_lane_queries(ls, nq))) return rc;
   Workspace* ws = dg->ws;  // timing events live with the graph's workspace
   if (!ws && (rc = ensure_ws(dg, 1ull << 16, 1))) return rc;
   ws = dg->ws;
@@ -2786,10 +2799,7 @@ static int selftest_wait(DevGraph* dg, const mg_csr_view* q, uint32_t spin_limit
   if ((rc = ensure_lanes(dg, 1, kLaneCap, std::max<uint32_t>(P.k, 2)))) return rc;
   LaneSet* ls = dg->lanes;
   Lane& L = ls->lanes[0];
-  if (ls->plans_cap < 1) {
-    if ((rc = lane_alloc(ls, (void**)&ls->plans, sizeof(PlanDev)))) return rc;
-    ls->plans_cap = 1;
-  }
+  if ((rc = ensure_lane_queries(ls, 1))) return rc;
   cudaStream_t st = L.st;
   const uint64_t rows = 2 * WS_ROWS;
   std::vector<unsigned long long> ctr(C_NUM, 0);

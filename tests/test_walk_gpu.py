@@ -4,6 +4,7 @@ import numpy as np
 import pytest
 
 import matrixgraph_b200 as mg
+from matrixgraph_b200 import _lib as L
 from helpers import oracle_count
 
 pytestmark = pytest.mark.gpu
@@ -47,3 +48,18 @@ def test_chained_levels_read_what_the_level_before_wrote(dense):
         for q, w in zip(qs, want):
             got, st = dg.count(q, stats=True, no_tail=1)
             assert got == w["count"] and st["level_rows"] == w["level_rows"]
+
+
+def test_batch_after_lanes_that_did_not_fit(dense):
+    """Lane tables for 2^31 rows (over 400 GB) are refused as often as they are asked
+    for, and leave nothing behind that a later batch would use."""
+    g, dg = dense
+    qs = [mg.query_walk(g, "4-clique", seed=s) for s in range(3)]
+    want = [oracle_count(g, q, threads=4)["count"] for q in qs]
+    for _ in range(2):
+        with pytest.raises(L.MGError) as e:
+            dg.batch_count(qs, chunk_rows=1 << 31, lanes=2)
+        assert e.value.code == L.MG_E_OOM
+    assert dg.batch_count(qs, lanes=2).tolist() == want
+    assert dg.batch_count(qs * 40, lanes=2).tolist() == want * 40
+    assert dg.batch_count(qs, lanes=2).tolist() == want
