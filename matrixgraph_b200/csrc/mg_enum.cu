@@ -35,6 +35,7 @@
 #include <type_traits>
 
 #include "mg_device.cuh"
+#include "mg_limits.h"
 #include "mg_row_sort.cuh"
 
 namespace mg {
@@ -2678,7 +2679,7 @@ static int subiso_batch_lanes(DevGraph* dg, std::vector<PlanDev>& plans, const m
     a.scan_status = L.status;
     a.tile_row = L.tile_row;
     int last = P.zero ? -1 : last_level(P, a.tail_dense != 0, a.star != 0);
-    if (o.max_elements && t0[j] > o.max_elements) last = -1;
+    if (lane_start(t0[j], o.max_elements, ls->seg_cap) != LaneStart::kRun) last = -1;
     a.T0 = t0[j];
     a.root_first = first[j];
     uint64_t rows = 1;
@@ -2736,6 +2737,8 @@ static int subiso_batch_lanes(DevGraph* dg, std::vector<PlanDev>& plans, const m
   MG_CK(cudaEventElapsedTime(&ms, ws->ev0, ws->ev1));
   res->ms = ms;
   for (uint32_t j = 0; j < nq; ++j) {
+    if (lane_start(t0[j], o.max_elements, ls->seg_cap) == LaneStart::kChunked)
+      err[j] |= ERR_OVERFLOW;
     if (err[j]) continue;  // charged by its re-run below
     res->balg += balg[2ull * j] + t0[j] * root_charge(dg);
     res->balgc += balg[2ull * j + 1] + t0[j] * root_charge(dg);

@@ -1,0 +1,35 @@
+"""Limits of an enumeration call at sizes that no test puts on a device."""
+import os
+import subprocess
+
+import pytest
+
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
+
+
+@pytest.fixture(scope="module")
+def limits(tmp_path_factory):
+    exe = str(tmp_path_factory.mktemp("limits") / "limits")
+    subprocess.run(["g++", "-O1", "-std=c++17", "-Wall", "-Werror", "-I",
+                    os.path.join(ROOT, "matrixgraph_b200", "csrc"),
+                    os.path.join(ROOT, "tests", "limits_main.cpp"), "-o", exe], check=True)
+
+    def run(*args):
+        r = subprocess.run([exe] + [str(a) for a in args], capture_output=True, text=True,
+                           check=True)
+        return [int(x) for x in r.stdout.split()]
+    return run
+
+
+RUN, UNKNOWN, CHUNKED = 0, 1, 2
+SEG = 1 << 30  # elements of a lane's expand launch
+
+
+@pytest.mark.parametrize("t0, budget, want", [
+    (0, 0, RUN), (1, 0, RUN), (SEG, 0, RUN), (SEG + 1, 0, CHUNKED), ((1 << 32) - 1, 0, CHUNKED),
+    (100, 100, RUN), (101, 100, UNKNOWN), (SEG + 1, SEG, UNKNOWN), (SEG + 1, SEG + 1, CHUNKED),
+])
+def test_first_bucket_of_a_batch_query(limits, t0, budget, want):
+    """A bucket larger than a lane's launch is counted on the chunked path: the lane
+    has no kernel at level 0 that could say so, and would report 0."""
+    assert limits("lane_start", t0, budget, SEG) == [want]
