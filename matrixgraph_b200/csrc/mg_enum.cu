@@ -135,7 +135,6 @@ constexpr int XSTAGE = 256;                       // survivors a warp stages at 
 constexpr uint64_t kSegment = 1ull << 30;         // elements per expand launch
 constexpr int WS_ROWS = 1024;                     // rows per work/scan tile (4 per thread)
 constexpr uint32_t kSpinLimit = 1u << 22;         // polls of a look-back wait (~0.3 s)
-constexpr uint32_t kEpochMax = (1u << 20) - 1;
 // Words of the result block of nq queries.
 constexpr uint64_t res_words(uint64_t nq) { return C_NUM + nq * (MAXK + 3); }
 
@@ -1404,16 +1403,6 @@ __global__ void __launch_bounds__(EXPAND_BLOCK, (MODE & X_TAIL) ? 3 : 4) k_expan
 }
 
 // ---- work and scan -----------------------------------------------------------
-// Look-back words of the single-pass work/scan: [epoch:20 | status:2 | value:42].
-constexpr int LB_VALUE_BITS = 42;
-constexpr unsigned long long LB_AGG = 1, LB_INC = 2;
-
-__device__ __forceinline__ unsigned long long lb_word(uint32_t epoch, unsigned long long st,
-                                                      unsigned long long v) {
-  return (uint64_t(epoch) << (LB_VALUE_BITS + 2)) | (st << LB_VALUE_BITS) |
-         (v & ((1ull << LB_VALUE_BITS) - 1));
-}
-
 // Sum of the tiles before `tile` (decoupled look-back by one warp, 32
 // predecessors at a time: back to the nearest inclusive prefix).  A tile only
 // waits for tiles claimed before it, whose blocks are running; every wait gives
@@ -1430,7 +1419,7 @@ __device__ __forceinline__ unsigned long long look_back(const StepArgs& a, uint3
       uint32_t spins = 0;
       for (;;) {
         w = *st;
-        if ((w >> (LB_VALUE_BITS + 2)) == epoch && ((w >> LB_VALUE_BITS) & 3ull)) break;
+        if (lb_epoch(w) == epoch && lb_state(w)) break;
         if (++spins > a.spin_limit) {
           atomicOr(&a.ctr[C_ERR], (unsigned long long)ERR_TIMEOUT);
           w = lb_word(epoch, LB_INC, 0);
@@ -1440,9 +1429,9 @@ __device__ __forceinline__ unsigned long long look_back(const StepArgs& a, uint3
       }
     }
     __syncwarp();
-    const uint32_t inc = __ballot_sync(FULL, ((w >> LB_VALUE_BITS) & 3ull) == LB_INC);
+    const uint32_t inc = __ballot_sync(FULL, lb_state(w) == LB_INC);
     const uint32_t upto = inc ? __ffs(inc) - 1 : 31u;
-    unsigned long long v = lane <= upto ? w & ((1ull << LB_VALUE_BITS) - 1) : 0ull;
+    unsigned long long v = lane <= upto ? lb_value(w) : 0ull;
     v = warp_sum(v);
     prefix += __shfl_sync(FULL, v, 0);
     if (inc) break;
@@ -1558,12 +1547,10 @@ __global__ void __launch_bounds__(256) k_work_scan(StepArgs a, uint32_t epoch) {
         atomicExch(a.scan_status + tile, lb_word(epoch, tile == 0 ? LB_INC : LB_AGG, tot));
       const unsigned long long prefix = look_back(a, epoch, tile);
       if (threadIdx.x == 0) {
-        if (tile > 0) atomicExch(a.scan_status + tile, lb_word(epoch, LB_INC, prefix + tot));
-        if (prefix + tot >= (1ull << LB_VALUE_BITS))
-          atomicOr(&a.ctr[C_ERR], (unsigned long long)ERR_OVERFLOW);
+        const unsigned long long T = lb_sum(prefix, tot);  // elements up to this tile
+        if (tile > 0) atomicExch(a.scan_status + tile, lb_word(epoch, LB_INC, T));
         s_prefix = prefix;
         if (tile + 1 == ntiles) {
-          const unsigned long long T = prefix + tot;
           a.woff[R] = T;
           a.ctr[lvl_slot(int(i), L_T)] = T;
           if (T <= a.seg_cap)
@@ -2065,12 +2052,13 @@ static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool cou
       set_level(l);
       a.t_limit = writes[l] ? std::min(held(l + 1), B.seg) : B.seg;
       if (one && o.max_elements) a.t_limit = std::min(a.t_limit, o.max_elements - elements);
-      if (++*B.epoch > kEpochMax) {
+      const bool clear = ++*B.epoch > LB_EPOCHS;
+      if (clear) {
         MG_CK(cudaMemsetAsync(B.status, 0, B.status_bytes, st));
         *B.epoch = 1;
       }
-      launch_chained(k_work_scan, grid_for(rows, WS_ROWS, sms * 4), 256u, st, one && l > l0, a,
-                     *B.epoch);
+      launch_chained(k_work_scan, grid_for(rows, WS_ROWS, sms * 4), 256u, st,
+                     one && l > l0 && !clear, a, *B.epoch);
       res->launches++;
       const uint64_t bound = std::min(bounded_product(rows, widest[l]), a.t_limit);
       if (int r = expand(l, bound)) return r;
@@ -2099,7 +2087,11 @@ static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool cou
       if (h[C_STOP] == uint64_t(l) + 1) {
         cur[l] = 0;
         *stop = l;
-        return T[l] > budget - elements ? refuse() : int(MG_OK);
+        if (T[l] > budget - elements) return refuse();
+        if (T[l] >= LB_MAX)
+          return set_error(MG_E_LIMIT, "a level of 2^%d or more candidate elements",
+                           LB_VALUE_BITS);
+        return MG_OK;
       }
       if (T[l] > budget - elements) return refuse();
       cur[l] = T[l];
@@ -2692,7 +2684,7 @@ static int subiso_batch_lanes(DevGraph* dg, std::vector<PlanDev>& plans, const m
       a.dstart = L.dstart[l];
       a.dci = L.dci[l];
       if (l > 0) {
-        if (++L.epoch > kEpochMax) {
+        if (++L.epoch > LB_EPOCHS) {
           MG_CK(cudaMemsetAsync(L.status, 0, (cap / WS_ROWS + 2) * 8, L.st));
           L.epoch = 1;
         }
@@ -2834,7 +2826,7 @@ static int selftest_wait(DevGraph* dg, const mg_csr_view* q, uint32_t spin_limit
   a.scan_status = L.status;
   a.spin_limit = spin_limit;
   a.root_step = 1;
-  if (++L.epoch > kEpochMax) {
+  if (++L.epoch > LB_EPOCHS) {
     MG_CK(cudaMemsetAsync(L.status, 0, (ls->cap / WS_ROWS + 2) * 8, st));
     L.epoch = 1;
   }

@@ -4,7 +4,35 @@
 
 #include <cstdint>
 
+#ifdef __CUDACC__
+#define MG_HD __host__ __device__ __forceinline__
+#else
+#define MG_HD inline
+#endif
+
 namespace mg {
+
+// Look-back words of the single-pass work/scan: [epoch:8 | state:2 | value:54].
+// A level's element total can pass 2^42 in ordinary use (a position that is not
+// joined to the one before it), so the value has what the epoch does not need;
+// the words are cleared when the epochs run out.  Sums stay at LB_MAX once they
+// reach it, which no walk could expand anyway (days at 10^11 elements/s).
+constexpr int LB_VALUE_BITS = 54;
+constexpr uint32_t LB_EPOCHS = (1u << (62 - LB_VALUE_BITS)) - 1;  // 1..LB_EPOCHS
+constexpr unsigned long long LB_AGG = 1, LB_INC = 2;  // a tile's sum, sum up to it
+constexpr unsigned long long LB_MAX = (1ull << LB_VALUE_BITS) - 1;
+
+// a + b, at most LB_MAX (a and b themselves may be any sums below 2^63).
+MG_HD unsigned long long lb_sum(unsigned long long a, unsigned long long b) {
+  const unsigned long long s = a + b;
+  return s < LB_MAX ? s : LB_MAX;
+}
+MG_HD unsigned long long lb_word(uint32_t epoch, unsigned long long state, unsigned long long v) {
+  return (unsigned long long)(epoch) << (LB_VALUE_BITS + 2) | state << LB_VALUE_BITS | v;
+}
+MG_HD uint32_t lb_epoch(unsigned long long w) { return uint32_t(w >> (LB_VALUE_BITS + 2)); }
+MG_HD unsigned long long lb_state(unsigned long long w) { return w >> LB_VALUE_BITS & 3ull; }
+MG_HD unsigned long long lb_value(unsigned long long w) { return w & LB_MAX; }
 
 // What a batch lane does with a query of t0 level-0 candidates.  Its expand
 // launch covers at most seg_cap elements; at the later levels k_work_scan flags a

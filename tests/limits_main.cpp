@@ -12,5 +12,12 @@ int main(int argc, char** argv) {
     std::printf("%d\n", int(mg::lane_start(arg(2), arg(3), arg(4))));
     return 0;
   }
+  if (!std::strcmp(what, "look_back")) {  // epoch, state, a, b: the word of a + b, taken apart
+    const unsigned long long w =
+        mg::lb_word(uint32_t(arg(2)), arg(3), mg::lb_sum(arg(4), arg(5)));
+    std::printf("%u %llu %llu %llu %u\n", mg::lb_epoch(w), mg::lb_state(w), mg::lb_value(w),
+                mg::LB_MAX, mg::LB_EPOCHS);
+    return 0;
+  }
   return 2;
 }

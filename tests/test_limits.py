@@ -33,3 +33,16 @@ def test_first_bucket_of_a_batch_query(limits, t0, budget, want):
     """A bucket larger than a lane's launch is counted on the chunked path: the lane
     has no kernel at level 0 that could say so, and would report 0."""
     assert limits("lane_start", t0, budget, SEG) == [want]
+
+
+@pytest.mark.parametrize("epoch", [1, 2, 255])
+@pytest.mark.parametrize("state", [1, 2])
+@pytest.mark.parametrize("a, b", [
+    (0, 0), ((1 << 42) - 1, 1), (9 * 10 ** 12, 0), ((1 << 53), (1 << 53) - 2),
+    ((1 << 54) - 2, 1), ((1 << 54) - 1, 1), ((1 << 54) - 1, 1 << 42), (1 << 61, 1 << 42),
+])
+def test_look_back_words(limits, epoch, state, a, b):
+    """Element sums pass 2^42 unharmed and stop at the largest value, in words that
+    keep their epoch and state."""
+    most = (1 << 54) - 1
+    assert limits("look_back", epoch, state, a, b) == [epoch, state, min(a + b, most), most, 255]

@@ -63,3 +63,32 @@ def test_batch_after_lanes_that_did_not_fit(dense):
     assert dg.batch_count(qs, lanes=2).tolist() == want
     assert dg.batch_count(qs * 40, lanes=2).tolist() == want * 40
     assert dg.batch_count(qs, lanes=2).tolist() == want
+
+
+def test_level_of_more_than_2_42_elements_meets_the_budget():
+    """A second vertex that is not joined to the first: 2.2M rows of 2.2M candidates
+    each, refused by the work budget in a single call and reported as unknown in a
+    batch, whose other queries are counted."""
+    n = 2_200_000
+    v = np.arange(n, dtype=np.uint32)
+    g = mg.CSRGraph.from_edges(n, v, np.roll(v, -1), np.zeros(n, np.uint32), symmetrize=True)
+    dg = mg.DeviceGraph(g)
+    q = mg.CSRGraph.query(3, [(0, 1), (1, 2)], [0, 0, 0])
+    with pytest.raises(L.MGError) as e:
+        dg.count(q, given_order=[0, 2, 1], max_elements=1 << 30)
+    assert e.value.code == L.MG_E_LIMIT
+    counts, _, _ = dg.batch_count_orders([q, q], [[0, 2, 1], [1, 0, 2]], max_elements=1 << 30)
+    assert counts.tolist() == [2 ** 64 - 1, 2 * n]
+    assert dg.count(q) == 2 * n
+    dg.free()
+
+
+def test_more_work_scans_than_epochs(dense):
+    """Hundreds of chunks in one call: the look-back words are cleared when their
+    epochs run out."""
+    g, dg = dense
+    q = mg.query_walk(g, "4-cycle", seed=3)
+    want = oracle_count(g, q, threads=4)
+    got, st = dg.count(q, stats=True, chunk_rows=1500)
+    assert st["chunks"] > 600
+    assert got == want["count"] and st["level_rows"] == want["level_rows"]
