@@ -2283,13 +2283,14 @@ static int run_levels(DevGraph* dg, std::vector<PlanDev> plans, bool count_mode,
   B.done = ws->ev1;
   B.ev2 = ws->ev2;
   B.ev3 = ws->ev3;
-  if ((rc = walk_levels(dg, plans.data(), nq, count_mode, o, a, B, res))) {
+  rc = walk_levels(dg, plans.data(), nq, count_mode, o, a, B, res);
+  float ms = 0;
+  if (rc == MG_OK || res->emit_full) MG_CK(cudaEventElapsedTime(&ms, ws->ev0, ws->ev1));
+  res->ms = ms;
+  if (rc) {
     cudaStreamSynchronize(st);
     return rc;
   }
-  float ms = 0;
-  MG_CK(cudaEventElapsedTime(&ms, ws->ev0, ws->ev1));
-  res->ms = ms;
   const unsigned long long *cnt = ws->h_res + C_NUM, *lvl = cnt + nq, *qel = lvl + MAXK + 1;
   std::vector<unsigned long long> all;
   if (batch) {
@@ -2426,30 +2427,33 @@ int subiso_emit(DevGraph* dg, const mg_csr_view* q, const mg_opts* opts, const R
   if (rc) return rc;
   std::vector<PlanDev> plans(1, P);
   cudaStream_t s = dg->stream;
-  RunResult res, res2;
+  RunResult tried, counted, res;  // an attempt, a count, the pass that gave the rows
   RowBuf eb;
   uint64_t c = 0, unused = 0;
   const uint64_t room = std::min(std::max(sink.cap_rows, kEmitTryMin), kEmitTry);
   rc = emit_buffer(dg, P.k, room, &eb);
-  if (rc == MG_OK) rc = run_levels(dg, plans, false, &eb, o, &unused, &res2);
+  const bool no_room = rc == MG_E_OOM;
   if (rc == MG_OK) {
-    c = *n_rows = res2.emitted;
-  } else {
-    // Too many for the buffer, or refused: counted first.
+    rc = run_levels(dg, plans, false, &eb, o, &unused, &res);
+    if (rc == MG_OK) c = *n_rows = res.emitted;
+    else if (res.emit_full) std::swap(tried, res);
+  }
+  if (no_room || tried.emit_full) {
+    // More matches than the buffer holds, or no memory for it: counted first.
+    // Every other failure (a refused budget, a wait that gave up) is the call's.
     clear_error();
-    res2 = RunResult();
-    if ((rc = run_levels(dg, plans, true, nullptr, o, &c, &res))) return rc;
-    *n_rows = c;
-    if (c >= (1ull << 31))
-      return set_error(MG_E_LIMIT, "%llu matches: emit supports fewer than 2^31 rows",
-                       (unsigned long long)c);
-    rc = emit_buffer(dg, P.k, c, &eb);
-    if (rc == MG_OK) rc = run_levels(dg, plans, false, &eb, o, &unused, &res2);
-    if (rc == MG_OK && res2.emitted != c)
+    rc = run_levels(dg, plans, true, nullptr, o, &c, &counted);
+    if (rc == MG_OK) *n_rows = c;
+    if (rc == MG_OK && c >= (1ull << 31))
+      rc = set_error(MG_E_LIMIT, "%llu matches: emit supports fewer than 2^31 rows",
+                     (unsigned long long)c);
+    if (rc == MG_OK) rc = emit_buffer(dg, P.k, c, &eb);
+    if (rc == MG_OK) rc = run_levels(dg, plans, false, &eb, o, &unused, &res);
+    if (rc == MG_OK && res.emitted != c)
       rc = set_error(MG_E_CUDA, "emit pass produced %llu rows, count pass %llu",
-                     (unsigned long long)res2.emitted, (unsigned long long)c);
-    res2.balg = res.balg;
-    res2.balgc = res.balgc;
+                     (unsigned long long)res.emitted, (unsigned long long)c);
+    res.balg = counted.balg;
+    res.balgc = counted.balgc;
   }
   if (rc == MG_OK) {
     const uint64_t n_copy = std::min(c, sink.cap_rows);
@@ -2461,8 +2465,9 @@ int subiso_emit(DevGraph* dg, const mg_csr_view* q, const mg_opts* opts, const R
   cudaStreamSynchronize(s);
   trim_emit(dg);
   if (rc) return rc;
-  fill_stats(st, P, res2, c);
-  if (st) st->device_ms = res.ms + res2.ms;
+  res.ms += tried.ms + counted.ms;
+  res.launches += tried.launches + counted.launches;
+  fill_stats(st, P, res, c);
   if (c > sink.cap_rows)
     return set_error(MG_E_CAPACITY, "%llu matches, %llu rows written",
                      (unsigned long long)c, (unsigned long long)sink.cap_rows);

@@ -5,7 +5,7 @@ import pytest
 
 import matrixgraph_b200 as mg
 from matrixgraph_b200 import _lib as L
-from helpers import oracle_count
+from helpers import oracle_count, oracle_rows
 
 pytestmark = pytest.mark.gpu
 
@@ -92,3 +92,24 @@ def test_more_work_scans_than_epochs(dense):
     got, st = dg.count(q, stats=True, chunk_rows=1500)
     assert st["chunks"] > 600
     assert got == want["count"] and st["level_rows"] == want["level_rows"]
+
+
+def test_emit_falls_back_only_when_its_buffer_is_full(dense):
+    """An emit whose matches pass its buffer counts and emits again, and its launches
+    say so; one that its budget refuses is refused at once and counted as nothing."""
+    g, dg = dense
+    q = mg.query_walk(g, "4-clique", seed=7)
+    want = oracle_rows(g, q)
+    assert len(want) > 1 << 16  # rows that an attempt has room for at least
+    for _ in range(2):  # (the level tables have grown at the second call)
+        counted = dg.count(q, stats=True)[1]["launches"]
+        dg.emit(q, cap=len(want))
+    rows, n, once = dg.emit(q, cap=len(want), stats=True)
+    assert n == len(want) and np.array_equal(rows, want)
+    rows, n, again = dg.emit(q, cap=10, stats=True)
+    assert n == len(want) and np.array_equal(rows, want[:10])
+    assert again["launches"] >= once["launches"] + counted
+    with pytest.raises(L.MGError) as e:
+        dg.emit(q, max_elements=1000)
+    assert e.value.code == L.MG_E_LIMIT
+    assert np.array_equal(dg.emit(q), want)
