@@ -2383,9 +2383,14 @@ int subiso_count(DevGraph* dg, const mg_csr_view* q, const mg_opts* opts, uint64
 // as needed and is given back by trim_emit when it is large.
 constexpr uint64_t kEmitKeep = 1ull << 30;
 
-static int emit_buffer(DevGraph* dg, uint32_t k, uint64_t cap, RowBuf* B) {
+static uint32_t id_bits(const DevGraph* dg) {
   uint32_t bits = 1;
   while (bits < 32 && dg->max_gid >> bits) ++bits;
+  return bits;
+}
+
+static int emit_buffer(DevGraph* dg, uint32_t k, uint64_t cap, RowBuf* B) {
+  const uint32_t bits = id_bits(dg);
   const uint64_t bytes = B->carve(nullptr, k, bits, cap);
   if (dg->emit_bytes < bytes) {
     MG_CK(cudaStreamSynchronize(dg->stream));
@@ -2411,14 +2416,12 @@ static void trim_emit(DevGraph* dg) {
   dg->emit_bytes = 0;
 }
 
-// Matches are emitted at once into a buffer for the caller's rows (bounded by
-// kEmitTry); only a query with more of them is counted first and emitted into a
-// buffer of that size.  With a count before every emit, nine allocations a call
-// and the column-wise sort, an emit of some thousand rows on a 10,000-vertex
-// graph took 1,384 us; it takes 185 us.  Triangles of R-MAT scale 18 (16,000 to
-// 2 million rows): 2.1 -> 0.9 ms.
-constexpr uint64_t kEmitTryMin = 1ull << 16, kEmitTry = 1ull << 22;
-
+// Matches are emitted at once into a buffer for the caller's rows (emit_room);
+// only a query with more of them, or a caller with room for very many, is
+// counted first and emitted into a buffer of that size.  With a count before
+// every emit, nine allocations a call and the column-wise sort, an emit of some
+// thousand rows on a 10,000-vertex graph took 1,384 us; it takes 185 us.
+// Triangles of R-MAT scale 18 (16,000 to 2 million rows): 2.1 -> 0.9 ms.
 int subiso_emit(DevGraph* dg, const mg_csr_view* q, const mg_opts* opts, const RowSink& sink,
                 uint64_t* n_rows, mg_stats* st) {
   const mg_opts o = resolve_opts(opts);
@@ -2430,10 +2433,12 @@ int subiso_emit(DevGraph* dg, const mg_csr_view* q, const mg_opts* opts, const R
   RunResult tried, counted, res;  // an attempt, a count, the pass that gave the rows
   RowBuf eb;
   uint64_t c = 0, unused = 0;
-  const uint64_t room = std::min(std::max(sink.cap_rows, kEmitTryMin), kEmitTry);
-  rc = emit_buffer(dg, P.k, room, &eb);
-  const bool no_room = rc == MG_E_OOM;
-  if (rc == MG_OK) {
+  const uint64_t room = emit_room(!sink.alloc, sink.cap_rows, kEmitKeep, [&](uint64_t rows) {
+    return RowBuf().carve(nullptr, P.k, id_bits(dg), rows);
+  });
+  if (room) rc = emit_buffer(dg, P.k, room, &eb);
+  const bool no_room = !room || rc == MG_E_OOM;
+  if (!no_room && rc == MG_OK) {
     rc = run_levels(dg, plans, false, &eb, o, &unused, &res);
     if (rc == MG_OK) c = *n_rows = res.emitted;
     else if (res.emit_full) std::swap(tried, res);

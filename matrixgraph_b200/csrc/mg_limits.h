@@ -47,4 +47,22 @@ inline LaneStart lane_start(uint64_t t0, uint64_t budget, uint64_t seg_cap) {
   return t0 > seg_cap ? LaneStart::kChunked : LaneStart::kRun;
 }
 
+// Rows that an emit call makes room for before it knows how many there are, or 0:
+// count first.  The caller has memory for cap_rows rows (known), or takes any
+// number.  A buffer of up to `limit` bytes is tried at its full size, so that
+// what fits the caller is enumerated once; a larger one is counted first, since
+// an attempt at less than the caller's room would be a third enumeration of just
+// those results that are large.  bytes(rows): size of the buffer.
+constexpr uint64_t kEmitTryMin = 1ull << 16, kEmitTry = 1ull << 22;
+
+template <class Bytes>
+inline uint64_t emit_room(bool known, uint64_t cap_rows, uint64_t limit, Bytes bytes) {
+  if (known) {
+    if (cap_rows >= 1ull << 31) return 0;
+    const uint64_t room = cap_rows > kEmitTryMin ? cap_rows : kEmitTryMin;
+    return bytes(room) <= limit ? room : 0;
+  }
+  return kEmitTry;
+}
+
 }  // namespace mg

@@ -46,3 +46,18 @@ def test_look_back_words(limits, epoch, state, a, b):
     keep their epoch and state."""
     most = (1 << 54) - 1
     assert limits("look_back", epoch, state, a, b) == [epoch, state, min(a + b, most), most, 255]
+
+
+MIN, TRY = 1 << 16, 1 << 22
+GIB = 1 << 30
+
+
+@pytest.mark.parametrize("cap, limit, row, want", [
+    (0, GIB, 33, MIN), (1, GIB, 33, MIN), (MIN, GIB, 33, MIN), (MIN + 1, GIB, 33, MIN + 1),
+    (TRY, GIB, 33, TRY), (TRY + 1, GIB, 33, TRY + 1), (5 * 10 ** 6, GIB, 33, 5 * 10 ** 6),
+    (GIB // 33, GIB, 33, GIB // 33), (GIB // 33 + 1, GIB, 33, 0), ((1 << 31) - 1, GIB, 33, 0),
+    (1 << 31, GIB, 0, 0), ((1 << 64) - 1, GIB, 33, 0), (10, MIN * 33 - 1, 33, 0),
+])
+def test_room_for_a_callers_buffer(limits, cap, limit, row, want):
+    """The whole buffer or a count first: never an attempt at part of it."""
+    assert limits("emit_room", 1, cap, limit, row) == [want]

@@ -113,3 +113,22 @@ def test_emit_falls_back_only_when_its_buffer_is_full(dense):
         dg.emit(q, max_elements=1000)
     assert e.value.code == L.MG_E_LIMIT
     assert np.array_equal(dg.emit(q), want)
+
+
+def test_emit_of_more_than_2_22_rows_is_one_enumeration():
+    """5 million edges of a ring of chords, written into a buffer of just their size:
+    as many launches as levels, and the rows are the edges."""
+    n, chords = 50_000, 50
+    v = np.repeat(np.arange(n, dtype=np.uint32), chords)
+    w = (v + np.tile(np.arange(1, chords + 1, dtype=np.uint32), n)) % n
+    g = mg.CSRGraph.from_edges(n, v, w, np.zeros(n, np.uint32), symmetrize=True)
+    dg = mg.DeviceGraph(g)
+    q = mg.CSRGraph.query(2, [(0, 1)], [0, 0])
+    total = 2 * n * chords
+    assert total > 1 << 22
+    dg.emit(q, cap=total)  # (the level tables have grown at the second call)
+    rows, got, st = dg.emit(q, cap=total, stats=True)
+    assert got == total and st["launches"] <= 4
+    both = np.concatenate([np.stack([v, w], 1), np.stack([w, v], 1)]).astype(np.uint32)
+    assert np.array_equal(rows, both[np.lexsort((both[:, 1], both[:, 0]))])
+    dg.free()
