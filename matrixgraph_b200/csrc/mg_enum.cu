@@ -2380,8 +2380,9 @@ int subiso_count(DevGraph* dg, const mg_csr_view* q, const mg_opts* opts, uint64
 }
 
 // Lays out an emit buffer for `cap` rows in the graph's emit block, which grows
-// as needed and is given back by trim_emit when it is large.
-constexpr uint64_t kEmitKeep = 1ull << 30;
+// as needed and is given back by trim_emit when it is large: 256 MiB hold 2^22
+// rows of up to 4 ids whatever their bits.
+constexpr uint64_t kEmitKeep = 1ull << 28;
 
 static uint32_t id_bits(const DevGraph* dg) {
   uint32_t bits = 1;
@@ -2433,9 +2434,10 @@ int subiso_emit(DevGraph* dg, const mg_csr_view* q, const mg_opts* opts, const R
   RunResult tried, counted, res;  // an attempt, a count, the pass that gave the rows
   RowBuf eb;
   uint64_t c = 0, unused = 0;
-  const uint64_t room = emit_room(!sink.alloc, sink.cap_rows, kEmitKeep, [&](uint64_t rows) {
-    return RowBuf().carve(nullptr, P.k, id_bits(dg), rows);
-  });
+  const uint64_t limit = o.mem_budget_bytes ? std::min(o.mem_budget_bytes, kEmitKeep) : kEmitKeep;
+  const uint64_t room = emit_room(
+      !sink.alloc, sink.cap_rows, uint64_t(dg->g.n) + dg->info.m_out, limit, dg->emit_bytes,
+      [&](uint64_t rows) { return RowBuf().carve(nullptr, P.k, id_bits(dg), rows); });
   if (room) rc = emit_buffer(dg, P.k, room, &eb);
   const bool no_room = !room || rc == MG_E_OOM;
   if (!no_room && rc == MG_OK) {

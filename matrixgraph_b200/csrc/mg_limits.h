@@ -49,20 +49,30 @@ inline LaneStart lane_start(uint64_t t0, uint64_t budget, uint64_t seg_cap) {
 
 // Rows that an emit call makes room for before it knows how many there are, or 0:
 // count first.  The caller has memory for cap_rows rows (known), or takes any
-// number.  A buffer of up to `limit` bytes is tried at its full size, so that
-// what fits the caller is enumerated once; a larger one is counted first, since
-// an attempt at less than the caller's room would be a third enumeration of just
-// those results that are large.  bytes(rows): size of the buffer.
+// number.  bytes(rows): size of the buffer; limit: bytes it may take; held: bytes
+// that an earlier call left with the graph.
+//   known    A buffer of up to `limit` is tried at its full size, so that what
+//            fits the caller is enumerated once; a larger one is counted first,
+//            since an attempt at less than the caller's room would be a third
+//            enumeration of just those results that are large.
+//   unknown  Room as the level tables start: by the graph's entries (vertices and
+//            adjacency), so that ten rows of a small graph do not take 130 MB, and
+//            as much as the block that is there holds anyway.
 constexpr uint64_t kEmitTryMin = 1ull << 16, kEmitTry = 1ull << 22;
 
 template <class Bytes>
-inline uint64_t emit_room(bool known, uint64_t cap_rows, uint64_t limit, Bytes bytes) {
+inline uint64_t emit_room(bool known, uint64_t cap_rows, uint64_t entries, uint64_t limit,
+                          uint64_t held, Bytes bytes) {
+  uint64_t room = kEmitTryMin;
   if (known) {
     if (cap_rows >= 1ull << 31) return 0;
-    const uint64_t room = cap_rows > kEmitTryMin ? cap_rows : kEmitTryMin;
-    return bytes(room) <= limit ? room : 0;
+    if (cap_rows > room) room = cap_rows;
+  } else {
+    while (room < kEmitTry && ((room < 4 * entries && bytes(2 * room) <= limit) ||
+                               bytes(2 * room) <= held))
+      room <<= 1;
   }
-  return kEmitTry;
+  return bytes(room) <= limit || bytes(room) <= held ? room : 0;
 }
 
 }  // namespace mg

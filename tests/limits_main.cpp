@@ -19,10 +19,11 @@ int main(int argc, char** argv) {
                 mg::LB_MAX, mg::LB_EPOCHS);
     return 0;
   }
-  if (!std::strcmp(what, "emit_room")) {  // known, cap_rows, limit, bytes of a row
-    const unsigned long long row = arg(5);
+  if (!std::strcmp(what, "emit_room")) {  // known, cap_rows, entries, limit, held, bytes of a row
+    const unsigned long long row = arg(7);
     std::printf("%llu\n", (unsigned long long)mg::emit_room(
-                              arg(2) != 0, arg(3), arg(4), [&](uint64_t rows) { return rows * row; }));
+                              arg(2) != 0, arg(3), arg(4), arg(5), arg(6),
+                              [&](uint64_t rows) { return rows * row; }));
     return 0;
   }
   return 2;

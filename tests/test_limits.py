@@ -60,4 +60,24 @@ GIB = 1 << 30
 ])
 def test_room_for_a_callers_buffer(limits, cap, limit, row, want):
     """The whole buffer or a count first: never an attempt at part of it."""
-    assert limits("emit_room", 1, cap, limit, row) == [want]
+    assert limits("emit_room", 1, cap, 0, limit, 0, row) == [want]
+
+
+KEEP = 1 << 28
+
+
+@pytest.mark.parametrize("entries, limit, held, want", [
+    (0, KEEP, 0, MIN), (110_000, KEEP, 0, 1 << 19), (MIN // 4, KEEP, 0, MIN),
+    (MIN // 4 + 1, KEEP, 0, 2 * MIN), (1 << 30, KEEP, 0, TRY), (1 << 30, 33 << 20, 0, 1 << 20),
+    (1 << 30, 33 * MIN - 1, 0, 0),
+    # what the graph holds already is used, however small the graph
+    (0, KEEP, 33 * MIN * 8, MIN * 8), (0, KEEP, 33 * MIN * 8 - 1, MIN * 4), (0, 0, 33 * TRY, TRY),
+])
+def test_room_for_any_number_of_rows(limits, entries, limit, held, want):
+    assert limits("emit_room", 0, (1 << 64) - 1, entries, limit, held, 33) == [want]
+
+
+def test_room_of_a_large_held_block(limits):
+    """A block that is there serves a caller's buffer beyond the limit, too."""
+    assert limits("emit_room", 1, 10 ** 7, 0, KEEP, 33 * 10 ** 7, 33) == [10 ** 7]
+    assert limits("emit_room", 1, 10 ** 7, 0, KEEP, 33 * 10 ** 7 - 1, 33) == [0]

@@ -132,3 +132,17 @@ def test_emit_of_more_than_2_22_rows_is_one_enumeration():
     both = np.concatenate([np.stack([v, w], 1), np.stack([w, v], 1)]).astype(np.uint32)
     assert np.array_equal(rows, both[np.lexsort((both[:, 1], both[:, 0]))])
     dg.free()
+
+
+def test_small_graph_keeps_a_small_emit_block():
+    """The first emit of a graph of some ten thousand edges does not take room for
+    millions of rows."""
+    torch = pytest.importorskip("torch")
+    g = mg.chung_lu(2000, avg_deg=6, n_labels=4)
+    dg = mg.DeviceGraph(g)
+    q = mg.CSRGraph.query(4, [(0, 1), (1, 2), (2, 3), (3, 0)], [0, 1, 0, 1])
+    n = dg.count(q)  # the level tables
+    before = torch.cuda.mem_get_info()[0]
+    assert np.array_equal(dg.emit(q), oracle_rows(g, q)) and n == len(dg.emit(q))
+    assert before - torch.cuda.mem_get_info()[0] <= 32 << 20
+    dg.free()
