@@ -2201,10 +2201,10 @@ static int run_levels(DevGraph* dg, std::vector<PlanDev> plans, bool count_mode,
   if (rc) return rc;
   Workspace* ws = dg->ws;
   if (o.mem_budget_bytes) {  // tables of earlier calls count too
-    uint64_t held = 0;
-    for (int l = 0; l < MAXK; ++l) held += ws->rows[l] * level_row_bytes(l);
-    if (held > o.mem_budget_bytes)
-      for (int l = 0; l < MAXK; ++l) {
+    const uint32_t mask = tables_to_free(ws->rows, MAXK, int(kmax), cap, o.mem_budget_bytes,
+                                         [](int l) { return level_row_bytes(l); });
+    for (int l = 0; l < MAXK; ++l)
+      if (mask >> l & 1u) {
         cudaFree(ws->block[l]);
         ws->block[l] = nullptr;
         ws->rows[l] = 0;

@@ -47,6 +47,24 @@ inline LaneStart lane_start(uint64_t t0, uint64_t budget, uint64_t seg_cap) {
   return t0 > seg_cap ? LaneStart::kChunked : LaneStart::kRun;
 }
 
+// Level tables to give back (a bit per level) before a call that uses levels
+// 1..used-1 with up to cap rows each may grow its own: none when what it will hold
+// at most, with the tables that earlier calls left, is within the budget; else
+// those of levels it does not use and those of more than cap rows.  rows[l]: rows
+// that table l has now; row_bytes(l): bytes of a row.  cap rows of every used
+// level are within the budget.
+template <class RowBytes>
+inline uint32_t tables_to_free(const uint64_t* rows, int levels, int used, uint64_t cap,
+                               uint64_t budget, RowBytes row_bytes) {
+  uint64_t most = 0;
+  uint32_t mask = 0;
+  for (int l = 1; l < levels; ++l) {
+    most += (l < used && rows[l] < cap ? cap : rows[l]) * row_bytes(l);
+    if (rows[l] && (l >= used || rows[l] > cap)) mask |= 1u << l;
+  }
+  return most > budget ? mask : 0;
+}
+
 // Rows that an emit call makes room for before it knows how many there are, or 0:
 // count first.  The caller has memory for cap_rows rows (known), or takes any
 // number.  bytes(rows): size of the buffer; limit: bytes it may take; held: bytes

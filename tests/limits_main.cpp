@@ -26,5 +26,14 @@ int main(int argc, char** argv) {
                               [&](uint64_t rows) { return rows * row; }));
     return 0;
   }
+  if (!std::strcmp(what, "tables")) {  // used, cap, budget, rows of level 0, 1, ...
+    uint64_t rows[16] = {};
+    for (int l = 0; l < 16; ++l) rows[l] = arg(5 + l);
+    const uint32_t mask = mg::tables_to_free(rows, 16, int(arg(2)), arg(3), arg(4),
+                                             [](int l) { return uint64_t(l) * 4 + 21; });
+    for (int l = 0; l < 16; ++l)
+      if (mask >> l & 1u) std::printf("%d\n", l);
+    return 0;
+  }
   return 2;
 }

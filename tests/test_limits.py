@@ -81,3 +81,24 @@ def test_room_of_a_large_held_block(limits):
     """A block that is there serves a caller's buffer beyond the limit, too."""
     assert limits("emit_room", 1, 10 ** 7, 0, KEEP, 33 * 10 ** 7, 33) == [10 ** 7]
     assert limits("emit_room", 1, 10 ** 7, 0, KEEP, 33 * 10 ** 7 - 1, 33) == [0]
+
+
+# rows of 25, 29, 33 bytes at levels 1, 2, 3; a call of 4 vertices uses the three
+@pytest.mark.parametrize("cap, budget, rows, want", [
+    (1000, 87_000, [], []),
+    (1000, 87_000, [4, 1000, 1000, 1000], []),
+    (1000, 87_000, [4, 1001], [1]),              # level 1 as it is, 2 and 3 grown to cap
+    (1000, 90_000, [4, 1001], []),
+    (1000, 87_000, [4, 500, 3000, 10], [2]),     # within the budget alone, not once grown
+    (1000, 87_000, [4, 500, 500, 500, 1], [4]),  # a level that this call does not use
+    (1000, 87_000, [4, 2000, 500, 2000, 0, 7], [1, 3, 5]),
+    (1, 87, [1 << 20], []),                      # level 0 is the call's queries
+])
+def test_tables_of_earlier_calls_under_a_budget(limits, cap, budget, rows, want):
+    got = limits("tables", 4, cap, budget, *rows)
+    assert got == want
+    size = {1: 25, 2: 29, 3: 33, 4: 37, 5: 41}
+    left = {level: n for level, n in enumerate(rows) if level and n and level not in got}
+    held = {level: max(left.get(level, 0), cap) for level in (1, 2, 3)}
+    held.update({level: n for level, n in left.items() if level > 3})
+    assert sum(n * size[level] for level, n in held.items()) <= budget

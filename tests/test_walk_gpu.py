@@ -146,3 +146,28 @@ def test_small_graph_keeps_a_small_emit_block():
     assert np.array_equal(dg.emit(q), oracle_rows(g, q)) and n == len(dg.emit(q))
     assert before - torch.cuda.mem_get_info()[0] <= 32 << 20
     dg.free()
+
+
+def test_memory_budget_covers_tables_of_earlier_calls():
+    """A call without a budget leaves a large table at level 1; one with a budget of
+    56 MiB, whose deeper levels grow as far as they may, stays within it."""
+    torch = pytest.importorskip("torch")
+    n = 1 << 21
+    v = np.arange(n, dtype=np.uint32)
+    g = mg.CSRGraph.from_edges(n, np.tile(v, 3), np.concatenate([np.roll(v, -s) for s in (1, 2, 3)]),
+                               np.zeros(n, np.uint32), symmetrize=True)
+    dg = mg.DeviceGraph(g, hub_bytes=0)
+    first = torch.cuda.mem_get_info()[0]
+    path = mg.CSRGraph.query(3, [(0, 1), (1, 2)], [0] * 3)
+    cycle = mg.CSRGraph.query(4, [(0, 1), (1, 2), (2, 3), (3, 0)], [0] * 4)
+    # every vertex has neighbours at these distances
+    steps = (-3, -2, -1, 1, 2, 3)
+    closed = [(a, a + b, a + b + c) for a in steps for b in steps for c in steps
+              if len({0, a, a + b, a + b + c}) == 4 and -(a + b + c) in steps]
+    # (the path's last position is closed in place: one table, of 2^21 rows)
+    assert dg.count(path, no_tail=1, chunk_rows=1 << 21) == n * 6 * 5
+    budget = 56 << 20
+    assert dg.count(cycle, mem_budget_bytes=budget) == n * len(closed)
+    held = first - torch.cuda.mem_get_info()[0]
+    assert held <= budget + (16 << 20)  # and the scratch that is not tables
+    dg.free()
