@@ -54,8 +54,6 @@ struct GraphDev {
   // d-neighbour of v.
   const uint16_t* hub_slot[2];
   const uint32_t* hub_bits[2];
-  const uint32_t* hub_vid[2];  // vertex of each hub slot
-  uint32_t n_hubs[2];
   uint32_t hub_words;
 };
 constexpr uint16_t NO_HUB = 0xFFFF;

@@ -91,8 +91,8 @@ struct Workspace {
 // Counter slots.  A level's slots lie together, so that clearing everything
 // from a level on is one memset.
 enum : int {
-  C_OUT = 0, C_BALG = 1, C_BALGC = 2, C_ERR = 3, C_EMIT = 4, C_TILE = 6,
-  C_LVL = 8,                    // slots of level l from C_LVL + 4 * l on:
+  C_BALG = 0, C_BALGC = 1, C_ERR = 2, C_EMIT = 3,
+  C_LVL = 4,                    // slots of level l from C_LVL + 4 * l on:
   L_OUT = 0,                    // rows the expand of level l wrote (= rows of level l+1)
   L_TILE = 1,                   // work-queue position of the expand of level l
   L_T = 2,                      // candidate elements of level l
@@ -1820,19 +1820,20 @@ static cudaError_t launch_chained(void (*kernel)(Args...), unsigned grid, unsign
   return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-static void launch_expand(const StepArgs& a, int mode, unsigned grid, cudaStream_t st,
-                          bool chained) {
+static cudaError_t launch_expand(const StepArgs& a, int mode, unsigned grid, cudaStream_t st,
+                                 bool chained) {
   switch (mode) {
 #define MG_X(m) \
   case m:       \
-    launch_chained(k_expand<m>, grid, EXPAND_BLOCK, st, chained, a); \
-    break;
-    // emit runs hold one query, whose level either writes or emits
+    return launch_chained(k_expand<m>, grid, EXPAND_BLOCK, st, chained, a);
+    // a batch's level, by what some query of it does there
     MG_X(0) MG_X(1) MG_X(4) MG_X(5) MG_X(8) MG_X(9) MG_X(12) MG_X(13)
-    MG_X(16) MG_X(17) MG_X(18) MG_X(20) MG_X(21) MG_X(24) MG_X(25) MG_X(28) MG_X(29)
+    // one query's level does one of them (emit runs hold one query)
+    MG_X(16) MG_X(17) MG_X(18) MG_X(20) MG_X(24)
     MG_X(52) MG_X(56) MG_X(116) MG_X(120) MG_X(144) MG_X(145) MG_X(272) MG_X(273)
 #undef MG_X
   }
+  return cudaErrorInvalidDeviceFunction;  // no such shape
 }
 
 // Tail keys (da, la, db, lb, lp) of the plans that end in a two-position
@@ -2028,7 +2029,7 @@ static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool cou
   };
   auto expand = [&](int l, uint64_t bound) -> int {
     if (o.kernel_events && B.ev2) MG_CK(cudaEventRecord(B.ev2, st));
-    launch_expand(a, mode[l], grid_for(bound, 256, sms * 4), st, one && a.dev);
+    MG_CK(launch_expand(a, mode[l], grid_for(bound, 256, sms * 4), st, one && a.dev));
     if (o.kernel_events && B.ev2) {
       MG_CK(cudaEventRecord(B.ev3, st));
       MG_CK(cudaEventSynchronize(B.ev3));
@@ -2057,8 +2058,8 @@ static int walk_levels(DevGraph* dg, const PlanDev* plans, uint32_t nq, bool cou
         MG_CK(cudaMemsetAsync(B.status, 0, B.status_bytes, st));
         *B.epoch = 1;
       }
-      launch_chained(k_work_scan, grid_for(rows, WS_ROWS, sms * 4), 256u, st,
-                     one && l > l0 && !clear, a, *B.epoch);
+      MG_CK(launch_chained(k_work_scan, grid_for(rows, WS_ROWS, sms * 4), 256u, st,
+                           one && l > l0 && !clear, a, *B.epoch));
       res->launches++;
       const uint64_t bound = std::min(bounded_product(rows, widest[l]), a.t_limit);
       if (int r = expand(l, bound)) return r;
@@ -2713,8 +2714,8 @@ static int subiso_batch_lanes(DevGraph* dg, std::vector<PlanDev>& plans, const m
       a.tile_slot = lvl_slot(l, L_TILE);
       const uint64_t bound =
           l == 0 ? t0[j] : bounded_product(rows, row_bound(dg, &P, 1, l));
-      launch_expand(a, expand_mode(a, uint32_t(l), &P, 1, true, writes),
-                    grid_for(bound, 256, sms * 4), L.st, false);
+      MG_CK(launch_expand(a, expand_mode(a, uint32_t(l), &P, 1, true, writes),
+                          grid_for(bound, 256, sms * 4), L.st, false));
       rows = std::min(bound, cap);
       res->launches++;
       res->expand_launches++;

@@ -470,18 +470,17 @@ static int build_hubs(DevGraph* dg, int d, const std::vector<uint32_t>& deg, uin
   int rc;
   if ((rc = dev_alloc(dg, (void**)&d_slot, uint64_t(n) * 2))) return rc;
   if ((rc = dev_alloc(dg, (void**)&d_bits, hub_vid.size() * row_bytes))) return rc;
-  if ((rc = dev_alloc(dg, (void**)&d_vid, hub_vid.size() * 4))) return rc;
+  MG_CK(cudaMallocAsync((void**)&d_vid, hub_vid.size() * 4, st));
   MG_CK(cudaMemcpyAsync(d_slot, slot.data(), uint64_t(n) * 2, cudaMemcpyHostToDevice, st));
   MG_CK(cudaMemcpyAsync(d_vid, hub_vid.data(), hub_vid.size() * 4, cudaMemcpyHostToDevice, st));
   MG_CK(cudaMemsetAsync(d_bits, 0, hub_vid.size() * row_bytes, st));
   k_hub_bits<<<unsigned(hub_vid.size()), 256, 0, st>>>(dg->g.adj[d], dg->g.loff[d], n, dg->g.L,
                                                       d_vid, words, d_bits);
   MG_CK(cudaGetLastError());
+  cudaFreeAsync(d_vid, st);
   MG_CK(cudaStreamSynchronize(st));
   dg->g.hub_slot[d] = d_slot;
   dg->g.hub_bits[d] = d_bits;
-  dg->g.hub_vid[d] = d_vid;
-  dg->g.n_hubs[d] = uint32_t(hub_vid.size());
   dg->g.hub_words = words;
   dg->info.hubs += uint32_t(hub_vid.size());
   dg->info.hub_min_degree = cut;
@@ -738,8 +737,6 @@ static int upload(const mg_csr_view* v, int device, const mg_upload_opts& uo, De
   if (sym) {
     dg->g.hub_slot[1] = dg->g.hub_slot[0];
     dg->g.hub_bits[1] = dg->g.hub_bits[0];
-    dg->g.hub_vid[1] = dg->g.hub_vid[0];
-    dg->g.n_hubs[1] = dg->g.n_hubs[0];
   }
   return MG_OK;
 }
