@@ -1449,8 +1449,10 @@ __device__ __forceinline__ unsigned long long look_back(const StepArgs& a, uint3
 // past seg_cap) stops the walk before the level is expanded.
 //
 // One launch and one pass over the rows in place of a work kernel, three scan
-// kernels and a tile-row search, with no size returned to the host.
-__global__ void __launch_bounds__(256) k_work_scan(StepArgs a, uint32_t epoch) {
+// kernels and a tile-row search, with no size returned to the host.  Five blocks
+// per SM (48 registers) is what the compiler takes by itself, but unasked it
+// spills 28 bytes there.
+__global__ void __launch_bounds__(256, 5) k_work_scan(StepArgs a, uint32_t epoch) {
   const uint32_t i = a.level;
   chain_begin();
   chain_wait();
