@@ -466,18 +466,17 @@ static int build_hubs(DevGraph* dg, int d, const std::vector<uint32_t>& deg, uin
   if (hub_vid.empty()) return MG_OK;
   cudaStream_t st = dg->stream;
   uint16_t* d_slot;
-  uint32_t *d_bits, *d_vid;
+  uint32_t* d_bits;  // the rows, and behind them the vertices they are built from
   int rc;
   if ((rc = dev_alloc(dg, (void**)&d_slot, uint64_t(n) * 2))) return rc;
-  if ((rc = dev_alloc(dg, (void**)&d_bits, hub_vid.size() * row_bytes))) return rc;
-  MG_CK(cudaMallocAsync((void**)&d_vid, hub_vid.size() * 4, st));
+  if ((rc = dev_alloc(dg, (void**)&d_bits, hub_vid.size() * (row_bytes + 4)))) return rc;
+  uint32_t* d_vid = d_bits + hub_vid.size() * words;
   MG_CK(cudaMemcpyAsync(d_slot, slot.data(), uint64_t(n) * 2, cudaMemcpyHostToDevice, st));
   MG_CK(cudaMemcpyAsync(d_vid, hub_vid.data(), hub_vid.size() * 4, cudaMemcpyHostToDevice, st));
   MG_CK(cudaMemsetAsync(d_bits, 0, hub_vid.size() * row_bytes, st));
   k_hub_bits<<<unsigned(hub_vid.size()), 256, 0, st>>>(dg->g.adj[d], dg->g.loff[d], n, dg->g.L,
                                                       d_vid, words, d_bits);
   MG_CK(cudaGetLastError());
-  cudaFreeAsync(d_vid, st);
   MG_CK(cudaStreamSynchronize(st));
   dg->g.hub_slot[d] = d_slot;
   dg->g.hub_bits[d] = d_bits;
