@@ -1,5 +1,7 @@
 """The walk over the level tables where it stops and goes on: levels larger than
 their table, more blocks than tiles, and the limits of a call, against the oracle."""
+import itertools
+
 import numpy as np
 import pytest
 
@@ -170,4 +172,50 @@ def test_memory_budget_covers_tables_of_earlier_calls():
     assert dg.count(cycle, mem_budget_bytes=budget) == n * len(closed)
     held = first - torch.cuda.mem_get_info()[0]
     assert held <= budget + (16 << 20)  # and the scratch that is not tables
+    dg.free()
+
+
+@pytest.mark.parametrize("k", [4, 5])
+def test_tail_sums_in_place_without_memory_for_its_table(k):
+    """A pendant tail whose table (48 MiB here) does not fit the free memory is summed
+    where it is closed; with memory, the same call takes the table."""
+    torch = pytest.importorskip("torch")
+    # A ring with chords; every fourth vertex carries the label of the path's end.
+    path = mg.CSRGraph.query(k, [(i, i + 1) for i in range(k - 1)], [0] * (k - 1) + [1])
+    per_4 = 0
+    for start in range(4):
+        for steps in itertools.product((-2, -1, 1, 2), repeat=k - 1):
+            at = np.cumsum((start,) + steps)
+            per_4 += len(set(at.tolist())) == k and \
+                (at % 4 == 3).tolist() == [False] * (k - 1) + [True]
+
+    def ring(n):
+        v = np.arange(n, dtype=np.uint32)
+        g = mg.CSRGraph.from_edges(n, np.tile(v, 2), np.concatenate([np.roll(v, -1), np.roll(v, -2)]),
+                                   (v % 4 == 3).astype(np.uint32), symmetrize=True)
+        return g, mg.DeviceGraph(g, hub_bytes=0)
+
+    g, dg = ring(1000)
+    assert dg.count(path) == 250 * per_4 > 0  # (its kernels are loaded)
+    dg.free()
+    n = 1 << 22
+    table = 16 * (n - n // 4)
+    g, dg = ring(n)
+    assert dg.count(path, no_tail=1) == n // 4 * per_4  # the level tables
+    torch.cuda.synchronize()
+    filler = [torch.empty(torch.cuda.mem_get_info()[0] - (64 << 20), dtype=torch.uint8,
+                          device="cuda")]
+    try:  # what the driver keeps back for allocations, too
+        while True:
+            filler.append(torch.empty(16 << 20, dtype=torch.uint8, device="cuda"))
+    except torch.OutOfMemoryError:
+        pass
+    del filler[-1:]
+    torch.cuda.empty_cache()  # 16 MiB and less than a chunk are left
+    assert dg.count(path) == n // 4 * per_4
+    del filler
+    torch.cuda.empty_cache()
+    free = torch.cuda.mem_get_info()[0]
+    assert dg.count(path) == n // 4 * per_4
+    assert free - torch.cuda.mem_get_info()[0] >= table  # the table is there now
     dg.free()
