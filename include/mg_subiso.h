@@ -93,9 +93,9 @@ typedef struct mg_opts {
   void*    model;            /* order model for MG_ORDER_LEARNED (may be NULL:
                                 then the reference order is used)            */
   uint64_t chunk_rows;       /* partial-match rows per level chunk; 0 = auto */
-  uint32_t grab;             /* expand tiles (256 candidates each) a block
-                                takes from the device work queue at a time;
-                                0 = auto                                     */
+  uint32_t grab;             /* expand tasks (up to 1,024 candidates each) a
+                                warp takes from the device work queue at a
+                                time; 0 = auto                               */
   uint32_t root_step;        /* level-0 candidates are the bucket positions
                                 root_begin, root_begin + root_step, ... below
                                 root_end (0 or 1: every position).  A stride
@@ -141,7 +141,8 @@ typedef struct mg_stats {
   uint64_t balg_bytes;       /* algorithmic bytes, full-slice definition     */
   uint64_t balg_count_bytes; /* algorithmic bytes, count-mode definition     */
   double   device_ms;        /* device time from first launch to result      */
-  uint64_t launches;         /* kernels launched by this call                */
+  uint64_t launches;         /* kernels launched by this call (emits: by all
+                                of its walks, without the row sort)          */
   uint64_t chunks;           /* level chunks processed                       */
   uint64_t elements;         /* candidate elements expanded                  */
   double   expand_ms;        /* summed durations of the expand-kernel launches

@@ -6,7 +6,9 @@ bucket is timed under every candidate setting of
 * ``lanes``      concurrent per-query launch pipelines of a batch call,
 * ``probe_min``  shortest hub slice probed in the hub bitmap (binary search
                  below it),
-* ``grab``       expand tiles a block takes from the work queue at a time,
+* ``grab``       expand tasks (up to 1,024 candidates each) a warp takes from
+                 the work queue at a time (tables tuned when it meant tiles of
+                 256 candidates a block took are to be tuned again),
 
 and the fastest setting is kept.  Results go to a small text table keyed by
 the graph's signature and the bucket, read back by :func:`load_table` and by

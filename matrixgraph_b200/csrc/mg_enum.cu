@@ -844,7 +844,8 @@ __device__ __forceinline__ void probe_all(const uint32_t* const (&p)[U], const u
 // candidates, 71% issue).  R-MAT scale 18, 5-paths whose ends share a label:
 // 90 -> 184 and 47 -> 191 G candidates/s; scale 22, 5-path: 6.5 -> 5.5 ms, and
 // 2.6 ms with all a tail needs in one 16-byte table entry instead of six loads
-// (3.6 ms at four blocks per SM, whose 64 registers spill: tails get 80).
+// (3.6 ms at four blocks per SM with 64 registers; the tail shapes get three blocks
+// and 80 registers, of which 56 and 120 still spill 36 and 44 bytes and 24 spills 24).
 //
 // X_PAIR, the commonest shape (two lists intersected), leaves out what the
 // others may need and has the registers for three candidates a lane: 4-cycle
@@ -2253,8 +2254,8 @@ static int run_levels(DevGraph* dg, std::vector<PlanDev> plans, bool count_mode,
     a.root_keep = ws->root_keep;
     res->launches++;
   }
-  // Pendant tails counted in closed form (count mode): tail-key table and
-  // memo table of two-hop aggregates, shared by every query of the call.
+  // Pendant tails counted in closed form (count mode): the tables of two-hop
+  // aggregates of their keys, shared by every query of the call.
   if (count_mode && o.no_tail != 1) {
     if ((rc = setup_tails(dg, plans, ws->tails, st, &a, &res->launches))) return rc;
   }
@@ -2487,10 +2488,10 @@ int subiso_emit(DevGraph* dg, const mg_csr_view* q, const mg_opts* opts, const R
 // ---------------------------------------------------------------------------
 // Batch lane pipeline
 //
-// Each query of a batch runs as a fixed sequence of launches (per level: the
-// single-pass work/scan, the tile-row lookup, the expand) whose kernels read
-// every size from device counters, so nothing returns to the host between
-// levels or between queries.  Queries are dealt round-robin to `lanes`
+// Each query of a batch runs as a fixed sequence of launches (level 0: the
+// expand; every level after it: the single-pass work/scan and the expand) whose
+// kernels read every size from device counters, so nothing returns to the host
+// between levels or between queries.  Queries are dealt round-robin to `lanes`
 // streams that run concurrently; each lane owns level tables of `cap` rows.
 // The host waits once per batch; a query whose rows or elements did not fit
 // its lane (ERR_OVERFLOW) is counted again on the chunked path, which has no
@@ -2637,8 +2638,8 @@ static int subiso_batch_lanes(DevGraph* dg, std::vector<PlanDev>& plans, const m
   MG_CK(cudaEventRecord(ws->ev0, st));
   StepArgs a;
   std::memset(&a, 0, sizeof(a));
-  // Pendant tails closed from hub aggregates (their table is filled on the
-  // graph's stream before the lanes start).
+  // Pendant tails closed from tables of two-hop aggregates (filled on the graph's
+  // stream before the lanes start).
   if (o.no_tail != 1) {
     if ((rc = setup_tails(dg, plans, ls->tails, st, &a, &res->launches))) return rc;
   } else {
